@@ -31,6 +31,8 @@ SIGNATURES = {
     "ebsd_grid_fz_write": (i32, [i32, i32, vp, sz, vp, vp, vp, vp]),
     "ebsd_gather_rows": (i32, [vp, i64, i32, vp, i64, vp, vp]),
     "ebsd_project_dictionary": (i32, [vp, i32, i32, vp, i32, vp, i64, i32, vp, i64, vp, i32, i64, vp, vp, vp]),
+    "ebsd_sampling_quads": (i32, [vp, i32, i32, vp, vp]),
+    "ebsd_project_dictionary_quads": (i32, [vp, i32, i32, vp, i32, vp, i64, i32, vp, i64, vp, i32, i64, vp, vp, vp]),
     "ebsd_prep_patterns": (i32, [vp, i64, i32, i32, i64, i32, vp, i32, i32, vp, i64, vp, i32, i64, vp, vp, vp]),
     "ebsd_prep_patterns_typed": (i32, [vp, i32, i64, i32, i32, i64, i32, vp, i32, i32, vp, i64, vp, i32, i64, vp,
                                        vp, vp]),
@@ -101,6 +103,7 @@ DEVICE_TIMEOUT = 0x7001
 # kernels launched by one successful call of each entry point
 LAUNCHES_PER_CALL = {
     "ebsd_grid_fz_count": 2, "ebsd_grid_fz_write": 1, "ebsd_gather_rows": 1, "ebsd_project_dictionary": 1,
+    "ebsd_sampling_quads": 1, "ebsd_project_dictionary_quads": 1,
     "ebsd_prep_patterns": 1, "ebsd_prep_patterns_typed": 1, "ebsd_sample_master_pattern": 1, "ebsd_avg_pool": 1,
     "ebsd_match_topk": 1, "ebsd_match_topk_tiled": 1,
     "ebsd_merge_rescore": 1, "ebsd_merge_rescore_gated": 1, "ebsd_manhattan_topk": 1, "ebsd_gemm_nt": 1, "ebsd_gemm_f32": 1, "ebsd_col_mean": 1, "ebsd_split3_bf16": 1,

@@ -13,14 +13,17 @@
 // a unit-norm copy in the low-precision matching type (bf16, or e4m3 with a
 // per-row absmax scale), zero padded to the GEMM row length.
 #include <algorithm>
+#include <cstring>
+#include <type_traits>
 
 #include "common.cuh"
 #include "sampling.cuh"
 
 namespace ebsd {
 
-constexpr int kRowThreads = 512;
-constexpr int kProjIlp = 2;  // independent pixels per projector thread and step
+// Rows up to this length take 256-thread CTAs, six of which fit an SM beside an
+// L1 that still holds the rays; longer rows 512-thread CTAs (two to an SM).
+constexpr int kSmallRowPix = 6656;
 constexpr int kMaxRowPix = 57344;  // 224 KiB of fp32 in shared memory
 
 struct RowOut {
@@ -33,159 +36,309 @@ struct RowOut {
   float* lp_scale;
 };
 
+// Sum of the 2^k lane-group values red[0 .. n_warps) in every thread, n_warps
+// a power of two up to 32.
+template <typename T>
+__device__ __forceinline__ T sum_of_warps(const T* red, int n_warps) {
+  T v = red[threadIdx.x & (n_warps - 1)];
+  for (int o = n_warps >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// sqrt of an FP64 sum, rounded to FP32: one Newton step in FP64 from the FP32
+// reciprocal root (relative error 2^-22 squared), instead of the FP64 square
+// root's long dependent chain in every thread of the block.
+__device__ __forceinline__ float root_of_sum(double x) {
+  if (!(x >= 1e-30 && x <= 1e30)) return (float)sqrt(x);
+  const float r = rsqrtf((float)x);
+  const double y = x * (double)r;
+  return (float)fma(0.5 * (double)r, fma(-y, y, x), y);
+}
+
+// Two FP32 values as e4m3 (round to nearest even, saturating) in 16 bits.
+__device__ __forceinline__ uint32_t e4m3x2(float lo, float hi) {
+  return __nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, __NV_E4M3);
+}
+
+// Scratch of one block's row reductions.
+struct RowScratch {
+  double sum[16], sq[16];
+  float amax[16];
+};
+
 // Row values are in row[0..n); part_sum is this thread's sum of the values it
 // wrote. Finalise and write the outputs of row `r` (the shared row itself is
-// left as it was): mean (FP64 block sum), then the norm and absmax of the
-// zero-mean row, then the FP32 and low-precision rows in one pass (16-byte
-// stores when the row length and strides allow).
-__device__ void finalize_row(const float* row, int n, int subtract_mean, float part_sum, int64_t r,
-                             const RowOut& o, float* fred, double* dred) {
-  const int tid = threadIdx.x;
-  double mean = 0.0;
-  if (subtract_mean) mean = block_sum<double>((double)part_sum, dred) / (double)n;
-  const float meanf = (float)mean;
+// left as it was): the mean (FP64 sum), then, where a norm or low-precision
+// row is wanted, the norm and absmax of the zero-mean row, then the rows, in
+// 16-byte stores where length and strides allow. The caller's block holds a
+// power-of-two number of warps, has not synchronised since writing the row,
+// and synchronises before the row or the scratch are written again.
+__device__ __forceinline__ void finalize_row(const float* row, int n, double inv_n, int subtract_mean,
+                                             double part_sum, int64_t r, const RowOut& o, RowScratch& red) {
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5, n_warps = nt >> 5;
+  part_sum = warp_sum(part_sum);
+  if (lane == 0) red.sum[wid] = part_sum;
+  __syncthreads();
+  const float meanf = subtract_mean ? (float)(sum_of_warps(red.sum, n_warps) * inv_n) : 0.0f;
+  const float4* row4 = reinterpret_cast<const float4*>(row);
+  float* f32 = o.f32 ? o.f32 + r * o.ld_f32 : nullptr;
+  const bool vec_f32 = (n & 3) == 0 && (reinterpret_cast<uintptr_t>(f32) & 15) == 0;
+  if (!o.lp && !o.norm && !o.lp_scale) {
+    if (vec_f32) {
+      for (int c = tid; c < n / 4; c += nt) {
+        const float4 a = row4[c];
+        reinterpret_cast<float4*>(f32)[c] = make_float4(a.x - meanf, a.y - meanf, a.z - meanf, a.w - meanf);
+      }
+    } else {
+      for (int p = tid; p < n; p += nt) f32[p] = row[p] - meanf;
+    }
+    return;
+  }
   float ss = 0.0f, amax = 0.0f;
-  for (int p = tid; p < n; p += blockDim.x) {
+  for (int c = tid; c < n / 4; c += nt) {
+    const float4 a = row4[c];
+    const float v[4] = {a.x - meanf, a.y - meanf, a.z - meanf, a.w - meanf};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      ss = fmaf(v[e], v[e], ss);
+      amax = fmaxf(amax, fabsf(v[e]));
+    }
+  }
+  for (int p = (n & ~3) + tid; p < n; p += nt) {
     const float v = row[p] - meanf;
-    ss += v * v;
+    ss = fmaf(v, v, ss);
     amax = fmaxf(amax, fabsf(v));
   }
-  const double nrm2 = block_sum<double>((double)ss, dred);
-  const float nrm = (float)sqrt(nrm2);
+  const bool e4m3 = o.lp && o.lp_dtype == EBSD_DT_E4M3;
+  const double wss = warp_sum((double)ss);
+  if (e4m3) amax = warp_max(amax);
+  if (lane == 0) {
+    red.sq[wid] = wss;
+    red.amax[wid] = amax;
+  }
+  __syncthreads();
+  const float nrm = root_of_sum(sum_of_warps(red.sq, n_warps));
   const float inv = nrm > 0.0f ? 1.0f / nrm : 0.0f;
   float qscale = 1.0f;
-  if (o.lp && o.lp_dtype == EBSD_DT_E4M3) {
-    const float m = block_max(amax, fred) * inv;  // absmax of the unit row
+  if (e4m3) {
+    const float m = warp_max(red.amax[lane & (n_warps - 1)]) * inv;  // absmax of the unit row
     qscale = m > 0.0f ? m / 448.0f : 1.0f;
   }
   if (tid == 0) {
     if (o.norm) o.norm[r] = nrm;
     if (o.lp_scale) o.lp_scale[r] = qscale;
   }
-  float* f32 = o.f32 ? o.f32 + r * o.ld_f32 : nullptr;
-  const bool bf16 = o.lp && o.lp_dtype == EBSD_DT_BF16;
-  __nv_bfloat16* lp16 = bf16 ? reinterpret_cast<__nv_bfloat16*>(o.lp) + r * o.ld_lp : nullptr;
-  const bool vec = (n & 7) == 0 && (!f32 || ((reinterpret_cast<uintptr_t>(f32) & 15) == 0)) &&
-                   (!lp16 || ((reinterpret_cast<uintptr_t>(lp16) & 15) == 0)) && (o.lp == nullptr || bf16);
-  if (vec) {
-    // eight values per thread and step: two float4 loads and stores, one
-    // 16-byte bf16 store
-    for (int c = tid; c < n / 8; c += blockDim.x) {
-      const float4 a = reinterpret_cast<const float4*>(row)[2 * c];
-      const float4 b = reinterpret_cast<const float4*>(row)[2 * c + 1];
-      const float v[8] = {a.x - meanf, a.y - meanf, a.z - meanf, a.w - meanf,
-                          b.x - meanf, b.y - meanf, b.z - meanf, b.w - meanf};
-      if (f32) {
+  if (f32 && !vec_f32)
+    for (int p = tid; p < n; p += nt) f32[p] = row[p] - meanf;
+  if (!o.lp) {
+    if (f32 && vec_f32)
+      for (int c = tid; c < n / 4; c += nt) {
+        const float4 a = row4[c];
+        reinterpret_cast<float4*>(f32)[c] = make_float4(a.x - meanf, a.y - meanf, a.z - meanf, a.w - meanf);
+      }
+    return;
+  }
+  // eight values per thread and step: two float4 loads, the FP32 stores, one
+  // 16-byte bf16 or 8-byte e4m3 store; zero from n to the row stride
+  const int ld_lp = (int)o.ld_lp;
+  const float sc = e4m3 ? inv / qscale : inv;
+  uint8_t* lp = static_cast<uint8_t*>(o.lp) + r * o.ld_lp * (e4m3 ? 1 : 2);
+  const bool vec_lp = (ld_lp & 7) == 0 && (reinterpret_cast<uintptr_t>(o.lp) & 15) == 0;
+  for (int c = tid; c < (ld_lp + 7) / 8; c += nt) {
+    float v[8];
+    if (8 * c + 8 <= n) {
+      const float4 a = row4[2 * c], b = row4[2 * c + 1];
+      v[0] = a.x - meanf;
+      v[1] = a.y - meanf;
+      v[2] = a.z - meanf;
+      v[3] = a.w - meanf;
+      v[4] = b.x - meanf;
+      v[5] = b.y - meanf;
+      v[6] = b.z - meanf;
+      v[7] = b.w - meanf;
+      if (f32 && vec_f32) {
         reinterpret_cast<float4*>(f32)[2 * c] = make_float4(v[0], v[1], v[2], v[3]);
         reinterpret_cast<float4*>(f32)[2 * c + 1] = make_float4(v[4], v[5], v[6], v[7]);
       }
-      if (lp16) {
-        __align__(16) __nv_bfloat16 h[8];
+    } else {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) h[e] = __float2bfloat16_rn(v[e] * inv);
-        reinterpret_cast<uint4*>(lp16)[c] = *reinterpret_cast<const uint4*>(h);
+      for (int e = 0; e < 8; ++e) {
+        const int p = 8 * c + e;
+        v[e] = p < n ? row[p] - meanf : 0.0f;
+        if (f32 && vec_f32 && p < n) f32[p] = v[e];
       }
     }
-    if (lp16)
-      for (int p = n + tid; p < o.ld_lp; p += blockDim.x) lp16[p] = __float2bfloat16_rn(0.0f);
-    return;
-  }
-  if (f32)
-    for (int p = tid; p < n; p += blockDim.x) f32[p] = row[p] - meanf;
-  if (lp16) {
-    for (int p = tid; p < o.ld_lp; p += blockDim.x) lp16[p] = __float2bfloat16_rn(p < n ? (row[p] - meanf) * inv : 0.0f);
-  } else if (o.lp) {
-    __nv_fp8_e4m3* dst = reinterpret_cast<__nv_fp8_e4m3*>(o.lp) + r * o.ld_lp;
-    const float sc = inv / qscale;
-    for (int p = tid; p < o.ld_lp; p += blockDim.x) dst[p] = __nv_fp8_e4m3(p < n ? (row[p] - meanf) * sc : 0.0f);
+    if (e4m3) {
+      uint2 h;
+      h.x = e4m3x2(v[0] * sc, v[1] * sc) | (e4m3x2(v[2] * sc, v[3] * sc) << 16);
+      h.y = e4m3x2(v[4] * sc, v[5] * sc) | (e4m3x2(v[6] * sc, v[7] * sc) << 16);
+      if (vec_lp) {
+        reinterpret_cast<uint2*>(lp)[c] = h;
+      } else {
+        for (int e = 0; e < 8 && 8 * c + e < ld_lp; ++e) lp[8 * c + e] = (uint8_t)((e < 4 ? h.x : h.y) >> (8 * (e & 3)));
+      }
+    } else {
+      __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) h[e] = __float2bfloat16_rn(v[e] * sc);
+      if (vec_lp) {
+        reinterpret_cast<uint4*>(lp)[c] = *reinterpret_cast<const uint4*>(h);
+      } else {
+        for (int e = 0; e < 8 && 8 * c + e < ld_lp; ++e) reinterpret_cast<__nv_bfloat16*>(lp)[8 * c + e] = h[e];
+      }
+    }
   }
 }
 
-__global__ void __launch_bounds__(kRowThreads, 2) k_project(
-    const float* __restrict__ mp, int mp_h, int mp_w2, const float* __restrict__ rays, int n_pix,
-    const float4* __restrict__ quats, int64_t n_rows, int subtract_mean, RowOut o) {
-  extern __shared__ float row[];
-  __shared__ float fred[32];
-  __shared__ double dred[32];
+// quads[y][x] = the four values a bilinear sample with lower tap (x, y)
+// blends, upper taps clamped to the border.
+__global__ void k_sampling_quads(const float* __restrict__ mp, int h, int w, float4* __restrict__ quads) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+  if (x >= w) return;
+  const int x1 = min(x + 1, w - 1);
+  const float* lo = mp + (int64_t)y * w;
+  const float* hi = mp + (int64_t)min(y + 1, h - 1) * w;
+  quads[(int64_t)y * w + x] = make_float4(__ldg(lo + x), __ldg(lo + x1), __ldg(hi + x), __ldg(hi + x1));
+}
+
+// The four taps of a sample: one float4 of a gather table, or four values of
+// the image (upper taps clamped to the border).
+template <bool QUADS>
+__device__ __forceinline__ float4 load_taps(const float* __restrict__ img, int mp_h, const LambertGrid& g, int i) {
+  if constexpr (QUADS) return __ldg(reinterpret_cast<const float4*>(img) + i);
+  const int y0 = i / (int)g.w, x0 = i - y0 * (int)g.w;
+  const float* lo = img + i;
+  const float* hi = y0 < mp_h - 1 ? lo + g.w : lo;
+  const int dx = x0 < (int)g.w - 1 ? 1 : 0;
+  return make_float4(__ldg(lo), __ldg(lo + dx), __ldg(hi), __ldg(hi + dx));
+}
+
+// One CTA per dictionary row, grid-stride; each thread computes the taps of
+// its next pixel while the gather of the current one is in flight. QUADS:
+// `img` holds the four taps of every pixel as one float4, so a sample is one
+// 16-byte gather instead of four 4-byte ones: neighbouring rays fall on
+// different image rows, so each gather of a warp touches up to 32 lines, and
+// those accesses bound the plain route. Bound by instruction issue now (issue
+// slots 0.61 busy with two unpipelined pixels a thread and half the warps).
+// 36,829 rows of 60^2 px: 98.5 G samples/s with IEEE-rounded divisions by two,
+// floors and four gathers, 125 with lambert_tap and the table, 150 pipelined
+// with 48 warps on an SM; 16,384 rows of 128^2: 97.7, 132, 150; 8,192 of
+// 160^2: 52, 93, 115. All bit for bit the same rows.
+// Both thread counts add pixels p = c (mod 512) in ascending order into one
+// FP32 partial sum per class c, so the row mean does not depend on the count.
+template <int THREADS, bool QUADS>
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 2) k_project(
+    const float* __restrict__ img, int mp_h, const LambertGrid g, const float* __restrict__ rays, int n_pix,
+    double inv_n, const float4* __restrict__ quats, int64_t n_rows, int subtract_mean, RowOut o) {
+  static_assert(THREADS == 512 || THREADS == 256, "partial sums by pixel modulo 512");
+  extern __shared__ __align__(16) float row[];
+  __shared__ RowScratch red;
   const float* rx = rays;
   const float* ry = rays + n_pix;
   const float* rz = rays + 2 * (int64_t)n_pix;
   for (int64_t r = blockIdx.x; r < n_rows; r += gridDim.x) {
     const float4 q = quats[r];
-    float part = 0.0f;
-    // kProjIlp pixels per thread and step, their master-pattern gathers
-    // issued together: the projector is bound by the gather latency through
-    // L2, and independent gathers in flight hide it
-    for (int p0 = threadIdx.x; p0 < n_pix; p0 += kProjIlp * blockDim.x) {
-      BorderTaps t[kProjIlp];
-#pragma unroll
-      for (int k = 0; k < kProjIlp; ++k) {
-        const int p = min(p0 + k * (int)blockDim.x, n_pix - 1);
-        const float3 v = rotate(q, __ldg(rx + p), __ldg(ry + p), __ldg(rz + p));
-        const float2 uv = lambert_side_by_side(v.x, v.y, v.z);
-        t[k] = border_taps(mp_h, mp_w2, uv.x, uv.y);
-      }
-      float g[kProjIlp][4];
-#pragma unroll
-      for (int k = 0; k < kProjIlp; ++k) {
-        g[k][0] = __ldg(mp + t[k].i00);
-        g[k][1] = __ldg(mp + t[k].i01);
-        g[k][2] = __ldg(mp + t[k].i10);
-        g[k][3] = __ldg(mp + t[k].i11);
-      }
-#pragma unroll
-      for (int k = 0; k < kProjIlp; ++k) {
-        const int p = p0 + k * (int)blockDim.x;
-        if (p < n_pix) {
-          const float val = g[k][0] * t[k].w00 + g[k][1] * t[k].w01 + g[k][2] * t[k].w10 + g[k][3] * t[k].w11;
-          row[p] = val;
-          part += val;
-        }
-      }
+    const float3 q2 = make_float3(2.0f * q.y, 2.0f * q.z, 2.0f * q.w);
+    float part = 0.0f, part_b = 0.0f;
+    int p = threadIdx.x;
+    LambertTap t = {0, 0.0f, 0.0f};
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (p < n_pix) {
+      t = lambert_tap(g, q, q2, __ldg(rx + p), __ldg(ry + p), __ldg(rz + p));
+      v = load_taps<QUADS>(img, mp_h, g, t.i);
     }
-    __syncthreads();
-    finalize_row(row, n_pix, subtract_mean, part, r, o, fred, dred);
+#pragma unroll 2
+    for (; p < n_pix; p += THREADS) {
+      const int pn = min(p + THREADS, n_pix - 1);
+      const LambertTap tn = lambert_tap(g, q, q2, __ldg(rx + pn), __ldg(ry + pn), __ldg(rz + pn));
+      const float4 vn = load_taps<QUADS>(img, mp_h, g, tn.i);
+      const float val = blend(t, v.x, v.y, v.z, v.w);
+      row[p] = val;
+      if constexpr (THREADS == 512) {
+        part += val;
+      } else {
+        const float s = part + val;
+        part = part_b;
+        part_b = s;
+      }
+      t = tn;
+      v = vn;
+    }
+    finalize_row(row, n_pix, inv_n, subtract_mean, (double)part + (double)part_b, r, o, red);
     __syncthreads();
   }
 }
 
-__device__ __forceinline__ float load_pixel(const float* p, int64_t i) { return __ldg(p + i); }
-__device__ __forceinline__ float load_pixel(const uint16_t* p, int64_t i) { return (float)__ldg(p + i); }
-__device__ __forceinline__ float load_pixel(const uint8_t* p, int64_t i) { return (float)__ldg(p + i); }
-__device__ __forceinline__ float load_pixel(const __half* p, int64_t i) { return __half2float(__ldg(p + i)); }
+__device__ __forceinline__ float as_float(float v) { return v; }
+__device__ __forceinline__ float as_float(uint16_t v) { return (float)v; }
+__device__ __forceinline__ float as_float(uint8_t v) { return (float)v; }
+__device__ __forceinline__ float as_float(__half v) { return __half2float(v); }
+template <typename T>
+__device__ __forceinline__ float load_pixel(const T* p, int64_t i) {
+  return as_float(__ldg(p + i));
+}
+
+// Four consecutive values, loaded as one word of their size.
+template <typename T>
+struct alignas(4 * sizeof(T)) Vec4 {
+  T v[4];
+};
+template <typename T>
+__device__ __forceinline__ Vec4<T> load_vec4(const Vec4<T>* p) {
+  using Word = std::conditional_t<sizeof(T) == 4, float4, std::conditional_t<sizeof(T) == 2, uint2, unsigned>>;
+  const Word x = __ldg(reinterpret_cast<const Word*>(p));
+  Vec4<T> r;
+  memcpy(&r, &x, sizeof(r));
+  return r;
+}
 
 // Patterns of type T (fp32, uint16 or uint8 detector counts, fp16) -> rows.
-template <typename T>
-__global__ void __launch_bounds__(kRowThreads) k_prep(const T* __restrict__ pats, int64_t n_rows,
-                                                      int h, int w, int64_t stride, int b,
-                                                      const int32_t* __restrict__ pix, int n_pix,
-                                                      int subtract_mean, RowOut o) {
-  extern __shared__ float row[];
-  __shared__ float fred[32];
-  __shared__ double dred[32];
+// Bound by HBM: one CTA per row, several rows' loads in flight per SM. vec4:
+// whole unbinned patterns whose length, stride and base allow loads of four
+// values.
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_prep(const T* __restrict__ pats, int64_t n_rows,
+                                                  int h, int w, int64_t stride, int b,
+                                                  const int32_t* __restrict__ pix, int n_pix, double inv_n,
+                                                  int vec4, int subtract_mean, RowOut o) {
+  extern __shared__ __align__(16) float row[];
+  __shared__ RowScratch red;
   const int wb = w / b;
   const float cnt = (float)(b * b);
   for (int64_t r = blockIdx.x; r < n_rows; r += gridDim.x) {
     const T* img = pats + r * stride;
     float part = 0.0f;
-    for (int p = threadIdx.x; p < n_pix; p += blockDim.x) {
-      const int idx = pix ? __ldg(pix + p) : p;
-      float v;
-      if (b == 1) {
-        v = load_pixel(img, idx);
-      } else {
+    if (vec4) {
+      const Vec4<T>* img4 = reinterpret_cast<const Vec4<T>*>(img);
+      float4* row4 = reinterpret_cast<float4*>(row);
+#pragma unroll 4
+      for (int c = threadIdx.x; c < n_pix / 4; c += THREADS) {
+        const Vec4<T> x = load_vec4(img4 + c);
+        const float4 f = make_float4(as_float(x.v[0]), as_float(x.v[1]), as_float(x.v[2]), as_float(x.v[3]));
+        row4[c] = f;
+        part += (f.x + f.y) + (f.z + f.w);
+      }
+    } else if (b == 1) {
+#pragma unroll 4
+      for (int p = threadIdx.x; p < n_pix; p += THREADS) {
+        const float v = load_pixel(img, pix ? __ldg(pix + p) : p);
+        row[p] = v;
+        part += v;
+      }
+    } else {
+      for (int p = threadIdx.x; p < n_pix; p += THREADS) {
+        const int idx = pix ? __ldg(pix + p) : p;
         const int i = idx / wb, j = idx - i * wb;
         const int64_t src = (int64_t)(i * b) * w + j * b;
         float s = 0.0f;
         for (int a = 0; a < b; ++a)
           for (int c = 0; c < b; ++c) s += load_pixel(img, src + (int64_t)a * w + c);
-        v = s / cnt;
+        const float v = s / cnt;
+        row[p] = v;
+        part += v;
       }
-      row[p] = v;
-      part += v;
     }
-    __syncthreads();
-    finalize_row(row, n_pix, subtract_mean, part, r, o, fred, dred);
+    finalize_row(row, n_pix, inv_n, subtract_mean, (double)part, r, o, red);
     __syncthreads();
   }
 }
@@ -218,40 +371,89 @@ static int check_row_out(const RowOut& o, int n_pix) {
   return 0;
 }
 
-static int row_grid(int64_t n_rows, size_t smem, const void* fn) {
+static int row_grid(int64_t n_rows, size_t smem, const void* fn, int threads) {
   int per_sm = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kRowThreads, smem) != cudaSuccess ||
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess ||
       per_sm < 1)
     per_sm = 1;
   const int64_t cap = (int64_t)device_sm_count() * per_sm * 8;
   return (int)std::min<int64_t>(n_rows, cap);
 }
 
+template <int THREADS, bool QUADS>
+static int launch_project(const float* img, int mp_h, int mp_w2, const float* rays, int n_pix, const float4* quats,
+                          int64_t n_rows, int subtract_mean, const RowOut& o, cudaStream_t s) {
+  const size_t smem = (size_t)n_pix * sizeof(float);
+  const auto fn = k_project<THREADS, QUADS>;
+  EBSD_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int grid = row_grid(n_rows, smem, (const void*)fn, THREADS);
+  fn<<<grid, THREADS, smem, s>>>(img, mp_h, lambert_grid(mp_h, mp_w2), rays, n_pix, 1.0 / n_pix, quats, n_rows, subtract_mean, o);
+  EBSD_LAUNCH_CHECK();
+  return 0;
+}
+
 }  // namespace ebsd
 
 using namespace ebsd;
+
+template <bool QUADS>
+static int project_rows(const float* img, int mp_h, int mp_w2, const float* rays_soa, int n_pix, const float* quats,
+                        int64_t n_rows, int subtract_mean, const RowOut& o, void* stream) {
+  EBSD_ARG_CHECK(img && rays_soa && quats, "ebsd_project_dictionary: null input");
+  EBSD_ARG_CHECK(mp_h >= 1 && mp_w2 >= 1, "master pattern shape (%d, %d) invalid", mp_h, mp_w2);
+  EBSD_ARG_CHECK(n_pix >= 1 && n_pix <= kMaxRowPix, "row length %d outside [1, %d]", n_pix,
+                 kMaxRowPix);
+  EBSD_ARG_CHECK(n_rows >= 0, "n_rows < 0");
+  EBSD_ARG_CHECK((reinterpret_cast<uintptr_t>(quats) & 15) == 0, "quats must be 16-byte aligned");
+  EBSD_ARG_CHECK(!QUADS || (reinterpret_cast<uintptr_t>(img) & 15) == 0, "quads must be 16-byte aligned");
+  if (int rc = check_row_out(o, n_pix)) return rc;
+  if (n_rows == 0) return 0;
+  const float4* q = reinterpret_cast<const float4*>(quats);
+  cudaStream_t s = as_stream(stream);
+  if (n_pix <= kSmallRowPix)
+    return launch_project<256, QUADS>(img, mp_h, mp_w2, rays_soa, n_pix, q, n_rows, subtract_mean, o, s);
+  return launch_project<512, QUADS>(img, mp_h, mp_w2, rays_soa, n_pix, q, n_rows, subtract_mean, o, s);
+}
 
 extern "C" int ebsd_project_dictionary(const float* master_pattern, int mp_h, int mp_w2,
                                        const float* rays_soa, int n_pix, const float* quats,
                                        int64_t n_rows, int subtract_mean, float* out_f32,
                                        int64_t ld_f32, void* out_lp, int lp_dtype, int64_t ld_lp,
                                        float* out_norm, float* out_lp_scale, void* stream) {
-  EBSD_ARG_CHECK(master_pattern && rays_soa && quats, "ebsd_project_dictionary: null input");
-  EBSD_ARG_CHECK(mp_h >= 1 && mp_w2 >= 1, "master pattern shape (%d, %d) invalid", mp_h, mp_w2);
-  EBSD_ARG_CHECK(n_pix >= 1 && n_pix <= kMaxRowPix, "row length %d outside [1, %d]", n_pix,
-                 kMaxRowPix);
-  EBSD_ARG_CHECK(n_rows >= 0, "n_rows < 0");
-  EBSD_ARG_CHECK((reinterpret_cast<uintptr_t>(quats) & 15) == 0, "quats must be 16-byte aligned");
-  RowOut o{out_f32, ld_f32, out_lp, lp_dtype, ld_lp, out_norm, out_lp_scale};
-  if (int rc = check_row_out(o, n_pix)) return rc;
-  if (n_rows == 0) return 0;
+  const RowOut o{out_f32, ld_f32, out_lp, lp_dtype, ld_lp, out_norm, out_lp_scale};
+  return project_rows<false>(master_pattern, mp_h, mp_w2, rays_soa, n_pix, quats, n_rows, subtract_mean, o, stream);
+}
+
+extern "C" int ebsd_sampling_quads(const float* master_pattern, int mp_h, int mp_w2, float* quads, void* stream) {
+  EBSD_ARG_CHECK(master_pattern && quads, "ebsd_sampling_quads: null pointer");
+  EBSD_ARG_CHECK(mp_h >= 1 && mp_h <= 65535 && mp_w2 >= 1, "master pattern shape (%d, %d) invalid", mp_h, mp_w2);
+  EBSD_ARG_CHECK((reinterpret_cast<uintptr_t>(quads) & 15) == 0, "quads must be 16-byte aligned");
+  k_sampling_quads<<<dim3(ceil_div(mp_w2, 256), mp_h), 256, 0, as_stream(stream)>>>(
+      master_pattern, mp_h, mp_w2, reinterpret_cast<float4*>(quads));
+  EBSD_LAUNCH_CHECK();
+  return 0;
+}
+
+extern "C" int ebsd_project_dictionary_quads(const float* quads, int mp_h, int mp_w2, const float* rays_soa,
+                                             int n_pix, const float* quats, int64_t n_rows, int subtract_mean,
+                                             float* out_f32, int64_t ld_f32, void* out_lp, int lp_dtype,
+                                             int64_t ld_lp, float* out_norm, float* out_lp_scale, void* stream) {
+  const RowOut o{out_f32, ld_f32, out_lp, lp_dtype, ld_lp, out_norm, out_lp_scale};
+  return project_rows<true>(quads, mp_h, mp_w2, rays_soa, n_pix, quats, n_rows, subtract_mean, o, stream);
+}
+
+template <typename T, int THREADS>
+static int launch_prep_threads(const T* patterns, int64_t n_rows, int height, int width, int64_t pattern_stride,
+                               int binning, const int32_t* pix_index, int n_pix, int subtract_mean, const RowOut& o,
+                               cudaStream_t s) {
   const size_t smem = (size_t)n_pix * sizeof(float);
-  EBSD_CUDA_CHECK(cudaFuncSetAttribute(k_project, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
-  const int grid = row_grid(n_rows, smem, (const void*)k_project);
-  k_project<<<grid, kRowThreads, smem, as_stream(stream)>>>(
-      master_pattern, mp_h, mp_w2, rays_soa, n_pix, reinterpret_cast<const float4*>(quats), n_rows,
-      subtract_mean, o);
+  const auto fn = k_prep<T, THREADS>;
+  EBSD_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int grid = row_grid(n_rows, smem, (const void*)fn, THREADS);
+  const int vec4 = binning == 1 && !pix_index && n_pix % 4 == 0 && pattern_stride % 4 == 0 &&
+                   reinterpret_cast<uintptr_t>(patterns) % (4 * sizeof(T)) == 0;
+  fn<<<grid, THREADS, smem, s>>>(patterns, n_rows, height, width, pattern_stride, binning, pix_index, n_pix,
+                                 1.0 / n_pix, vec4, subtract_mean, o);
   EBSD_LAUNCH_CHECK();
   return 0;
 }
@@ -260,13 +462,14 @@ template <typename T>
 static int launch_prep(const T* patterns, int64_t n_rows, int height, int width, int64_t pattern_stride,
                        int binning, const int32_t* pix_index, int n_pix, int subtract_mean, const RowOut& o,
                        void* stream) {
-  const size_t smem = (size_t)n_pix * sizeof(float);
-  EBSD_CUDA_CHECK(cudaFuncSetAttribute(k_prep<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int grid = row_grid(n_rows, smem, (const void*)k_prep<T>);
-  k_prep<T><<<grid, kRowThreads, smem, as_stream(stream)>>>(patterns, n_rows, height, width, pattern_stride,
-                                                           binning, pix_index, n_pix, subtract_mean, o);
-  EBSD_LAUNCH_CHECK();
-  return 0;
+  // Threads for a row: enough CTAs on an SM to keep HBM busy, enough threads
+  // for a long row. 60^2 px: 128 threads 6.03, 256 5.18 TB/s; 80^2 (e4m3):
+  // 5.34, 5.96; 128^2: 256 threads 5.44, 512 5.12; 160^2: 4.88, 5.31.
+#define EBSD_PREP(THREADS)                                                                                       \
+  launch_prep_threads<T, THREADS>(patterns, n_rows, height, width, pattern_stride, binning, pix_index, n_pix, \
+                                  subtract_mean, o, as_stream(stream))
+  return n_pix <= 4096 ? EBSD_PREP(128) : n_pix <= 16384 ? EBSD_PREP(256) : EBSD_PREP(512);
+#undef EBSD_PREP
 }
 
 extern "C" int ebsd_prep_patterns_typed(const void* patterns, int pattern_dtype, int64_t n_rows, int height,

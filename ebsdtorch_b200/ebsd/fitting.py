@@ -238,13 +238,15 @@ def _search_dft(mp_t, padded, quats, pix64, z_vals, tilt, sec_tilt, det, bs, bat
     sub = max(1, min(bs, n_dict, MAX_SIM_BYTES // (hp * wp * 4)))
     sims = torch.empty((sub, hp * wp), dtype=torch.float32, device=dev)
     spec = torch.empty((sub, spec_len), dtype=torch.float32, device=dev)
+    quads = kernels.sampling_quads(mp_t)
     for zi in range(len(z_vals)):
         rays = _rays_soa(pix64, float(z_vals[zi]), tilt, sec_tilt, det, dev)
         for j in range(0, n_dict, bs):
             j_end = min(j + bs, n_dict)
             for s in range(j, j_end, sub):
                 n = min(sub, j_end - s)
-                kernels.project(mp_t, rays, quats[s:s + n], RowBuffers(f32=sims[:n]), subtract_mean=False)
+                kernels.project(mp_t, rays, quats[s:s + n], RowBuffers(f32=sims[:n]), subtract_mean=False,
+                               quads=quads)
                 call("ebsd_pcfit_spectra", ptr(sims), hp * wp, n, hp, wp, ptr(tables), ptr(spec), ptr(status), stream)
                 call("ebsd_pcfit_xcorr_max", ptr(spec), n, ptr(terms), B, hp, wp, ptr(tables), ptr(keys),
                      (s - j) if batch_local else s, ptr(status), stream)
@@ -265,13 +267,15 @@ def _search_fft(mp_t, padded, quats, pix64, z_vals, tilt, sec_tilt, det, bs, bat
     wf = wp // 2 + 1
     sub = max(1, min(bs, MAX_PRODUCT_BYTES // (B * hp * wf * 8)))
     sims = torch.empty((min(sub, n_dict), hp * wp), dtype=torch.float32, device=dev)
+    quads = kernels.sampling_quads(mp_t)
     for zi in range(len(z_vals)):
         rays = _rays_soa(pix64, float(z_vals[zi]), tilt, sec_tilt, det, dev)
         for j in range(0, n_dict, bs):
             j_end = min(j + bs, n_dict)
             for s in range(j, j_end, sub):
                 n = min(sub, j_end - s)
-                kernels.project(mp_t, rays, quats[s:s + n], RowBuffers(f32=sims[:n]), subtract_mean=False)
+                kernels.project(mp_t, rays, quats[s:s + n], RowBuffers(f32=sims[:n]), subtract_mean=False,
+                               quads=quads)
                 spec = torch.fft.rfft2(sims[:n].view(n, hp, wp))
                 corr = torch.fft.irfft2(spec[:, None] * pat_fft[None], s=(hp, wp)).contiguous()
                 base = (s - j) if batch_local else s

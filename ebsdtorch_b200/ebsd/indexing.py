@@ -407,15 +407,16 @@ def pca_dictionary_index_orientations(
                     sample_ori_fz_laue_angle(mp.laue_group, dictionary_resolution_index_deg, dev)
                 del ori_learn
             proj = _Projector(comps)
+            quads = kernels.sampling_quads(mp_t)
             n_comp = comps.shape[0]
             pats = _pattern_source(experiment_patterns, dev)
             qfill_full = _query_fill(pats, virtual_binning, pix_index, P, subtract, dev)
 
-            def fill_dict(d0, d1, bufs, mp_t=mp_t, rays=rays, ori=ori, proj=proj):
+            def fill_dict(d0, d1, bufs, mp_t=mp_t, quads=quads, rays=rays, ori=ori, proj=proj):
                 for s0 in range(d0, d1, sub_chunk):
                     s1 = min(d1, s0 + sub_chunk)
                     X = torch.empty((s1 - s0, P), dtype=torch.float32, device=dev)
-                    kernels.project(mp_t, rays, ori[s0:s1], RowBuffers(f32=X), subtract_mean=True)
+                    kernels.project(mp_t, rays, ori[s0:s1], RowBuffers(f32=X), subtract_mean=True, quads=quads)
                     Y = bufs.f32[s0 - d0:s1 - d0] if bufs.f32 is not None else torch.empty(
                         (s1 - s0, n_comp), dtype=torch.float32, device=dev)
                     proj(X, Y)

@@ -114,6 +114,15 @@ int ebsd_project_dictionary(const float* master_pattern, int mp_h, int mp_w2, co
                             int n_pix, const float* quats, int64_t n_rows, int subtract_mean,
                             float* out_f32, int64_t ld_f32, void* out_lp, int lp_dtype, int64_t ld_lp,
                             float* out_norm, float* out_lp_scale, void* stream);
+/* The same rows from a gather table of the master pattern: quads holds, for
+ * every pixel (y, x), the values at (y, x), (y, x + 1), (y + 1, x) and
+ * (y + 1, x + 1), clamped to the border (mp_h * mp_w2 * 4 floats, 16-byte
+ * aligned, filled by ebsd_sampling_quads). A sample is then one 16-byte gather. */
+int ebsd_sampling_quads(const float* master_pattern, int mp_h, int mp_w2, float* quads, void* stream);
+int ebsd_project_dictionary_quads(const float* quads, int mp_h, int mp_w2, const float* rays_soa, int n_pix,
+                                  const float* quats, int64_t n_rows, int subtract_mean, float* out_f32,
+                                  int64_t ld_f32, void* out_lp, int lp_dtype, int64_t ld_lp, float* out_norm,
+                                  float* out_lp_scale, void* stream);
 
 /* ---- A8: pattern preparation ----------------------------------------------
  * Replaces ExperimentPatterns.get_patterns (experiment_pats.py:318-346:
