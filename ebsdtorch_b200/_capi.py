@@ -67,6 +67,8 @@ SIGNATURES = {
     "ebsd_clahe": (i32, [vp, i64, i32, i32, i64, vp, i32, f32, i32, i32, i32, i32, vp, i64, vp]),
     "ebsd_nlpar_dists": (i32, [vp, i32, i32, i32, i64, i32, vp, i32, i32, i32, vp, vp]),
     "ebsd_nlpar_average": (i32, [vp, i32, i32, i32, i64, i32, vp, i32, i32, i32, vp, i32, vp, i64, vp]),
+    "ebsd_nlpar_dists_window": (i32, [vp, i32, i32, i32, i64, i32, vp, i32, vp, vp]),
+    "ebsd_nlpar_average_window": (i32, [vp, i32, i32, i32, i64, i32, vp, i32, vp, vp, i64, vp]),
     "ebsd_nlpar_workspace_bytes": (sz, [i32, i32]),
     "ebsd_pcfit_prep": (i32, [vp, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp]),
     "ebsd_pcfit_reduce": (i32, [vp, i32, i32, i32, i32, i64, vp, vp, vp]),
@@ -110,7 +112,8 @@ LAUNCHES_PER_CALL = {
     "ebsd_disori_angle": 1, "ebsd_match_topk_noalloc": 2, "ebsd_zh_to_qu": 1, "ebsd_qu_to_zh": 1,
     "ebsd_cell_to_row": 2, "ebsd_local_search": 1, "ebsd_refine_grid": 1,
     "ebsd_pattern_mean": 2, "ebsd_subtract_pattern": 1, "ebsd_normalize_patterns": 1, "ebsd_clahe": 1,
-    "ebsd_nlpar_dists": 1, "ebsd_nlpar_average": 1, "ebsd_nlpar_weights": 14,
+    "ebsd_nlpar_dists": 1, "ebsd_nlpar_average": 1,
+    "ebsd_nlpar_dists_window": 1, "ebsd_nlpar_average_window": 1, "ebsd_nlpar_weights": 14,
     "ebsd_pcfit_prep": 1, "ebsd_pcfit_reduce": 1, "ebsd_pcfit_xcorr_tables": 1, "ebsd_pcfit_spectra": 1,
     "ebsd_pcfit_pattern_terms": 1, "ebsd_pcfit_xcorr_max": 1, "ebsd_pcfit_fold": 1,
     "ebsd_rot6d_sym_loss": 1, "ebsd_cnn_im2col": 1, "ebsd_cnn_col2im": 1, "ebsd_cnn_bias_act": 1,

@@ -8,8 +8,8 @@
 // do_nlpar), ebsdtorch/preprocessing/clahe.py:17-130 and
 // ebsdtorch/preprocessing/nlpar.py:19-192 (Brewick et al. 2019). Every pass
 // here is an image pass over FP32 patterns: HBM-bound (mean, subtract,
-// normalise, CLAHE) or shared-memory-bound (the NLPAR window passes, whose
-// scan tile and halo are staged in shared memory once per pixel chunk).
+// normalise, CLAHE) or bound on the SM (the NLPAR window passes, whose scan
+// tile and halo are staged in shared memory once per pixel chunk).
 #include <algorithm>
 #include <climits>
 
@@ -405,216 +405,381 @@ __global__ void __launch_bounds__(kClaheThreads) k_clahe(const ClaheArgs a) {
 
 // --------------------------------------------------------------------- NLPAR
 
-constexpr int kNlTile = 8;          // 8 x 8 scan points per CTA
-constexpr int kNlChunk = 32;        // pattern pixels per shared-memory chunk
-constexpr int kNlPitch = 24;        // row pitch of the staged tile + halo (side <= 22)
+constexpr int kNlTile = 8;          // scan points per row segment (and rows) of an averaging CTA
 constexpr int kNlMaxRad = 7;
-constexpr int kNlThreads = 256;
-constexpr int kNlMaxOffsets = 128;  // offsets per launch
-constexpr int kNlPairs = kNlMaxOffsets / (kNlThreads / (kNlTile * kNlTile));  // 32 per thread
+constexpr int kNlMaxCells = (2 * kNlMaxRad + 1) * (2 * kNlMaxRad + 1);
+constexpr int kNlMaxOffsets = kNlMaxCells;  // offsets per launch
+constexpr int kNlBlockOffsets = 128;        // of the entry points that take a block of offsets
 
-// Words per staged pixel plane: odd, so the 32 pixels a warp stores land in
-// distinct banks; with the pitch of 24 the 4 x 8 scan points a warp reads at
-// one offset land in distinct banks as well.
-__host__ __device__ constexpr int nl_plane(int halo) { return (kNlTile + 2 * halo) * kNlPitch + 1; }
-
-constexpr int kNlMaxRows = (kNlTile + 2 * kNlMaxRad) * (kNlTile + 2 * kNlMaxRad);
-
-// Per CTA, once: for each row (yy, xx) of the staged tile + halo, the scan
-// point it holds (-1 outside the scan) and its shared-memory offset.
-template <int HALO>
-__device__ __forceinline__ void nl_rows(int* src_s, int* dst_s, int hs, int ws, int y0, int x0) {
-  constexpr int side = kNlTile + 2 * HALO;
-  for (int r = threadIdx.x; r < side * side; r += blockDim.x) {
-    const int yy = r / side, xx = r - (r / side) * side;
-    const int y = y0 - HALO + yy, x = x0 - HALO + xx;
-    src_s[r] = (y >= 0 && y < hs && x >= 0 && x < ws) ? y * ws + x : -1;
-    dst_s[r] = yy * kNlPitch + xx;
-  }
+// Two FP32 values in one 64-bit register pair: the packed FP32 instructions
+// issue two lanes' worth of FADD / FFMA at a time, each value rounded as usual.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
 }
 
-// T[q * plane + yy * pitch + xx] = data[point (y0 - halo + yy, x0 - halo + xx), p0 + q]
-// by 4-byte cp.async (lane = pixel q, one row per warp and step); zero
-// outside the scan (the reference zero-pads the data, nlpar.py:56-61) and
-// beyond the last pixel. Completes before return.
-template <int HALO>
-__device__ __forceinline__ void nl_load_chunk(float* T, const float* __restrict__ data, int64_t ld,
-                                              const int* src_s, const int* dst_s, int p0, int np) {
-  constexpr int side = kNlTile + 2 * HALO, plane = nl_plane(HALO);
-  static_assert(kNlChunk == 32, "one warp lane per pixel of the chunk");
-  const int q = threadIdx.x & 31;
-  for (int row = threadIdx.x >> 5; row < side * side; row += blockDim.x >> 5) {
-    const int src = src_s[row];
-    float* dst = T + q * plane + dst_s[row];
-    if (src >= 0 && q < np)
-      cp_async4(dst, data + (int64_t)src * ld + p0 + q);
-    else
-      *dst = 0.f;
-  }
-  cp_async_commit();
-  cp_async_wait<0>();
-}
+// The window passes stage scan points in shared memory, kNlPix pixels of each
+// at a time, several chunks ahead (cp.async); a lane owns pixels 2 lane and
+// 2 lane + 1 of each half of a chunk.
+constexpr int kNlPix = 64;
 
-// Offsets of one launch as shared-memory displacements; an offset outside
-// [-halo, halo]^2 reads the point itself and is flagged (its results are NaN).
-__device__ __forceinline__ void nl_load_offsets(int* off_s, unsigned char* bad_s, const int* __restrict__ offsets,
-                                                int o0, int n_off, int halo) {
-  for (int o = threadIdx.x; o < n_off; o += blockDim.x) {
-    const int di = offsets[2 * (o0 + o)], dj = offsets[2 * (o0 + o) + 1];
-    const bool ok = di >= -halo && di <= halo && dj >= -halo && dj <= halo;
-    off_s[o] = ok ? di * kNlPitch + dj : 0;
-    bad_s[o] = ok ? 0 : 1;
-  }
-}
-
-// dists[pt, o0 + o] = sum_p (x[pt + off[o]] - x[pt])^2. Thread: one scan
-// point (tid % 64) and the offsets o = tid / 64 + 4 j (a warp shares o); per
-// chunk the point's own 32 values sit in registers and each offset costs one
-// shared-memory load (immediate offset) per pixel.
-template <int HALO>
-__global__ void __launch_bounds__(kNlThreads, 3) k_nlpar_dists(const float* __restrict__ data, int hs, int ws,
-                                                           int n_pix, int64_t ld, const int* __restrict__ offsets,
-                                                           int o0, int n_off, int per_group, int n_off_total,
-                                                           float* __restrict__ dists) {
-  constexpr int plane = nl_plane(HALO);
-  extern __shared__ __align__(16) float T[];
-  __shared__ int off_s[kNlMaxOffsets];
-  __shared__ unsigned char bad_s[kNlMaxOffsets];
-  __shared__ int src_s[kNlMaxRows], dst_s[kNlMaxRows];
-  // this CTA's group of offsets (blockIdx.y) within the launch's block
-  o0 += blockIdx.y * per_group;
-  n_off = min(per_group, n_off - (int)blockIdx.y * per_group);
-  const int tiles_x = (ws + kNlTile - 1) / kNlTile;
-  const int y0 = (blockIdx.x / tiles_x) * kNlTile, x0 = (blockIdx.x % tiles_x) * kNlTile;
-  const int pt = threadIdx.x % (kNlTile * kNlTile), ob = threadIdx.x / (kNlTile * kNlTile);
-  const int self = (pt / kNlTile + HALO) * kNlPitch + pt % kNlTile + HALO;
-  const int nj = (n_off - ob + 3) / 4;  // offsets of this thread
-  nl_load_offsets(off_s, bad_s, offsets, o0, n_off, HALO);
-  nl_rows<HALO>(src_s, dst_s, hs, ws, y0, x0);
-  float acc[kNlPairs];
-#pragma unroll
-  for (int j = 0; j < kNlPairs; ++j) acc[j] = 0.f;
-  for (int p0 = 0; p0 < n_pix; p0 += kNlChunk) {
-    __syncthreads();
-    nl_load_chunk<HALO>(T, data, ld, src_s, dst_s, p0, min(kNlChunk, n_pix - p0));
-    __syncthreads();
-    // two halves of 16 pixels keep 16 own values in registers (3 CTAs per SM)
-#pragma unroll 1
-    for (int h = 0; h < kNlChunk; h += kNlChunk / 2) {
-      const float* Th = T + h * plane;
-      float sv[kNlChunk / 2];
-#pragma unroll
-      for (int q = 0; q < kNlChunk / 2; ++q) sv[q] = Th[q * plane + self];
-#pragma unroll
-      for (int j = 0; j < kNlPairs; ++j) {
-        if (j < nj) {
-          const float* b = Th + self + off_s[ob + 4 * j];
-          float a = acc[j];
-#pragma unroll
-          for (int q = 0; q < kNlChunk / 2; ++q) {
-            const float e = b[q * plane] - sv[q];
-            a = fmaf(e, e, a);
-          }
-          acc[j] = a;
-        }
-      }
+// T[i * kNlPix + q] = pixel p0 + q of staged point i, the pattern at
+// data + src[i], or zeros where src[i] is negative (the reference pads the scan
+// with zeros) and beyond the last pixel. VEC: 16-byte copies; a thread copies
+// the same pixels of every point it takes.
+template <bool VEC, int POINTS, int THREADS>
+__device__ __forceinline__ void nl_stage(float* T, const float* __restrict__ data, const int64_t* src, int p0,
+                                         int n_pix) {
+  constexpr int kBytes = VEC ? 16 : 4, kPer = kNlPix * 4 / kBytes;
+  static_assert(THREADS % 32 == 0 && kNlPix % 32 == 0, "whole warps per point");
+  constexpr int kStep = THREADS >= kPer ? THREADS / kPer : 1;  // points per pass (whole points only)
+  constexpr int kUsed = kStep * kPer;
+  const int q = (int)threadIdx.x % kPer, p = p0 + q * (kBytes / 4);
+  const float* base = data + p;
+  uint32_t dst = smem_u32(T + ((int)threadIdx.x / kPer) * kNlPix) + q * kBytes;
+  if ((int)threadIdx.x < kUsed) {
+#pragma unroll 4
+    for (int i = (int)threadIdx.x / kPer; i < POINTS; i += kStep, dst += kStep * kNlPix * 4) {
+      const int64_t o = src[i];
+      const bool ok = o >= 0 && p < n_pix;
+      const float* g = ok ? base + o : data;
+      if constexpr (VEC)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(g), "r"(ok ? 16 : 0) : "memory");
+      else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(g), "r"(ok ? 4 : 0) : "memory");
     }
   }
-  const int y = y0 + pt / kNlTile, x = x0 + pt % kNlTile;
-  if (y >= hs || x >= ws) return;
+}
+
+__device__ __forceinline__ f32x2 nl_px(const float* point, int lane) {
+  return reinterpret_cast<const f32x2*>(point)[lane];
+}
+
+// Shape of the distance kernel for a window radius: PT scan points of one row
+// per warp, ROWS rows and all H + 1 row offsets of the half window per CTA,
+// STAGES chunks in flight. Registers hold PT (2 H + 1) packed accumulators, so
+// PT is halved for wide windows.
+template <int H>
+struct NlShape {
+  static constexpr int PT = H <= 3 ? 8 : 4;
+  static constexpr int ROWS = H <= 1 ? 6 : H == 2 ? 4 : H <= 4 ? 3 : H <= 6 ? 2 : 1;
+  static constexpr int WARPS = ROWS * (H + 1);
+  static constexpr int THREADS = 32 * WARPS;
+  static constexpr int SIDE = PT + 2 * H, POINTS = (ROWS + H) * SIDE;
+  static constexpr int STAGES = 4;
+  static constexpr size_t SMEM = (size_t)STAGES * POINTS * kNlPix * sizeof(float);
+};
+
+// v[i] of 32 values summed over the warp's lanes; lane i gets value i.
+__device__ __forceinline__ float transpose_sum(float (&v)[32], int lane) {
 #pragma unroll
-  for (int j = 0; j < kNlPairs; ++j) {
-    const int o = ob + 4 * j;
-    if (o < n_off) dists[((int64_t)y * ws + x) * n_off_total + o0 + o] = bad_s[o] ? NAN : acc[j];
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const float send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  return v[0];
+}
+
+// The (di, dj) -> offset lookup of one launch's offsets: first offset of a
+// window cell (-1: none), the next offset of the same cell, and whether any
+// offset lies outside the window.
+struct NlMap {
+  short first[kNlMaxCells];
+  short next[kNlMaxOffsets];
+  signed char di[kNlMaxOffsets], dj[kNlMaxOffsets];
+  int any_bad;
+};
+
+template <int H>
+__device__ __forceinline__ void nl_map(NlMap& m, const int* __restrict__ offsets, int o0, int n_off) {
+  constexpr int w2 = 2 * H + 1;
+  for (int c = threadIdx.x; c < w2 * w2; c += blockDim.x) m.first[c] = -1;
+  if (threadIdx.x == 0) m.any_bad = 0;
+  __syncthreads();
+  for (int o = threadIdx.x; o < n_off; o += blockDim.x) {
+    const int di = offsets[2 * (o0 + o)], dj = offsets[2 * (o0 + o) + 1];
+    const bool ok = di >= -H && di <= H && dj >= -H && dj <= H;
+    m.di[o] = (signed char)(ok ? di : 127);
+    m.dj[o] = (signed char)(ok ? dj : 127);
+    m.next[o] = -1;
+    if (!ok) m.any_bad = 1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int o = n_off - 1; o >= 0; --o) {
+      if (m.di[o] == 127) continue;
+      short& f = m.first[(m.di[o] + H) * w2 + m.dj[o] + H];
+      m.next[o] = f;
+      f = (short)o;
+    }
+  }
+  __syncthreads();
+}
+
+// One chunk of one warp's pairs: ZERO (row offset 0) the offsets dj = 0..H and
+// the squared norms, else dj = -H..H. own: the staged row of the warp's points,
+// starting at column -H; nb: the row dy below it.
+template <int H, bool ZERO, int N>
+__device__ __forceinline__ void nl_pairs(f32x2 (&acc)[N], const float* own, const float* nb, int lane) {
+  constexpr int PT = NlShape<H>::PT;
+  f32x2 c[PT];  // the points, negated
+#pragma unroll
+  for (int j = 0; j < PT; ++j) c[j] = nl_px(own + (j + H) * kNlPix, lane) ^ 0x8000000080000000ull;
+#pragma unroll
+  for (int k = ZERO ? 0 : -H; k < PT + H; ++k) {
+    const f32x2 v = nl_px(nb + (k + H) * kNlPix, lane);
+#pragma unroll
+    for (int j = 0; j < PT; ++j) {
+      const int dj = k - j;
+      if (dj < (ZERO ? 0 : -H) || dj > H) continue;
+      f32x2& s = acc[(ZERO ? dj : dj + H) * PT + j];
+      const f32x2 e = add2(v, c[j]);
+      s = fma2(e, e, s);
+    }
+    if (ZERO && k < PT) {
+      f32x2& s = acc[(H + 1) * PT + (k < PT && k >= 0 ? k : 0)];
+      s = fma2(v, v, s);
+    }
   }
 }
 
-// out[pt] (+)= sum_o w[pt, o0 + o] x[pt + off[o]]. Warp w: the 8 scan
-// points of tile row w, lane = pattern pixel of the chunk. The offsets are
-// walked by window row (di) and column (dj): for each di the warp loads the
-// 8 + 2 halo values of that row of the staged tile once, and every dj of the
-// row reuses them (8 FMAs per offset, two float4 weight loads). Each (di, dj)
-// may appear at most once per call; an offset outside the window makes the
-// outputs NaN.
-template <int HALO>
-__global__ void __launch_bounds__(kNlThreads) k_nlpar_average(const float* __restrict__ data, int hs, int ws,
+// dists[pt, o0 + o] = sum_p (x[pt + off[o]] - x[pt])^2. A distance belongs to
+// both points of a pair, so only the half window (di, dj) >= (0, 0) is
+// computed and each sum is stored twice; offsets that leave the scan (zeros
+// there) get the point's squared norm. Warp: PT points of one row against row
+// offset di; lanes: pattern pixels, so the pixels of a point are read once
+// from shared memory for all column offsets, two packed operations per pair
+// and pixel pair. Each lane sums its own pixels, the lanes are added at the end
+// (so the sums are also closer to 64 bits, 5e-8 against 1e-6).
+// Near the FP32 pipe's bound for wide windows and large scans: 65,536 patterns
+// of 60^2 px, k_rad 3: 2.70 -> 1.00 ms; 2,867 of 128^2 px, k_rad 5: 4.54 ->
+// 0.61 ms; 36,000 of 40^2, k_rad 1: 0.40 -> 0.10 ms. Bounded before by one
+// shared-memory load a pair and pixel, and by 256-thread CTAs of 64 points that
+// left a small scan on a third of the SMs.
+template <int H, bool VEC>
+__global__ void __launch_bounds__(NlShape<H>::THREADS, 1)
+    k_nlpar_dists(const float* __restrict__ data, int hs, int ws, int n_pix, int64_t ld,
+                  const int* __restrict__ offsets, int o0, int n_off, int n_off_total, float* __restrict__ dists) {
+  using S = NlShape<H>;
+  constexpr int PT = S::PT, w2 = 2 * H + 1;
+  constexpr int N = PT * (w2 > H + 2 ? w2 : H + 2), NB = (N + 31) / 32;
+  extern __shared__ __align__(16) float T[];
+  __shared__ NlMap map;
+  __shared__ int64_t src[S::POINTS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int segs = (ws + PT - 1) / PT;
+  const int y0 = (int)(blockIdx.x / segs) * S::ROWS, x0 = (int)(blockIdx.x % segs) * PT;
+  const int ry = wid / (H + 1), dy = wid % (H + 1), y = y0 + ry;
+  for (int i = threadIdx.x; i < S::POINTS; i += S::THREADS) {
+    const int py = y0 + i / S::SIDE, px = x0 - H + i % S::SIDE;
+    src[i] = py < hs && px >= 0 && px < ws ? ((int64_t)py * ws + px) * ld : -1;
+  }
+  nl_map<H>(map, offsets, o0, n_off);  // synchronises
+  const int n_chunks = (n_pix + kNlPix - 1) / kNlPix;
+#pragma unroll
+  for (int c = 0; c < S::STAGES - 1; ++c) {
+    if (c < n_chunks)
+      nl_stage<VEC, S::POINTS, S::THREADS>(T + c * S::POINTS * kNlPix, data, src, c * kNlPix, n_pix);
+    cp_async_commit();
+  }
+  f32x2 acc[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) acc[i] = 0ull;
+  for (int c = 0; c < n_chunks; ++c) {
+    cp_async_wait<S::STAGES - 2>();
+    __syncthreads();
+    const int ahead = c + S::STAGES - 1;
+    if (ahead < n_chunks)
+      nl_stage<VEC, S::POINTS, S::THREADS>(T + (ahead % S::STAGES) * S::POINTS * kNlPix, data, src, ahead * kNlPix,
+                                           n_pix);
+    cp_async_commit();
+    const float* own = T + ((c % S::STAGES) * S::POINTS + ry * S::SIDE) * kNlPix;
+    if (dy == 0)
+      nl_pairs<H, true>(acc, own, own, lane);
+    else
+      nl_pairs<H, false>(acc, own, own + dy * S::SIDE * kNlPix, lane);
+  }
+  cp_async_wait<0>();
+  if (y >= hs) return;
+
+  const int n_val = dy == 0 ? PT * (H + 2) : PT * w2;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      v[i] = 0.f;
+      if (32 * b + i < N) {
+        const float2 s = unpack2(acc[32 * b + i < N ? 32 * b + i : 0]);
+        v[i] = s.x + s.y;
+      }
+    }
+    const float val = transpose_sum(v, lane);
+    const int i = 32 * b + lane, t = i / PT, px = x0 + i % PT;
+    if (i >= n_val || px >= ws) continue;
+    const int64_t pt = (int64_t)y * ws + px;
+    if (dy == 0 && t == H + 1) {
+      // offsets out of the scan: the neighbour is zero; out of the window: NaN
+      if (px >= H && px + H < ws && y >= H && y + H < hs && !map.any_bad) continue;
+      for (int o = 0; o < n_off; ++o) {
+        const bool bad = map.di[o] == 127;
+        const int qy = y + map.di[o], qx = px + map.dj[o];
+        if (bad || qy < 0 || qy >= hs || qx < 0 || qx >= ws) dists[pt * n_off_total + o0 + o] = bad ? NAN : val;
+      }
+      continue;
+    }
+    const int dj = dy == 0 ? t : t - H, qx = px + dj, qy = y + dy;
+    if (qx < 0 || qx >= ws || qy >= hs) continue;
+    const int64_t q = (int64_t)qy * ws + qx;
+    for (int o = map.first[(dy + H) * w2 + dj + H]; o >= 0; o = map.next[o]) dists[pt * n_off_total + o0 + o] = val;
+    if (q != pt)
+      for (int o = map.first[(H - dy) * w2 + H - dj]; o >= 0; o = map.next[o]) dists[q * n_off_total + o0 + o] = val;
+  }
+}
+
+// Shape of the averaging kernel: warp = kNlTile points of one of ROWS rows.
+template <int H>
+struct NlAvg {
+  static constexpr int ROWS = H <= 5 ? 8 : 4, THREADS = 32 * ROWS;
+  static constexpr int SIDE = kNlTile + 2 * H, POINTS = (ROWS + 2 * H) * SIDE;
+  static constexpr size_t WEIGHTS = (size_t)(2 * H + 1) * SIDE * ROWS * kNlTile * sizeof(f32x2);
+  static constexpr size_t STAGE = (size_t)POINTS * kNlPix * sizeof(float);
+  static constexpr int STAGES = WEIGHTS + 3 * STAGE <= 224 * 1024 ? 3 : WEIGHTS + 2 * STAGE <= 224 * 1024 ? 2 : 1;
+  static constexpr size_t SMEM = WEIGHTS + STAGES * STAGE;
+};
+
+// out[pt] (+)= sum_o w[pt, o0 + o] x[pt + off[o]]. Warp: 8 scan points of one
+// row, lanes: pattern pixels. The window is walked by row di; a neighbour's
+// pixels are read from shared memory once and used for every point whose
+// window reaches it, one packed FFMA per weight and pixel pair. The weights
+// sit in shared memory as (w, w) pairs in the order of use: [di][neighbour
+// column][row][point]. Each (di, dj) may appear at most once per call; an
+// offset outside the window makes the outputs NaN. Bound by shared-memory reads
+// (the weights of a pixel pair): 65,536 patterns of 60^2 px, k_rad 3: 2.37 ->
+// 1.54 ms; 2,867 of 128^2 px, k_rad 5: 1.47 -> 0.78 ms.
+template <int H, bool VEC>
+__global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float* __restrict__ data, int hs, int ws,
                                                              int n_pix, int pix_per_split, int64_t ld,
                                                              const int* __restrict__ offsets, int o0, int n_off,
                                                              int n_off_total, const float* __restrict__ weights,
                                                              int accumulate, float* __restrict__ out,
                                                              int64_t ld_out) {
-  constexpr int plane = nl_plane(HALO);
-  constexpr int side = kNlTile + 2 * HALO, w2 = 2 * HALO + 1;
-  extern __shared__ __align__(16) float T[];
-  __shared__ int orow_s[(2 * kNlMaxRad + 1) * (2 * kNlMaxRad + 1)];  // (di, dj) -> offset of this call, or -1
+  using S = NlAvg<H>;
+  constexpr int side = S::SIDE, w2 = 2 * H + 1, PTS = S::ROWS * kNlTile;
+  extern __shared__ __align__(16) f32x2 w_s[];
+  float* T = reinterpret_cast<float*>(w_s + w2 * side * PTS);
   __shared__ int any_bad;
-  __shared__ int src_s[kNlMaxRows], dst_s[kNlMaxRows];
-  float* w_s = T + ((kNlChunk * plane + 3) & ~3);  // [o][64 points], 16-byte aligned
+  __shared__ int64_t src[S::POINTS];
   const int tiles_x = (ws + kNlTile - 1) / kNlTile;
-  const int y0 = (blockIdx.x / tiles_x) * kNlTile, x0 = (blockIdx.x % tiles_x) * kNlTile;
+  const int y0 = (blockIdx.x / tiles_x) * S::ROWS, x0 = (blockIdx.x % tiles_x) * kNlTile;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   // this CTA's range of pattern pixels (blockIdx.y); outputs are disjoint
   const int pix_begin = blockIdx.y * pix_per_split, pix_end = min(n_pix, pix_begin + pix_per_split);
-  for (int r = threadIdx.x; r < w2 * w2; r += blockDim.x) orow_s[r] = -1;
   if (threadIdx.x == 0) any_bad = 0;
-  nl_rows<HALO>(src_s, dst_s, hs, ws, y0, x0);
-  __syncthreads();
-  for (int o = threadIdx.x; o < n_off; o += blockDim.x) {
-    const int di = offsets[2 * (o0 + o)], dj = offsets[2 * (o0 + o) + 1];
-    if (di >= -HALO && di <= HALO && dj >= -HALO && dj <= HALO)
-      orow_s[(di + HALO) * w2 + dj + HALO] = o;
-    else
-      any_bad = 1;
+  for (int i = threadIdx.x; i < S::POINTS; i += S::THREADS) {
+    const int py = y0 - H + i / side, px = x0 - H + i % side;
+    src[i] = py >= 0 && py < hs && px >= 0 && px < ws ? ((int64_t)py * ws + px) * ld : -1;
   }
-  for (int t = threadIdx.x; t < kNlTile * kNlTile * n_off; t += blockDim.x) {
-    const int pt = t % (kNlTile * kNlTile), o = t / (kNlTile * kNlTile);
+  __syncthreads();
+  const int n_chunks = (pix_end - pix_begin + kNlPix - 1) / kNlPix;
+#pragma unroll
+  for (int c = 0; c < S::STAGES - 1; ++c) {
+    if (c < n_chunks)
+      nl_stage<VEC, S::POINTS, S::THREADS>(T + c * S::POINTS * kNlPix, data, src, pix_begin + c * kNlPix, pix_end);
+    cp_async_commit();
+  }
+  for (int i = threadIdx.x; i < w2 * side * PTS; i += S::THREADS) w_s[i] = 0ull;
+  __syncthreads();
+  for (int i = threadIdx.x; i < PTS * n_off; i += S::THREADS) {
+    const int o = i / PTS, pt = i % PTS;
+    const int di = offsets[2 * (o0 + o)], dj = offsets[2 * (o0 + o) + 1];
+    if (di < -H || di > H || dj < -H || dj > H) {
+      any_bad = 1;
+      continue;
+    }
     const int y = y0 + pt / kNlTile, x = x0 + pt % kNlTile;
-    w_s[t] = (y < hs && x < ws) ? weights[((int64_t)y * ws + x) * n_off_total + o0 + o] : 0.f;
+    const float w = y < hs && x < ws ? weights[((int64_t)y * ws + x) * n_off_total + o0 + o] : 0.f;
+    w_s[((di + H) * side + pt % kNlTile + dj + H) * PTS + pt] = pack2(w, w);
   }
   const int y = y0 + wid;
-  const float4* w4 = reinterpret_cast<const float4*>(w_s) + wid * 2;
-  for (int p0 = pix_begin; p0 < pix_end; p0 += kNlChunk) {
-    const int np = min(kNlChunk, pix_end - p0);
-    __syncthreads();
-    nl_load_chunk<HALO>(T, data, ld, src_s, dst_s, p0, np);
-    __syncthreads();
-    if (y >= hs) continue;
-    const float* rows = T + lane * plane + wid * kNlPitch;  // window row wid + (di + HALO)
-    float s[kNlTile];
-#pragma unroll
-    for (int k = 0; k < kNlTile; ++k) s[k] = 0.f;
-#pragma unroll 1
-    for (int a = 0; a < w2; ++a) {
-      const float* r = rows + a * kNlPitch;
-      float v[side];
-#pragma unroll
-      for (int x = 0; x < side; ++x) v[x] = r[x];
-#pragma unroll
-      for (int c = 0; c < w2; ++c) {
-        const int o = orow_s[a * w2 + c];
-        if (o < 0) continue;
-        const float4 wa = w4[o * (kNlTile * kNlTile / 4)], wb = w4[o * (kNlTile * kNlTile / 4) + 1];
-        s[0] = fmaf(wa.x, v[0 + c], s[0]);
-        s[1] = fmaf(wa.y, v[1 + c], s[1]);
-        s[2] = fmaf(wa.z, v[2 + c], s[2]);
-        s[3] = fmaf(wa.w, v[3 + c], s[3]);
-        s[4] = fmaf(wb.x, v[4 + c], s[4]);
-        s[5] = fmaf(wb.y, v[5 + c], s[5]);
-        s[6] = fmaf(wb.z, v[6 + c], s[6]);
-        s[7] = fmaf(wb.w, v[7 + c], s[7]);
-      }
+  for (int c = 0; c < n_chunks; ++c) {
+    const int p0 = pix_begin + c * kNlPix;
+    if constexpr (S::STAGES > 1) {
+      cp_async_wait<S::STAGES - 2>();
+      __syncthreads();
+      const int ahead = c + S::STAGES - 1;
+      if (ahead < n_chunks)
+        nl_stage<VEC, S::POINTS, S::THREADS>(T + (ahead % S::STAGES) * S::POINTS * kNlPix, data, src,
+                                             pix_begin + ahead * kNlPix, pix_end);
+      cp_async_commit();
+    } else {
+      __syncthreads();
+      nl_stage<VEC, S::POINTS, S::THREADS>(T, data, src, p0, pix_end);
+      cp_async_commit();
+      cp_async_wait<0>();
+      __syncthreads();
     }
-    if (lane < np) {
+    if (y >= hs) continue;
+    f32x2 s[kNlTile];
 #pragma unroll
-      for (int k = 0; k < kNlTile; ++k) {
-        if (x0 + k < ws) {
-          float* dp = out + ((int64_t)y * ws + x0 + k) * ld_out + p0 + lane;
-          const float val = any_bad ? NAN : s[k];
-          *dp = accumulate ? *dp + val : val;
+    for (int j = 0; j < kNlTile; ++j) s[j] = 0ull;
+    const float* row = T + ((c % S::STAGES) * S::POINTS + wid * side) * kNlPix;
+    const f32x2* wr = w_s + wid * kNlTile;
+#pragma unroll 1
+    for (int a = 0; a < w2; ++a, row += side * kNlPix, wr += side * PTS) {
+#pragma unroll
+      for (int k = 0; k < side; ++k) {
+        const f32x2 v = nl_px(row + k * kNlPix, lane);
+        const ulonglong2* w4 = reinterpret_cast<const ulonglong2*>(wr + k * PTS);
+#pragma unroll
+        for (int j = 0; j < kNlTile; j += 2) {
+          if (k - j < 0 || k - j - 1 > 2 * H) continue;
+          const ulonglong2 w = w4[j / 2];
+          if (k - j <= 2 * H) s[j] = fma2(w.x, v, s[j]);
+          if (k - j - 1 >= 0) s[j + 1] = fma2(w.y, v, s[j + 1]);
         }
       }
     }
+#pragma unroll
+    for (int j = 0; j < kNlTile; ++j) {
+      if (x0 + j >= ws) break;
+      float* dp = out + ((int64_t)y * ws + x0 + j) * ld_out + p0 + 2 * lane;
+      float2 r = unpack2(s[j]);
+      if (any_bad) r.x = r.y = NAN;
+      if (VEC) {
+        if (p0 + 2 * lane < pix_end) {
+          float2* d = reinterpret_cast<float2*>(dp);
+          if (accumulate) r = make_float2(d->x + r.x, d->y + r.y);
+          *d = r;
+        }
+      } else {
+        if (p0 + 2 * lane < pix_end) dp[0] = accumulate ? dp[0] + r.x : r.x;
+        if (p0 + 2 * lane + 1 < pix_end) dp[1] = accumulate ? dp[1] + r.y : r.y;
+      }
+    }
   }
+  cp_async_wait<0>();
 }
 
 // ---- NLPAR weights (nlpar.py:122-183): noise estimate, normalised
@@ -741,46 +906,37 @@ __global__ void k_nlpar_softmax(float* __restrict__ w, int hs, int ws, int K, co
   for (int o = lane; o < K; o += 32) r[o] = expf(r[o] - mx) / sum;
 }
 
-// Second grid dimension, so that small scans still fill the GPU: offset
-// groups (distances) or pixel ranges (average), each CTA writing disjoint
-// outputs. Aim for `waves` waves at the kernel's occupancy. A distance CTA
-// reloads the whole tile for fewer offsets, so distances split only to fill
-// one wave; the average splits its pixel range, which costs nothing extra.
-static int nl_splits(const void* func, size_t smem, int tiles, int max_splits, int waves) {
+// Pixel ranges of the average (second grid dimension), so that small scans
+// still fill the GPU: about `waves` waves at the kernel's occupancy.
+static int nl_splits(const void* func, int threads, size_t smem, int tiles, int max_splits, int waves) {
   int per_sm = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, kNlThreads, smem) != cudaSuccess || per_sm < 1)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, threads, smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   const int64_t want = (int64_t)waves * device_sm_count() * per_sm;
   return (int)std::max<int64_t>(1, std::min<int64_t>(max_splits, (want + tiles - 1) / tiles));
 }
 
-template <int HALO>
+template <int H, bool VEC>
 static int nl_launch(bool average, const float* data, int hs, int ws, int n_pix, int64_t ld, const int* offsets,
                      int o0, int n_off, int n_off_total, float* dists, const float* weights, int accumulate,
                      float* out, int64_t ld_out, cudaStream_t s) {
-  const int tiles = ceil_div(hs, kNlTile) * ceil_div(ws, kNlTile);
-  const size_t chunk_bytes = (size_t)kNlChunk * nl_plane(HALO) * sizeof(float);
   if (!average) {
-    EBSD_CUDA_CHECK(cudaFuncSetAttribute(k_nlpar_dists<HALO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)chunk_bytes));
-    // groups of at least 16 offsets
-    const int groups = nl_splits((const void*)k_nlpar_dists<HALO>, chunk_bytes, tiles, std::max(1, n_off / 16), 1);
-    const int per_group = ceil_div(n_off, groups);
-    const int n_groups = ceil_div(n_off, per_group);
-    k_nlpar_dists<HALO><<<dim3(tiles, n_groups), kNlThreads, chunk_bytes, s>>>(data, hs, ws, n_pix, ld, offsets, o0,
-                                                                              n_off, per_group, n_off_total, dists);
+    using S = NlShape<H>;
+    const auto fn = k_nlpar_dists<H, VEC>;
+    EBSD_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
+    fn<<<ceil_div(hs, S::ROWS) * ceil_div(ws, S::PT), S::THREADS, S::SMEM, s>>>(data, hs, ws, n_pix, ld, offsets, o0,
+                                                                               n_off, n_off_total, dists);
   } else {
-    const size_t smem = ((chunk_bytes + 15) & ~(size_t)15) + (size_t)kNlTile * kNlTile * n_off * sizeof(float);
-    EBSD_CUDA_CHECK(
-        cudaFuncSetAttribute(k_nlpar_average<HALO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // ranges of whole chunks, at least 4 chunks each
-    const int n_chunks = ceil_div(n_pix, kNlChunk);
-    const int splits = nl_splits((const void*)k_nlpar_average<HALO>, smem, tiles, std::max(1, n_chunks / 4), 3);
-    const int pix_per_split = ceil_div(n_chunks, splits) * kNlChunk;
-    const int n_splits = ceil_div(n_pix, pix_per_split);
-    k_nlpar_average<HALO><<<dim3(tiles, n_splits), kNlThreads, smem, s>>>(data, hs, ws, n_pix, pix_per_split, ld,
-                                                                         offsets, o0, n_off, n_off_total, weights,
-                                                                         accumulate, out, ld_out);
+    using S = NlAvg<H>;
+    const int tiles = ceil_div(hs, S::ROWS) * ceil_div(ws, kNlTile);
+    const auto fn = k_nlpar_average<H, VEC>;
+    EBSD_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
+    // ranges of whole chunks, at least 8 chunks each
+    const int n_chunks = ceil_div(n_pix, kNlPix);
+    const int splits = nl_splits((const void*)fn, S::THREADS, S::SMEM, tiles, std::max(1, n_chunks / 8), 3);
+    const int pix_per_split = ceil_div(n_chunks, splits) * kNlPix;
+    fn<<<dim3(tiles, ceil_div(n_pix, pix_per_split)), S::THREADS, S::SMEM, s>>>(
+        data, hs, ws, n_pix, pix_per_split, ld, offsets, o0, n_off, n_off_total, weights, accumulate, out, ld_out);
   }
   EBSD_LAUNCH_CHECK();
   return 0;
@@ -789,11 +945,16 @@ static int nl_launch(bool average, const float* data, int hs, int ws, int n_pix,
 static int nl_dispatch(bool average, const float* data, int hs, int ws, int n_pix, int64_t ld, int k_rad,
                        const int* offsets, int o0, int n_off, int n_off_total, float* dists, const float* weights,
                        int accumulate, float* out, int64_t ld_out, cudaStream_t s) {
+  // 16-byte accesses to every pattern
+  const bool vec = n_pix % 4 == 0 && ld % 4 == 0 && reinterpret_cast<uintptr_t>(data) % 16 == 0 &&
+                   (!average || (ld_out % 4 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0));
   switch (k_rad) {
-#define EBSD_NL_CASE(R)                                                                                          \
-  case R:                                                                                                        \
-    return nl_launch<R>(average, data, hs, ws, n_pix, ld, offsets, o0, n_off, n_off_total, dists, weights,      \
-                        accumulate, out, ld_out, s);
+#define EBSD_NL_CASE(R)                                                                                         \
+  case R:                                                                                                       \
+    return vec ? nl_launch<R, true>(average, data, hs, ws, n_pix, ld, offsets, o0, n_off, n_off_total, dists,   \
+                                    weights, accumulate, out, ld_out, s)                                        \
+               : nl_launch<R, false>(average, data, hs, ws, n_pix, ld, offsets, o0, n_off, n_off_total, dists,  \
+                                     weights, accumulate, out, ld_out, s);
     EBSD_NL_CASE(0)
     EBSD_NL_CASE(1)
     EBSD_NL_CASE(2)
@@ -909,13 +1070,14 @@ extern "C" int ebsd_clahe(const float* images, int64_t n, int height, int width,
 }
 
 static int nl_check(const float* data, int hs, int ws, int n_pix, int64_t ld, int halo, const int* offsets, int o0,
-                    int n_off, int n_off_total) {
+                    int n_off, int n_off_total, int max_off = kNlBlockOffsets) {
   EBSD_ARG_CHECK(data && offsets, "NLPAR: null pointer");
   EBSD_ARG_CHECK(hs >= 1 && ws >= 1 && n_pix >= 1 && ld >= n_pix, "NLPAR: bad sizes");
   EBSD_ARG_CHECK(halo >= 0 && halo <= kNlMaxRad, "NLPAR: kernel radius must be in [0, %d]", kNlMaxRad);
-  EBSD_ARG_CHECK(n_off >= 1 && n_off <= kNlMaxOffsets && o0 >= 0 && o0 + n_off <= n_off_total,
-                 "NLPAR: an offset block holds 1..%d offsets", kNlMaxOffsets);
-  EBSD_ARG_CHECK((int64_t)ceil_div(hs, kNlTile) * ceil_div(ws, kNlTile) <= INT_MAX, "NLPAR: scan too large");
+  EBSD_ARG_CHECK(n_off >= 1 && n_off <= max_off && o0 >= 0 && o0 + n_off <= n_off_total,
+                 "NLPAR: an offset block holds 1..%d offsets", max_off);
+  // the distance kernel's smallest tile: one row of four points
+  EBSD_ARG_CHECK((int64_t)hs * ceil_div(ws, 4) <= INT_MAX, "NLPAR: scan too large");
   return 0;
 }
 
@@ -935,6 +1097,24 @@ extern "C" int ebsd_nlpar_average(const float* data, int scan_h, int scan_w, int
   EBSD_ARG_CHECK(out != data, "NLPAR: the average cannot be written in place");
   return nl_dispatch(true, data, scan_h, scan_w, n_pix, ld, k_rad, offsets, o0, n_off, n_off_total, nullptr, weights,
                      accumulate, out, ld_out, as_stream(stream));
+}
+
+extern "C" int ebsd_nlpar_dists_window(const float* data, int scan_h, int scan_w, int n_pix, int64_t ld, int k_rad,
+                                       const int* offsets, int n_off, float* dists, void* stream) {
+  if (int rc = nl_check(data, scan_h, scan_w, n_pix, ld, k_rad, offsets, 0, n_off, n_off, kNlMaxOffsets)) return rc;
+  EBSD_ARG_CHECK(dists != nullptr, "NLPAR: null output");
+  return nl_dispatch(false, data, scan_h, scan_w, n_pix, ld, k_rad, offsets, 0, n_off, n_off, dists, nullptr, 0,
+                     nullptr, 0, as_stream(stream));
+}
+
+extern "C" int ebsd_nlpar_average_window(const float* data, int scan_h, int scan_w, int n_pix, int64_t ld, int k_rad,
+                                         const int* offsets, int n_off, const float* weights, float* out,
+                                         int64_t ld_out, void* stream) {
+  if (int rc = nl_check(data, scan_h, scan_w, n_pix, ld, k_rad, offsets, 0, n_off, n_off, kNlMaxOffsets)) return rc;
+  EBSD_ARG_CHECK(weights && out && ld_out >= n_pix, "NLPAR: bad output");
+  EBSD_ARG_CHECK(out != data, "NLPAR: the average cannot be written in place");
+  return nl_dispatch(true, data, scan_h, scan_w, n_pix, ld, k_rad, offsets, 0, n_off, n_off, nullptr, weights, 0, out,
+                     ld_out, as_stream(stream));
 }
 
 extern "C" size_t ebsd_nlpar_workspace_bytes(int scan_h, int scan_w) {

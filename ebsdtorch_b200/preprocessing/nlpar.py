@@ -3,9 +3,9 @@
 
 `nlpar` keeps the reference's signature and result. The two passes that read
 the patterns, the squared distances to every window neighbour and the
-weighted average, are CUDA kernels that stage an 8 x 8 tile of the scan plus
-its halo in shared memory once per 32-pixel chunk (`ebsd_nlpar_dists`,
-`ebsd_nlpar_average`). The per-point arithmetic between them follows the
+weighted average, are CUDA kernels that stage a tile of the scan plus its
+halo in shared memory, 64 pixels at a time (`ebsd_nlpar_dists_window`,
+`ebsd_nlpar_average_window`). The per-point arithmetic between them follows the
 reference's formulas in FP32 (`ebsd_nlpar_weights`): noise estimate from
 window offsets 1..8, normalised distances, the Newton fit of the global
 coefficient on offsets 0..8 (each iteration one launch whose last block
@@ -23,7 +23,6 @@ from .patterns import _stream, device_rows
 from .._device import on_data_device
 
 MAX_RADIUS = 7        # the kernels' halo limit
-OFFSETS_PER_CALL = 128
 
 
 def nlpar_offsets(k_rad: int) -> Tensor:
@@ -56,9 +55,7 @@ def nlpar(data: Tensor, k_rad: int = 5, coeff: float = 0.375, coeff_fit_tol: flo
     off_d = off.to(device=dev, dtype=torch.int32).contiguous()
 
     dists = torch.empty((hs * ws, K), dtype=torch.float32, device=dev)
-    for o0 in range(0, K, OFFSETS_PER_CALL):
-        call("ebsd_nlpar_dists", ptr(x), hs, ws, n_pix, x.stride(0), k_rad, ptr(off_d), o0,
-             min(OFFSETS_PER_CALL, K - o0), K, ptr(dists), stream)
+    call("ebsd_nlpar_dists_window", ptr(x), hs, ws, n_pix, x.stride(0), k_rad, ptr(off_d), K, ptr(dists), stream)
     # noise estimate, normalised distances, Newton fit of the coefficient
     # and the masked softmax, in place: dists becomes the weights
     ws_bytes = int(load().ebsd_nlpar_workspace_bytes(hs, ws))
@@ -68,7 +65,6 @@ def nlpar(data: Tensor, k_rad: int = 5, coeff: float = 0.375, coeff_fit_tol: flo
     weights = dists
 
     out = torch.empty_like(x)
-    for o0 in range(0, K, OFFSETS_PER_CALL):
-        call("ebsd_nlpar_average", ptr(x), hs, ws, n_pix, x.stride(0), k_rad, ptr(off_d), o0,
-             min(OFFSETS_PER_CALL, K - o0), K, ptr(weights), int(o0 > 0), ptr(out), out.stride(0), stream)
+    call("ebsd_nlpar_average_window", ptr(x), hs, ws, n_pix, x.stride(0), k_rad, ptr(off_d), K, ptr(weights), ptr(out),
+         out.stride(0), stream)
     return back(out).view(hs, ws, hp, wp)

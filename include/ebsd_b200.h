@@ -440,6 +440,12 @@ int ebsd_nlpar_dists(const float* data, int scan_h, int scan_w, int n_pix, int64
 int ebsd_nlpar_average(const float* data, int scan_h, int scan_w, int n_pix, int64_t ld, int k_rad,
                        const int* offsets, int o0, int n_off, int n_off_total, const float* weights, int accumulate,
                        float* out, int64_t ld_out, void* stream);
+/* Both passes over a whole window's offsets in one launch (up to 225, k_rad 7). */
+int ebsd_nlpar_dists_window(const float* data, int scan_h, int scan_w, int n_pix, int64_t ld, int k_rad,
+                            const int* offsets, int n_off, float* dists, void* stream);
+int ebsd_nlpar_average_window(const float* data, int scan_h, int scan_w, int n_pix, int64_t ld, int k_rad,
+                              const int* offsets, int n_off, const float* weights, float* out, int64_t ld_out,
+                              void* stream);
 /* The NLPAR weights between the two passes (nlpar.py:122-183), in place over
  * dists (scan_h * scan_w x n_off, offsets as above, n_off >= 9): noise
  * estimate sigma = sqrt(min(dists[:, 1..8]) / (2 n_pix)), normalised
