@@ -25,13 +25,14 @@ from __future__ import annotations
 
 from typing import List, Optional, Union
 
+import numpy as np
 import torch
 from torch import Tensor
 
 from .. import kernels
-from ..engine import Searcher, SearchConfig, default_budget, wave_query_tiles
+from ..engine import Searcher, SearchConfig, wave_query_tiles
 from ..kernels import RowBuffers, round_up
-from ..s2_and_so3.laue_fz_ori import sample_ori_fz_laue_angle
+from ..s2_and_so3.laue_fz_ori import FzOrientations, sample_ori_fz_laue_angle
 
 
 def _device(mp, device) -> torch.device:
@@ -64,22 +65,24 @@ def _similarity(distance_metric: str, similarity: str) -> str:
 
 
 def _unit_rays_soa(geometry, binning: int, signal_mask: Optional[Tensor], device) -> Tensor:
-    """(3, P') float32 unit rays of the masked, binned detector pixels."""
+    """(3, P') float32 unit rays of the masked, binned detector pixels. NumPy:
+    a few thousand pixels are a few ten microseconds on one core, where
+    PyTorch's CPU operators wake a pool of threads for each step."""
     coords = geometry.get_coords_sample_frame(binning=(binning, binning))
-    c = coords.detach().reshape(-1, 3).double().cpu()
-    c = c / c.norm(dim=-1, keepdim=True)
+    c = coords.detach().reshape(-1, 3).cpu().numpy().astype(np.float64)
+    c /= np.sqrt(np.einsum("ij,ij->i", c, c))[:, None]
     if signal_mask is not None:
-        m = signal_mask.reshape(-1).cpu().bool()
-        if m.numel() != c.shape[0]:
-            raise ValueError(f"signal_mask has {m.numel()} pixels but the binned detector has {c.shape[0]}")
+        m = signal_mask.reshape(-1).cpu().bool().numpy()
+        if m.size != c.shape[0]:
+            raise ValueError(f"signal_mask has {m.size} pixels but the binned detector has {c.shape[0]}")
         c = c[m]
-    return c.t().contiguous().float().to(device)
+    return torch.from_numpy(np.ascontiguousarray(c.T, dtype=np.float32)).to(device)
 
 
 def _pix_index(signal_mask: Optional[Tensor], device) -> Optional[Tensor]:
     if signal_mask is None:
         return None
-    return torch.nonzero(signal_mask.reshape(-1).cpu().bool()).reshape(-1).to(torch.int32).to(device)
+    return torch.from_numpy(np.flatnonzero(signal_mask.reshape(-1).cpu().bool().numpy()).astype(np.int32)).to(device)
 
 
 def _master_pattern_tensor(mp, binning: int, device) -> Tensor:
@@ -224,19 +227,19 @@ def dictionary_index_orientations(
                 # chunks of a few match waves, so each chunk's copy runs under the
                 # previous chunk's match and only the first copy is exposed
                 cfg.max_query_chunk = HOST_CHUNK_WAVES * wave_query_tiles(dev) * kernels.TILE_Q
-            ori = sample_ori_fz_laue_angle(mp.laue_group, dictionary_resolution_degrees, dev, permute=True)
+            grid = FzOrientations(mp.laue_group, dictionary_resolution_degrees, dev)
             rays = _unit_rays_soa(geometry, virtual_binning, signal_mask, dev)
             mp_t = _master_pattern_tensor(mp, virtual_binning, dev)
             pix_index = _pix_index(signal_mask, dev)
             n_pix = rays.shape[1]
             pats = _pattern_source(experiment_patterns, dev)
 
-            def fill_dict(d0, d1, bufs, mp_t=mp_t, rays=rays, ori=ori):
-                kernels.project(mp_t, rays, ori[d0:d1], bufs, subtract_mean=True)
+            def fill_dict(d0, d1, bufs, mp_t=mp_t, rays=rays, grid=grid):
+                kernels.project(mp_t, rays, grid.finish()[d0:d1], bufs, subtract_mean=True)
 
-            searcher = Searcher(ori.shape[0], n_q, n_pix, int(top_k_matches), cfg, dev)
+            searcher = Searcher(grid.n, n_q, n_pix, int(top_k_matches), cfg, dev)
             idx, val = searcher.run(fill_dict, _query_fill(pats, virtual_binning, pix_index, n_pix, subtract, dev))
-            _store(experiment_patterns, i, ori, idx, val, _metric_dtype(match_dtype))
+            _store(experiment_patterns, i, grid.finish(), idx, val, _metric_dtype(match_dtype))
     experiment_patterns.combine_indexing_results(higher_is_better=(distance_metric == "angular"))
 
 
@@ -432,9 +435,9 @@ def pca_dictionary_index_orientations(
                     proj(X, Y)
                     _finish_rows(Y, _slice(bufs, s0 - q0, s1 - q0))
 
-            budget = workspace_bytes or int(default_budget(dev) * 0.7)
             cfg = SearchConfig(precision=precision, rescore_k=rescore_k,
-                               similarity=_similarity(distance_metric, similarity), workspace_bytes=budget)
+                               similarity=_similarity(distance_metric, similarity), workspace_bytes=workspace_bytes,
+                               free_share=0.7)
             searcher = Searcher(ori.shape[0], n_q, n_comp, int(top_k_matches), cfg, dev)
             idx, val = searcher.run(fill_dict, fill_queries)
             if int(proj.status.item()) != 0:

@@ -74,6 +74,8 @@ class SearchConfig:
     rescore_k: int = 32
     similarity: str = "dot"
     workspace_bytes: Optional[int] = None
+    # share of the free memory the default budget may take
+    free_share: float = 1.0
     query_chunk: Optional[int] = None
     dict_chunk: Optional[int] = None
     # upper bound on the planned query chunk (host-resident patterns stream in
@@ -122,9 +124,14 @@ class RowSet:
         rows_pad = round_up(max(n_rows, 1), pad_rows)
         lp_t = LP_TORCH[lp_dtype]
         if storage is None:
-            self.lp = torch.zeros((rows_pad, self.k_pad), dtype=lp_t, device=device)
+            # the row producers write whole rows (zeros from n_pix to k_pad);
+            # rows beyond n_rows take part in the tensor-core tiles: zero them
+            self.lp = torch.empty((rows_pad, self.k_pad), dtype=lp_t, device=device)
             self.f32 = torch.empty((n_rows, n_pix), dtype=torch.float32, device=device) if keep_f32 else None
-            self.norm = torch.zeros(rows_pad, dtype=torch.float32, device=device)
+            self.norm = torch.empty(rows_pad, dtype=torch.float32, device=device)
+            if rows_pad > n_rows:
+                self.lp[n_rows:].zero_()
+                self.norm[n_rows:].zero_()
             self.lp_scale = torch.ones(rows_pad, dtype=torch.float32, device=device) \
                 if lp_dtype != kernels.DT_BF16 else None
             return
@@ -243,6 +250,17 @@ def default_budget(device) -> int:
     return int(free * 0.9)
 
 
+def cached_bytes(device) -> int:
+    """Device memory that PyTorch's allocator holds and does not use: what a
+    search can take without asking the driver (whose answer takes 0.1 to 6 ms
+    on a shared host)."""
+    try:
+        st = torch.cuda.memory_stats_as_nested_dict(device)
+        return int(st["reserved_bytes"]["all"]["current"]) - int(st["allocated_bytes"]["all"]["current"])
+    except (KeyError, RuntimeError):
+        return 0  # another allocator backend
+
+
 # A query provider fills rows [q0, q1) of a RowSet: fn(q0, q1, buffers)
 QueryFill = Callable[[int, int, RowBuffers], None]
 # A dictionary provider fills rows [d0, d1): fn(d0, d1, buffers)
@@ -275,10 +293,17 @@ class Searcher:
         self._plan()
 
     def _plan(self):
-        budget = self.cfg.workspace_bytes or default_budget(self.device)
         drow = RowSet.bytes_per_row(self.n_pix, self.lp_dtype, self.keep_f32)
         qrow_base = RowSet.bytes_per_row(self.n_pix, self.lp_dtype, self.keep_f32)
         qrow = qrow_base + self.k * 12
+        budget = self.cfg.workspace_bytes
+        if not budget and self.device.type == "cuda":
+            # all rows at once, where the allocator's cache already has room
+            whole = round_up(self.n_dict, TILE_D) * drow + round_up(self.n_queries, TILE_Q) * qrow
+            if whole <= 0.9 * self.cfg.free_share * cached_bytes(self.device):
+                budget = whole
+        if not budget:
+            budget = int(default_budget(self.device) * self.cfg.free_share)
         q_min = min(round_up(self.n_queries, TILE_Q), 16384)
         if self.cfg.dict_chunk:
             dchunk = round_up(self.cfg.dict_chunk, TILE_D)
@@ -344,6 +369,15 @@ class Searcher:
         n_dchunks = (D + self.dict_chunk - 1) // self.dict_chunk
         gate = kernels.rescore_gate(self.lp_dtype, q_rows.k_pad, self.n_pix) \
             if (self.rescore and cfg.rescore_gate and cfg.similarity != "euclidean") else 0.0
+        # one query chunk: its rows serve every dictionary chunk, and preparing
+        # them first keeps the GPU busy while fill_dict finishes its host set-up
+        one_chunk = Q <= qc
+        if one_chunk:
+            if Q < qc:  # rows of the last query tile beyond Q
+                q_rows.lp[Q:].zero_()
+                q_rows.norm[Q:].zero_()
+            with _Range(f"ebsd query rows [0, {Q})"):
+                fill_queries(0, Q, q_rows.buffers(0, Q))
         for ci, d0 in enumerate(range(0, D, self.dict_chunk)):
             d1 = min(D, d0 + self.dict_chunk)
             nd = d1 - d0
@@ -360,8 +394,9 @@ class Searcher:
             for q0 in range(0, Q, qc):
                 q1 = min(Q, q0 + qc)
                 nq = q1 - q0
-                with _Range(f"ebsd query rows [{q0}, {q1})"):
-                    fill_queries(q0, q1, q_rows.buffers(0, nq))
+                if not one_chunk:
+                    with _Range(f"ebsd query rows [{q0}, {q1})"):
+                        fill_queries(q0, q1, q_rows.buffers(0, nq))
                 row_scale = _row_scale(q_rows, self.cfg.similarity)
                 # the next chunk's host-to-device copy runs under this chunk's matching
                 prefetch = getattr(fill_queries, "prefetch", None)

@@ -43,28 +43,46 @@ def _cuda(t: torch.Tensor, name: str, dtype=None, contiguous=True) -> torch.Tens
 # ---------------------------------------------------------------- A1/A2 grid
 
 
+class GridFz:
+    """FZ quaternions of the edge^3 cubochoric grid in reference order. The
+    count pass is launched here; `count()` waits for it, so a caller can set
+    other things up (or launch more work) in between."""
+
+    def __init__(self, laue_id: int, edge_length: int, device):
+        self.device = torch.device(device)
+        self.laue, self.edge = int(laue_id), int(edge_length)
+        self.ws_bytes = int(_capi.load().ebsd_grid_workspace_bytes(self.edge))
+        if self.ws_bytes == 0:
+            raise ValueError(f"grid edge length {edge_length} must be positive")
+        self.ws = torch.empty(self.ws_bytes, dtype=torch.uint8, device=self.device)
+        self.cnt = torch.zeros(1, dtype=torch.int64, device=self.device)
+        call("ebsd_grid_fz_count", self.laue, self.edge, ptr(self.ws), self.ws_bytes, ptr(self.cnt),
+             _stream(self.device))
+        self.n: Optional[int] = None
+
+    def count(self) -> int:
+        if self.n is None:
+            self.n = int(self.cnt.item())
+        return self.n
+
+    def write(self, want_f64: bool = False, want_cells: bool = False):
+        """(q_f32 (n, 4), q_f64 (n, 4) or None, int32 cells (n) or None)."""
+        n = self.count()
+        q32 = torch.empty((n, 4), dtype=torch.float32, device=self.device)
+        q64 = torch.empty((n, 4), dtype=torch.float64, device=self.device) if want_f64 else None
+        cells = torch.empty(n, dtype=torch.int32, device=self.device) if want_cells else None
+        if n:
+            call("ebsd_grid_fz_write", self.laue, self.edge, ptr(self.ws), self.ws_bytes, ptr(q32), ptr(q64),
+                 ptr(cells), _stream(self.device))
+        return q32, q64, cells
+
+
 def grid_fz(laue_id: int, edge_length: int, device, want_f64: bool = False, want_cells: bool = False):
     """FZ quaternions of the edge^3 cubochoric grid in reference order.
     Returns (q_f32 (n, 4), q_f64 (n, 4) or None), plus the int32 grid cell of
     each point when want_cells."""
-    device = torch.device(device)
-    lib = _capi.load()
-    nbytes = int(lib.ebsd_grid_workspace_bytes(int(edge_length)))
-    if nbytes == 0:
-        raise ValueError(f"grid edge length {edge_length} must be positive")
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-    cnt = torch.zeros(1, dtype=torch.int64, device=device)
-    s = _stream(device)
-    call("ebsd_grid_fz_count", int(laue_id), int(edge_length), ptr(ws), nbytes, ptr(cnt), s)
-    n = int(cnt.item())
-    q32 = torch.empty((n, 4), dtype=torch.float32, device=device)
-    q64 = torch.empty((n, 4), dtype=torch.float64, device=device) if want_f64 else None
-    cells = torch.empty(n, dtype=torch.int32, device=device) if want_cells else None
-    if n:
-        call("ebsd_grid_fz_write", int(laue_id), int(edge_length), ptr(ws), nbytes, ptr(q32), ptr(q64), ptr(cells), s)
-    if want_cells:
-        return q32, q64, cells
-    return q32, q64
+    q32, q64, cells = GridFz(laue_id, edge_length, device).write(want_f64, want_cells)
+    return (q32, q64, cells) if want_cells else (q32, q64)
 
 
 def gather_rows(src: torch.Tensor, index: torch.Tensor) -> torch.Tensor:

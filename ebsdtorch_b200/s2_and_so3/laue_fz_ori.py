@@ -38,14 +38,35 @@ def _finish(q: Tensor, permute: bool) -> Tensor:
     return q
 
 
+class FzOrientations:
+    """sample_ori_fz_laue_angle in steps, for callers that have work to launch
+    meanwhile: the constructor starts the count, `n` waits for it and starts
+    the write, `finish()` draws the permutation (on the host, under the GPU's
+    work) and returns the orientations."""
+
+    def __init__(self, laue_id: int, angular_resolution_deg: float, device: torch.device, permute: bool = True):
+        get_laue_mult(laue_id)
+        self._grid = kernels.GridFz(laue_id, edge_length_for_resolution(laue_id, angular_resolution_deg), device)
+        self._permute, self._q, self._done = permute, None, None
+
+    @property
+    def n(self) -> int:
+        if self._q is None:
+            self._q = self._grid.write()[0]
+        return self._q.shape[0]
+
+    def finish(self) -> Tensor:
+        if self._done is None:
+            self.n
+            self._done = _finish(self._q, self._permute)
+        return self._done
+
+
 def sample_ori_fz_laue_angle(laue_id: int, angular_resolution_deg: float, device: torch.device,
                              permute: bool = True) -> Tensor:
     """(n, 4) float32 FZ quaternions (w, x, y, z), w >= 0, for a target
     resolution (laue_fz_ori.py:516-557)."""
-    get_laue_mult(laue_id)
-    edge = edge_length_for_resolution(laue_id, angular_resolution_deg)
-    q, _ = kernels.grid_fz(laue_id, edge, device)
-    return _finish(q, permute)
+    return FzOrientations(laue_id, angular_resolution_deg, device, permute).finish()
 
 
 def sample_ori_fz_laue(laue_id: int, target_n_samples: int, device: torch.device, permute: bool = True) -> Tensor:
