@@ -70,6 +70,10 @@ struct GemmParams {
   int64_t m_valid;
   float alpha;
   int accumulate;
+  int vec_c;             // MODE 1: rows of C are 16-byte aligned
+  int a_rows;            // k_tc_gemm_long: rows of A staged (32, 64 or 128)
+  int tile_n;            // k_tc_gemm_long: columns of a unit (16 or 32)
+  int stages;            // k_tc_gemm_long
   const float* bias;     // MODE 2: per-row (output channel) bias
   __nv_bfloat16* out16;  // MODE 2: bf16 activations, (n_valid x ld_out)
   float* out32;          // MODE 2: optional FP32 copy, same layout
@@ -113,6 +117,35 @@ __device__ __forceinline__ void topk_insert(float (&bv)[KC], int (&bi)[KC], floa
 __device__ __forceinline__ void report_timeout(const GemmParams& p, volatile int* abort_flag) {
   *abort_flag = 1;
   atomicExch(p.status, EBSD_DEVICE_TIMEOUT);
+}
+
+// C[grow, col0 + j] = alpha v[j] (+ C): 16-byte stores where the row allows (a
+// warp's lanes hold 32 different rows, so every store instruction touches 32
+// lines either way and their number is what costs: 262,144 x 288 x 64 0.68 ->
+// 0.30 ms, 65,536 x 576 x 128 0.29 -> 0.12).
+__device__ __forceinline__ void store_row32(const GemmParams& p, int64_t grow, int64_t col0, const float (&v)[32]) {
+  float* dst = p.C + grow * p.ldc + col0;
+  if (p.vec_c && col0 + 32 <= p.n_valid) {
+    float4* d4 = reinterpret_cast<float4*>(dst);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float4 r = make_float4(p.alpha * v[4 * j], p.alpha * v[4 * j + 1], p.alpha * v[4 * j + 2],
+                             p.alpha * v[4 * j + 3]);
+      if (p.accumulate) {
+        const float4 c = d4[j];
+        r = make_float4(c.x + r.x, c.y + r.y, c.z + r.z, c.w + r.w);
+      }
+      d4[j] = r;
+    }
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    if (col0 + j < p.n_valid) {
+      const float r = p.alpha * v[j];
+      dst[j] = p.accumulate ? dst[j] + r : r;
+    }
+  }
 }
 
 // MODE 0: top-k epilogue (BIAS: plus col_bias[col] * row_scale[row], the
@@ -392,15 +425,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           } else {
             const int64_t grow = (int64_t)m_tile * BM + row;
             if (grow < p.m_valid) {
-              float* dst = p.C + grow * p.ldc;
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const int64_t col = col0 + j;
-                if (col < p.n_valid) {
-                  const float r = p.alpha * v[j];
-                  dst[col] = p.accumulate ? dst[col] + r : r;
-                }
-              }
+              store_row32(p, grow, col0, v);
             }
           }
         }
@@ -456,6 +481,190 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, T::TMEM_COLS);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Store variant for products with a long K and few output tiles (the weight
+// gradients of the proposal network: K up to 10^6 pixels, 32 x 9 to 256 x 2304
+// outputs). With 128 x 256 tiles they ran in 1 to 18 CTAs that staged mostly
+// padding (48 KB per 64 of K) and took 5.6 of a training step's 12.7 ms. A unit
+// is 128 rows x 16 or 32 columns, only the rows of A that exist are staged, and
+// a stage holds 128 of K, so many stages are in flight and the chain of
+// dependent MMAs is the bound (60 ns each on one accumulator). K is not split:
+// every output keeps its one chain of accumulations in the order of k_tc_gemm,
+// and with it its value (the FP32 accumulators truncate, so a split sum of 10^6
+// terms differs by 10^-3). 32 x 9 x 1,048,576: 6.16 -> 3.97 ms, 64 x 288 x
+// 262,144: 1.53 -> 1.00, 256 x 1,152 x 16,384: 0.12 -> 0.07.
+//   warp 0 TMA producer, warp 1 TMEM (32 columns) and the MMAs, warps 2-5
+//   epilogue; waits and give-up as in k_tc_gemm.
+// ---------------------------------------------------------------------------
+constexpr int LONG_MAX_STAGES = 16;
+constexpr int LONG_BAR_BYTES = 8 * (2 * LONG_MAX_STAGES + 2) + 16;
+constexpr int LONG_DATA_BYTES = 216 * 1024;
+constexpr int LONG_SMEM_BYTES = 1024 + LONG_DATA_BYTES + LONG_BAR_BYTES;
+static_assert(LONG_SMEM_BYTES <= 232448, "shared memory budget");
+
+// Bytes of one 128-byte-wide half of a stage.
+__host__ __device__ inline int long_half_bytes(int a_rows, int tile_n) { return (a_rows + tile_n) * BKB; }
+
+template <int KIND>
+__global__ void __launch_bounds__(THREADS, 1)
+    k_tc_gemm_long(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const GemmParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_s = smem_u32(smem_raw);
+  uint8_t* smem = smem_raw + ((1024u - (raw_s & 1023u)) & 1023u);
+  const uint32_t sbase = smem_u32(smem);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + LONG_DATA_BYTES);
+  const uint32_t bar0 = smem_u32(bars);
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (LONG_MAX_STAGES + s); };
+  const uint32_t accf_bar = bar0 + 8u * (2 * LONG_MAX_STAGES);
+  const uint32_t drain_bar = accf_bar + 8u;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * LONG_MAX_STAGES + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int stages = p.stages, k_iters = p.k_iters, tile_n = p.tile_n;
+  const int m_tile = (int)blockIdx.x / p.n_tiles, n_tile = (int)blockIdx.x % p.n_tiles;
+  const uint32_t a_bytes = (uint32_t)p.a_rows * BKB, half = (uint32_t)long_half_bytes(p.a_rows, tile_n);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    mbar_init(accf_bar, 1);
+    mbar_init(drain_bar, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 0 && lane == 0) {
+    prefetch_tmap(&tmA);
+    prefetch_tmap(&tmB);
+  }
+  if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 32);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+  const uint64_t wait_ns = p.wait_ns;
+  constexpr int kx_step = BKB / kind_elem_bytes<KIND>();
+  int prod_stage = 0;
+  uint32_t prod_phase = 0;
+  int64_t issued = 0;
+  bool any_mma = false;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int k = 0; k < k_iters; k += 2) {
+        if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, wait_ns)) {
+          ok = false;
+          break;
+        }
+        const int halves = min(2, k_iters - k);
+        const uint32_t dst = sbase + (uint32_t)stage * 2u * half;
+        mbar_arrive_expect_tx(full_bar(stage), (uint32_t)halves * half);
+        for (int h = 0; h < halves; ++h) {
+          tma_load_2d(dst + h * half, &tmA, (k + h) * kx_step, m_tile * BM, full_bar(stage));
+          tma_load_2d(dst + h * half + a_bytes, &tmB, (k + h) * kx_step, n_tile * tile_n, full_bar(stage));
+        }
+        ++issued;
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+      if (!ok) report_timeout(p, abort_flag);
+      prod_stage = stage;
+      prod_phase = phase;
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      const uint32_t idesc = (make_idesc<KIND, 256>() & ~(0x3Fu << 17)) | ((uint32_t)(tile_n >> 3) << 17);
+      for (int k = 0; k < k_iters; k += 2) {
+        if (!mbar_wait(full_bar(stage), phase, abort_flag, wait_ns)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t base = sbase + (uint32_t)stage * 2u * half;
+        const int halves = min(2, k_iters - k);
+        for (int h = 0; h < halves; ++h) {
+          const uint32_t a_addr = base + h * half, b_addr = a_addr + a_bytes;
+#pragma unroll
+          for (int kk = 0; kk < BKB / 32; ++kk)
+            tc_mma<KIND>(tmem_base, smem_desc_sw128(a_addr + kk * 32), smem_desc_sw128(b_addr + kk * 32), idesc,
+                         (k | h | kk) != 0 ? 1u : 0u);
+        }
+        any_mma = true;
+        tc_commit(empty_bar(stage));
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+      if (ok)
+        tc_commit(accf_bar);
+      else
+        report_timeout(p, abort_flag);
+    }
+    __syncwarp();
+  } else {
+    const int wq = warp & 3;
+    const bool got = __all_sync(0xffffffffu, mbar_wait_sleep(accf_bar, 0, abort_flag, wait_ns));
+    if (got) {
+      tc_fence_after();
+      float v[32];
+      tmem_ld32(tmem_base + ((uint32_t)(wq * 32) << 16), v);
+      const int64_t grow = (int64_t)m_tile * BM + wq * 32 + lane, col0 = (int64_t)n_tile * tile_n;
+      if (grow < p.m_valid) {
+        float* dst = p.C + grow * p.ldc + col0;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          if (j < tile_n && col0 + j < p.n_valid) {
+            const float r = p.alpha * v[j];
+            dst[j] = p.accumulate ? dst[j] + r : r;
+          }
+        }
+      }
+    } else if (lane == 0) {
+      report_timeout(p, abort_flag);
+    }
+  }
+
+  __syncthreads();
+  if (*abort_flag) {
+    volatile int never = 0;
+    if (warp == 0 && lane == 0) {
+      const int64_t inflight = issued < stages ? issued : (int64_t)stages;
+      int s = prod_stage;
+      uint32_t ph = prod_phase;
+      for (int64_t i = 0; i < inflight; ++i) {
+        if (s == 0) {
+          s = stages - 1;
+          ph ^= 1u;
+        } else {
+          --s;
+        }
+        mbar_wait(full_bar(s), ph, &never);
+      }
+    } else if (warp == 1 && lane == 0 && any_mma) {
+      tc_commit(drain_bar);
+      mbar_wait(drain_bar, 0, &never);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 32);
   }
 }
 
@@ -1390,6 +1599,36 @@ extern "C" int ebsd_match_topk(const void* queries_lp, int64_t n_queries_pad, co
                                index_base, 256, 0, d_status, stream);
 }
 
+// Whether a product runs k_tc_gemm_long: K long enough that one unit's chain
+// outlasts its set-up, and too few 128 x 256 tiles to occupy half of the SMs
+// (with more, the wide tiles re-read A less often). At K = 4,096 and 18 wide
+// tiles the two take 0.030 and 0.033 ms, at K = 262,144 and 2 tiles 1.0 and 1.5.
+static bool takes_long_tiles(int64_t m_tiles, int64_t n_valid, int64_t k_bytes) {
+  return k_bytes >= 4096 && m_tiles * ceil_div(n_valid, 256) <= device_sm_count() / 2;
+}
+
+template <int KIND>
+static int launch_long(const void* A, const void* B, int lp_dtype, int64_t m_pad, int64_t n_pad, int64_t k_pad,
+                       const GemmParams& p_in, cudaStream_t s) {
+  GemmParams p = p_in;
+  const int64_t m_tiles = ceil_div(p.m_valid, BM);
+  p.a_rows = m_tiles > 1 || p.m_valid > 64 ? 128 : p.m_valid > 32 ? 64 : 32;
+  p.tile_n = m_tiles * ceil_div(p.n_valid, 32) <= device_sm_count() / 2 ? 16 : 32;
+  p.n_tiles = (int)ceil_div(p.n_valid, p.tile_n);
+  // the MMA reads 128 rows of A wherever its tile starts: keep the last one inside
+  const int half = long_half_bytes(p.a_rows, p.tile_n);
+  p.stages = std::min(LONG_MAX_STAGES, (LONG_DATA_BYTES - A_BYTES + half) / (2 * half));
+  p.wait_ns = wait_limit_ns();
+  CUtensorMap ta, tb;
+  if (int rc = make_tmap(&ta, A, lp_dtype, m_pad, k_pad, p.a_rows)) return rc;
+  if (int rc = make_tmap(&tb, B, lp_dtype, n_pad, k_pad, p.tile_n)) return rc;
+  const auto kern = k_tc_gemm_long<KIND>;
+  EBSD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LONG_SMEM_BYTES));
+  kern<<<(unsigned)(m_tiles * p.n_tiles), THREADS, LONG_SMEM_BYTES, s>>>(ta, tb, p);
+  EBSD_LAUNCH_CHECK();
+  return 0;
+}
+
 extern "C" int ebsd_gemm_nt(const void* A, int64_t m_pad, const void* B, int64_t n_pad, int64_t k_pad,
                             int lp_dtype, float alpha, int accumulate, float* C, int64_t ldc, int64_t m_valid,
                             int64_t n_valid, int splits, int* d_status, void* stream) {
@@ -1398,6 +1637,20 @@ extern "C" int ebsd_gemm_nt(const void* A, int64_t m_pad, const void* B, int64_t
   EBSD_ARG_CHECK(m_valid > 0 && m_valid <= m_pad && n_valid > 0 && n_valid <= n_pad,
                  "valid extents out of range");
   EBSD_ARG_CHECK(ldc >= n_valid, "ldc < n_valid");
+  const int64_t k_bytes = k_pad * (lp_dtype == EBSD_DT_BF16 ? 2 : 1);
+  if (splits <= 0 && takes_long_tiles(ceil_div(m_valid, BM), n_valid, k_bytes)) {
+    GemmParams p{};
+    p.k_iters = (int)(k_bytes / BKB);
+    p.n_valid = n_valid;
+    p.C = C;
+    p.ldc = ldc;
+    p.m_valid = m_valid;
+    p.alpha = alpha;
+    p.accumulate = accumulate;
+    p.status = d_status;
+    return lp_dtype == EBSD_DT_BF16 ? launch_long<0>(A, B, lp_dtype, m_pad, n_pad, k_pad, p, as_stream(stream))
+                                    : launch_long<1>(A, B, lp_dtype, m_pad, n_pad, k_pad, p, as_stream(stream));
+  }
   CUtensorMap ta, tb;
   if (int rc = make_tmap(&ta, A, lp_dtype, m_pad, k_pad, BM)) return rc;
   if (int rc = make_tmap(&tb, B, lp_dtype, n_pad, k_pad, 256)) return rc;
@@ -1413,6 +1666,7 @@ extern "C" int ebsd_gemm_nt(const void* A, int64_t m_pad, const void* B, int64_t
   p.m_valid = m_valid;
   p.alpha = alpha;
   p.accumulate = accumulate;
+  p.vec_c = ldc % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
   p.status = d_status;
   const int64_t m_tiles = m_pad / BM;
   EBSD_ARG_CHECK(m_tiles * p.splits < INT32_MAX, "too many work units");
@@ -1445,6 +1699,7 @@ extern "C" int ebsd_gemm_f32(const float* A, int64_t lda, int64_t m, const float
   p.m_valid = m;
   p.alpha = alpha;
   p.accumulate = accumulate;
+  p.vec_c = ldc % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
   p.status = d_status;
   EBSD_ARG_CHECK(m_tiles * p.splits < INT32_MAX, "too many work units");
   p.units = (int)(m_tiles * p.splits);
