@@ -26,6 +26,11 @@ void set_error(const char* fmt, ...);
 // Limit of the bounded waits of the next tensor-core kernel launches
 // (ebsd_set_wait_limit_ns; kWaitLimitNs by default).
 uint64_t wait_limit_ns();
+// Encodes a tiled tensor map (no interleave, zero fill outside the extents);
+// 0 or an EBSD_ERR code with the message set.
+int encode_tensor_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims,
+                      const cuuint64_t* strides, const cuuint32_t* box, const cuuint32_t* steps,
+                      CUtensorMapSwizzle swizzle);
 
 // Debug checks. In the checking build (-DEBSD_CHECK: `python -m
 // ebsdtorch_b200.build --check`, loaded when EBSD_CHECK_BUILD=1) a failed

@@ -1271,6 +1271,24 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
+int encode_tensor_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims,
+                      const cuuint64_t* strides, const cuuint32_t* box, const cuuint32_t* steps,
+                      CUtensorMapSwizzle swizzle) {
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) {
+    set_error("cuTensorMapEncodeTiled is unavailable from the CUDA driver");
+    return EBSD_ERR_UNSUPPORTED;
+  }
+  const CUresult r = enc(map, type, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, steps,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (CUresult %d) for a rank-%d map", (int)r, rank);
+    return EBSD_ERR_ARG;
+  }
+  return 0;
+}
+
 static int make_tmap(CUtensorMap* map, const void* ptr, int lp_dtype, int64_t rows, int64_t k_pad,
                      int box_rows) {
   EncodeTiledFn enc = encode_fn();

@@ -5,9 +5,9 @@ Architecture: five 3x3 / stride-2 / pad-1 convolutions with ReLU
 (1 -> 32 -> 64 -> 128 -> 256 -> 256 channels; a 128 x 128 pattern becomes
 4 x 4 x 256), then a two-layer head (4096 -> 64 with ReLU, 64 -> 6) that
 predicts the 6-D rotation representation of Zhou et al. (orientations.py:940);
-1.24 M parameters. Convolutions run in bf16 on the tcgen05 GEMM (im2col
-forward with bias, ReLU and the activation stores fused into the GEMM
-epilogue; weight- and column-gradient GEMMs + col2im backward), except the
+1.24 M parameters. Convolutions run in bf16 on tcgen05 (forward: patches
+gathered straight into the operand tiles, bias, ReLU and the activation stores
+fused; backward: weight- and column-gradient GEMMs + col2im), except the
 single-channel first layer, computed directly on the CUDA cores; the head in
 FP32. The loss is the symmetry-aware rotation loss min_g ||R(z) - R(g q)||_F^2
 (ebsd_rot6d_sym_loss), optimiser Adam on FP32 master weights.
@@ -73,8 +73,13 @@ class _Conv:
         out32 = torch.empty((M, self.cout), dtype=torch.float32, device=x.device) if want32 else None
         if self.cin == 1:
             # 9 taps: a direct SIMT convolution beats a GEMM padded to K = 64
-            call("ebsd_cnn_conv_c1", ptr(x), B, H, W, ptr(self.w16), self.K_pad, ptr(self.b), self.cout, 1, ptr(out),
+            call("ebsd_cnn_conv_c1" if x.dtype == torch.bfloat16 else "ebsd_cnn_conv_c1_f32", ptr(x), B, H, W, ptr(self.w16), self.K_pad, ptr(self.b), self.cout, 1, ptr(out),
                  ptr(out32), _stream(x))
+            keep.update(x=x)
+        elif _capi.load().ebsd_cnn_conv_supported(self.cin, self.cout, W):
+            # patches gathered into the operand tiles by strided copies, no columns
+            call("ebsd_cnn_conv_tc", ptr(x), B, H, W, self.cin, ptr(self.w16), self.K_pad, ptr(self.b), self.cout, 1,
+                 ptr(out), ptr(out32), ptr(self.status), _stream(x))
             keep.update(x=x)
         else:
             # one tcgen05 GEMM with the output channels on the 128-row side and
@@ -191,10 +196,12 @@ class OrientationCNN:
         B = x.shape[0]
         if B % 128:
             raise ValueError("batch size must be a multiple of 128")
-        x16 = torch.empty((B, self.H, self.W), dtype=torch.bfloat16, device=x.device)
-        call("ebsd_cnn_scale_cast", ptr(x.contiguous()), x.numel(), 1.0, ptr(x16), _stream(x))
+        a, h, w = x.contiguous(), self.H, self.W
+        if keep or a.dtype != torch.float32:
+            # bf16 pixels, which backward() reads again; inference rounds them in the first layer
+            a = torch.empty((B, h, w), dtype=torch.bfloat16, device=x.device)
+            call("ebsd_cnn_scale_cast", ptr(x.contiguous()), x.numel(), 1.0, ptr(a), _stream(x))
         self._keep = []
-        a, h, w = x16, self.H, self.W
         a32 = None
         for i, conv in enumerate(self.convs):
             saved = {}

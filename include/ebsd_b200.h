@@ -562,6 +562,9 @@ int ebsd_cnn_im2col(const void* x, int B, int H, int W, int C, int64_t m_pad, in
  * act(conv(x, w16[:, :9]) + bias), cout in {16, 32, 64}, w16 row stride ldw. */
 int ebsd_cnn_conv_c1(const void* x, int B, int H, int W, const void* w16, int ldw, const float* bias, int cout,
                      int relu, void* out16, float* out32, void* stream);
+/* The same from FP32 pixels, rounded to bf16 as they are read. */
+int ebsd_cnn_conv_c1_f32(const float* x, int B, int H, int W, const void* w16, int ldw, const float* bias, int cout,
+                         int relu, void* out16, float* out32, void* stream);
 int ebsd_cnn_col2im(const float* dcols, int64_t ld, int B, int H, int W, int C, float* dx, void* stream);
 /* Convolution forward as one tcgen05 GEMM with a fused epilogue:
  * out[r, c] = act(sum_k cols[r, k] w16[c, k] + bias[c]) for rows r < n_rows
@@ -572,6 +575,16 @@ int ebsd_cnn_col2im(const float* dcols, int64_t ld, int B, int H, int W, int C, 
 int ebsd_cnn_conv_fwd(const void* w16, int64_t cout_pad, const void* cols, int64_t rows_pad, int64_t k_pad,
                       const float* bias, int cout, int64_t n_rows, int relu, void* out16, int64_t ld_out,
                       float* out32, int splits, int* d_status, void* stream);
+/* The same convolution without columns: patches are gathered from x (batch x
+ * height x width x cin, bf16 NHWC) by strided TMA copies into the operand
+ * tiles; the same bits as im2col + ebsd_cnn_conv_fwd. w16: cout rows of 9 cin
+ * weights (row stride ldw, a multiple of 8), out16 / out32: contiguous rows of
+ * cout. All pointers 16-byte aligned. ebsd_cnn_conv_supported: 1 for the
+ * channel counts and widths it takes (32 -> 64, 64 -> 128, multiples of 64 ->
+ * 256; output rows of up to 128 pixels). */
+int ebsd_cnn_conv_supported(int cin, int cout, int width);
+int ebsd_cnn_conv_tc(const void* x, int batch, int height, int width, int cin, const void* w16, int64_t ldw,
+                     const float* bias, int cout, int relu, void* out16, float* out32, int* d_status, void* stream);
 int ebsd_cnn_bias_act(const float* y, int64_t ldy, const float* bias, int64_t M, int C, int relu, void* out,
                       int64_t ld_out, float* out32, void* stream);
 int ebsd_cnn_relu_grad(const float* dy, int64_t ldy, const void* act, int64_t lda, int64_t M, int C, float* g32,
