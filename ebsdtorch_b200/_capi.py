@@ -89,6 +89,9 @@ SIGNATURES = {
     "ebsd_cnn_bias_act": (i32, [vp, i64, vp, i64, i32, i32, vp, i64, vp, vp]),
     "ebsd_cnn_conv_c1": (i32, [vp, i32, i32, i32, vp, i32, vp, i32, i32, vp, vp, vp]),
     "ebsd_cnn_conv_c1_f32": (i32, [vp, i32, i32, i32, vp, i32, vp, i32, i32, vp, vp, vp]),
+    "ebsd_gemm_nt_group": (i32, [i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
+    "ebsd_cnn_im2col_t": (i32, [vp, i32, i32, i32, i32, vp, i64, vp]),
+    "ebsd_cnn_relu_grad_t": (i32, [vp, vp, i64, i32, vp, i64, vp, i64, vp, vp]),
     "ebsd_cnn_conv_supported": (i32, [i32, i32, i32]),
     "ebsd_cnn_conv_tc": (i32, [vp, i32, i32, i32, i32, vp, i64, vp, i32, i32, vp, vp, vp, vp]),
     "ebsd_cnn_conv_fwd": (i32, [vp, i64, vp, i64, i64, vp, i32, i64, i32, vp, i64, vp, i32, vp, vp]),
@@ -120,7 +123,7 @@ LAUNCHES_PER_CALL = {
     "ebsd_pcfit_prep": 1, "ebsd_pcfit_reduce": 1, "ebsd_pcfit_xcorr_tables": 1, "ebsd_pcfit_spectra": 1,
     "ebsd_pcfit_pattern_terms": 1, "ebsd_pcfit_xcorr_max": 1, "ebsd_pcfit_fold": 1,
     "ebsd_rot6d_sym_loss": 1, "ebsd_cnn_im2col": 1, "ebsd_cnn_col2im": 1, "ebsd_cnn_bias_act": 1,
-    "ebsd_cnn_conv_fwd": 1, "ebsd_cnn_conv_tc": 1, "ebsd_cnn_conv_c1": 1, "ebsd_cnn_conv_c1_f32": 1, "ebsd_cnn_relu_grad": 1, "ebsd_cnn_col_sum": 1,
+    "ebsd_cnn_conv_fwd": 1, "ebsd_cnn_im2col_t": 1, "ebsd_cnn_relu_grad_t": 1, "ebsd_gemm_nt_group": 1, "ebsd_cnn_conv_tc": 1, "ebsd_cnn_conv_c1": 1, "ebsd_cnn_conv_c1_f32": 1, "ebsd_cnn_relu_grad": 1, "ebsd_cnn_col_sum": 1,
     "ebsd_cnn_transpose": 1, "ebsd_cnn_scale_cast": 1,
     "ebsd_cnn_dense_fwd": 1, "ebsd_cnn_dense_bwd": 2, "ebsd_cnn_adam": 1,
 }

@@ -181,7 +181,151 @@ __global__ void __launch_bounds__(256) k_conv_c1(const T* __restrict__ x, int H,
   }
 }
 
+// out[(ky, kx, c), m] = x[b, 2 oy - 1 + ky, 2 ox - 1 + kx, c] for output pixel
+// m = (b, oy, ox): the columns of k_im2col, transposed (a weight gradient's
+// operand), straight from the activations. Block: 64 pixels x up to 64 channels
+// of one tap through shared memory, 16-byte loads and stores.
+constexpr int kTrPix = 64, kTrPitch = kTrPix + 8;
+
+__global__ void __launch_bounds__(256) k_im2col_t(const __nv_bfloat16* __restrict__ x, int H, int W, int C, int Ho,
+                                                  int Wo, int64_t M, __nv_bfloat16* __restrict__ out, int64_t ld) {
+  __shared__ __align__(16) __nv_bfloat16 tile[64 * kTrPitch];
+  const int cw = min(C, 64), blocks_c = C / cw;
+  const int tap = blockIdx.y / blocks_c, c0 = (blockIdx.y % blocks_c) * cw;
+  const int64_t m0 = (int64_t)blockIdx.x * kTrPix;
+  const int hw = Ho * Wo;
+  {
+    const int p = threadIdx.x & 63;
+    const int64_t m = m0 + p;
+    const uint4* src = nullptr;
+    if (m < M) {
+      const int b = (int)(m / hw), rem = (int)(m - (int64_t)b * hw);
+      const int oy = rem / Wo, ox = rem - oy * Wo;
+      const int iy = 2 * oy - 1 + tap / 3, ix = 2 * ox - 1 + tap % 3;
+      if (iy >= 0 && iy < H && ix >= 0 && ix < W)
+        src = reinterpret_cast<const uint4*>(x + (((int64_t)b * H + iy) * W + ix) * C + c0);
+    }
+    for (int k = threadIdx.x >> 6; k < cw / 8; k += 4) {
+      __align__(16) __nv_bfloat16 v[8];
+      *reinterpret_cast<uint4*>(v) = src ? __ldg(src + k) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) tile[(8 * k + e) * kTrPitch + p] = v[e];
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < cw * 8; i += 256) {
+    const int c = i >> 3, j = i & 7;
+    if (m0 + 8 * j < M)
+      *reinterpret_cast<uint4*>(out + ((int64_t)tap * C + c0 + c) * ld + m0 + 8 * j) =
+          *reinterpret_cast<const uint4*>(tile + c * kTrPitch + 8 * j);
+  }
+}
+
+// The same for a single channel: eight pixels of a tap per thread.
+__global__ void k_im2col_t1(const __nv_bfloat16* __restrict__ x, int H, int W, int Ho, int Wo, int64_t M,
+                            __nv_bfloat16* __restrict__ out, int64_t ld) {
+  const int tap = blockIdx.y, hw = Ho * Wo;
+  const int64_t m0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (m0 >= M) return;
+  __align__(16) __nv_bfloat16 v[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int64_t m = m0 + e;
+    const int b = (int)(m / hw), rem = (int)(m - (int64_t)b * hw);
+    const int oy = rem / Wo, ox = rem - oy * Wo;
+    const int iy = 2 * oy - 1 + tap / 3, ix = 2 * ox - 1 + tap % 3;
+    v[e] = (m < M && iy >= 0 && iy < H && ix >= 0 && ix < W) ? x[((int64_t)b * H + iy) * W + ix]
+                                                             : __float2bfloat16_rn(0.f);
+  }
+  *reinterpret_cast<uint4*>(out + tap * ld + m0) = *reinterpret_cast<const uint4*>(v);
+}
+
+// g = dy * (act > 0) of a convolution layer in one pass over its pixels: bf16
+// rows g16 (optional, row stride ld16, columns C .. ld16 zero), the bf16
+// transpose gT (C rows of ld_t) and the column sums added to db. Block: 64
+// pixels x 64 channels through shared memory, several pixel tiles per block.
+__global__ void __launch_bounds__(256) k_relu_grad_t(const float* __restrict__ dy,
+                                                     const __nv_bfloat16* __restrict__ act, int64_t M, int C,
+                                                     __nv_bfloat16* __restrict__ g16, int64_t ld16,
+                                                     __nv_bfloat16* __restrict__ gT, int64_t ld_t,
+                                                     float* __restrict__ db) {
+  __shared__ __align__(16) __nv_bfloat16 tile[64 * kTrPitch];
+  __shared__ float sums[64];
+  const int c0 = blockIdx.y * 64, cw = min(64, C - c0);
+  const int c4 = (threadIdx.x & 15) * 4, row = threadIdx.x >> 4;
+  if (threadIdx.x < 64) sums[threadIdx.x] = 0.f;
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int64_t m0 = (int64_t)blockIdx.x * kTrPix; m0 < M; m0 += (int64_t)gridDim.x * kTrPix) {
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int64_t m = m0 + row + 16 * k;
+      float g[4] = {0.f, 0.f, 0.f, 0.f};
+      if (m < M && c4 < cw) {
+        const float4 d = __ldg(reinterpret_cast<const float4*>(dy + m * C + c0 + c4));
+        const uint2 aw = __ldg(reinterpret_cast<const uint2*>(act + m * C + c0 + c4));
+        const __nv_bfloat16* a = reinterpret_cast<const __nv_bfloat16*>(&aw);
+        g[0] = __bfloat162float(a[0]) > 0.f ? d.x : 0.f;
+        g[1] = __bfloat162float(a[1]) > 0.f ? d.y : 0.f;
+        g[2] = __bfloat162float(a[2]) > 0.f ? d.z : 0.f;
+        g[3] = __bfloat162float(a[3]) > 0.f ? d.w : 0.f;
+      }
+      __align__(8) __nv_bfloat16 h[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        s[e] += g[e];
+        h[e] = __float2bfloat16_rn(g[e]);
+        tile[(c4 + e) * kTrPitch + row + 16 * k] = h[e];
+      }
+      if (g16 && m < M && c0 + c4 < ld16)
+        *reinterpret_cast<uint2*>(g16 + m * ld16 + c0 + c4) = *reinterpret_cast<const uint2*>(h);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < cw * 8; i += 256) {
+      const int c = i >> 3, j = i & 7;
+      if (m0 + 8 * j < M)
+        *reinterpret_cast<uint4*>(gT + (int64_t)(c0 + c) * ld_t + m0 + 8 * j) =
+            *reinterpret_cast<const uint4*>(tile + c * kTrPitch + 8 * j);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < 4; ++e) atomicAdd(&sums[c4 + e], s[e]);
+  __syncthreads();
+  if ((int)threadIdx.x < cw) atomicAdd(db + c0 + threadIdx.x, sums[threadIdx.x]);
+}
+
 // dx[b, iy, ix, c] = sum over the (output, tap) pairs that read it of dcols.
+// VEC: four channels per thread (C and ld multiples of 4, aligned).
+__global__ void k_col2im4(const float* __restrict__ dcols, int64_t ld, int B, int H, int W, int C, int Ho, int Wo,
+                          float* __restrict__ dx) {
+  const int c4s = C / 4;
+  const int64_t total = (int64_t)B * H * W * c4s;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const int c = (int)(t % c4s) * 4;
+    const int64_t p = t / c4s;
+    const int ix = (int)(p % W), iy = (int)((p / W) % H), b = (int)(p / ((int64_t)W * H));
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int ky = 0; ky < 3; ++ky) {
+      const int ny = iy + 1 - ky;  // = 2 oy
+      if (ny < 0 || (ny & 1) || (ny >> 1) >= Ho) continue;
+#pragma unroll
+      for (int kx = 0; kx < 3; ++kx) {
+        const int nx = ix + 1 - kx;
+        if (nx < 0 || (nx & 1) || (nx >> 1) >= Wo) continue;
+        const int64_t r = ((int64_t)b * Ho + (ny >> 1)) * Wo + (nx >> 1);
+        const float4 d = __ldg(reinterpret_cast<const float4*>(dcols + r * ld + (ky * 3 + kx) * C + c));
+        s.x += d.x;
+        s.y += d.y;
+        s.z += d.z;
+        s.w += d.w;
+      }
+    }
+    *reinterpret_cast<float4*>(dx + p * C + c) = s;
+  }
+}
+
 __global__ void k_col2im(const float* __restrict__ dcols, int64_t ld, int B, int H, int W, int C, int Ho, int Wo,
                          float* __restrict__ dx) {
   const int64_t total = (int64_t)B * H * W * C;
@@ -431,7 +575,48 @@ extern "C" int ebsd_cnn_col2im(const float* dcols, int64_t ld, int B, int H, int
                                void* stream) {
   EBSD_ARG_CHECK(dcols && dx && ld >= 9 * C, "ebsd_cnn_col2im: bad arguments");
   const int Ho = (H + 1) / 2, Wo = (W + 1) / 2;
+  if (C % 4 == 0 && ld % 4 == 0 && ((uintptr_t)dcols & 15) == 0 && ((uintptr_t)dx & 15) == 0) {
+    k_col2im4<<<nblocks((int64_t)B * H * W * (C / 4)), 256, 0, CNN_STREAM>>>(dcols, ld, B, H, W, C, Ho, Wo, dx);
+    EBSD_LAUNCH_CHECK();
+    return 0;
+  }
   k_col2im<<<nblocks((int64_t)B * H * W * C), 256, 0, CNN_STREAM>>>(dcols, ld, B, H, W, C, Ho, Wo, dx);
+  EBSD_LAUNCH_CHECK();
+  return 0;
+}
+
+extern "C" int ebsd_cnn_im2col_t(const void* x, int B, int H, int W, int C, void* out, int64_t ld, void* stream) {
+  const int Ho = (H + 1) / 2, Wo = (W + 1) / 2;
+  const int64_t M = (int64_t)B * Ho * Wo;
+  EBSD_ARG_CHECK(x && out && B > 0 && H > 0 && W > 0, "ebsd_cnn_im2col_t: bad arguments");
+  EBSD_ARG_CHECK(C == 1 || C == 32 || C % 64 == 0, "ebsd_cnn_im2col_t: %d channels not 1, 32 or a multiple of 64", C);
+  EBSD_ARG_CHECK(M % 8 == 0 && ld >= M && ld % 8 == 0, "ebsd_cnn_im2col_t: pixel counts must be multiples of 8");
+  EBSD_ARG_CHECK(((uintptr_t)x & 15) == 0 && ((uintptr_t)out & 15) == 0, "ebsd_cnn_im2col_t: pointers not 16-byte aligned");
+  EBSD_ARG_CHECK(ceil_div(M, kTrPix) < INT32_MAX, "ebsd_cnn_im2col_t: too many pixels");
+  const auto* xb = reinterpret_cast<const __nv_bfloat16*>(x);
+  auto* ob = reinterpret_cast<__nv_bfloat16*>(out);
+  if (C == 1)
+    k_im2col_t1<<<dim3(ceil_div(M, 8 * 256), 9), 256, 0, CNN_STREAM>>>(xb, H, W, Ho, Wo, M, ob, ld);
+  else
+    k_im2col_t<<<dim3(ceil_div(M, kTrPix), 9 * (C / std::min(C, 64))), 256, 0, CNN_STREAM>>>(xb, H, W, C, Ho, Wo, M,
+                                                                                            ob, ld);
+  EBSD_LAUNCH_CHECK();
+  return 0;
+}
+
+extern "C" int ebsd_cnn_relu_grad_t(const float* dy, const void* act, int64_t M, int C, void* g16, int64_t ld16,
+                                    void* gT, int64_t ld_t, float* db, void* stream) {
+  EBSD_ARG_CHECK(dy && act && gT && db && M > 0 && C > 0 && C % 4 == 0, "ebsd_cnn_relu_grad_t: bad arguments");
+  EBSD_ARG_CHECK(M % 8 == 0 && ld_t >= M && ld_t % 8 == 0, "ebsd_cnn_relu_grad_t: pixel counts must be multiples of 8");
+  EBSD_ARG_CHECK(!g16 || (ld16 >= C && ld16 % 4 == 0), "ebsd_cnn_relu_grad_t: bad ld16");
+  EBSD_ARG_CHECK((((uintptr_t)dy | (uintptr_t)act | (uintptr_t)g16 | (uintptr_t)gT) & 15) == 0,
+                 "ebsd_cnn_relu_grad_t: pointers not 16-byte aligned");
+  EBSD_CUDA_CHECK(cudaMemsetAsync(db, 0, sizeof(float) * C, CNN_STREAM));
+  const int cols = ceil_div(std::max<int64_t>(C, g16 ? ld16 : C), 64);
+  const int rows = (int)std::min<int64_t>((M + kTrPix - 1) / kTrPix, std::max(1, device_sm_count() * 8 / cols));
+  k_relu_grad_t<<<dim3(rows, cols), 256, 0, CNN_STREAM>>>(
+      dy, reinterpret_cast<const __nv_bfloat16*>(act), M, C, reinterpret_cast<__nv_bfloat16*>(g16), ld16,
+      reinterpret_cast<__nv_bfloat16*>(gT), ld_t, db);
   EBSD_LAUNCH_CHECK();
   return 0;
 }

@@ -509,9 +509,8 @@ static_assert(LONG_SMEM_BYTES <= 232448, "shared memory budget");
 __host__ __device__ inline int long_half_bytes(int a_rows, int tile_n) { return (a_rows + tile_n) * BKB; }
 
 template <int KIND>
-__global__ void __launch_bounds__(THREADS, 1)
-    k_tc_gemm_long(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                   const GemmParams p) {
+__device__ __forceinline__ void long_unit(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p,
+                                          int unit) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_s = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw_s & 1023u)) & 1023u);
@@ -526,7 +525,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int stages = p.stages, k_iters = p.k_iters, tile_n = p.tile_n;
-  const int m_tile = (int)blockIdx.x / p.n_tiles, n_tile = (int)blockIdx.x % p.n_tiles;
+  const int m_tile = unit / p.n_tiles, n_tile = unit % p.n_tiles;
   const uint32_t a_bytes = (uint32_t)p.a_rows * BKB, half = (uint32_t)long_half_bytes(p.a_rows, tile_n);
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -666,6 +665,29 @@ __global__ void __launch_bounds__(THREADS, 1)
     tc_fence_after();
     tmem_dealloc(tmem_base, 32);
   }
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(THREADS, 1)
+    k_tc_gemm_long(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const GemmParams p) {
+  long_unit<KIND>(tmA, tmB, p, (int)blockIdx.x);
+}
+
+// Several such products in one launch, longest chain first: the chains of the
+// short ones run beside that of the longest instead of after it.
+constexpr int LONG_GROUP = 8;
+struct LongGroup {
+  CUtensorMap a[LONG_GROUP], b[LONG_GROUP];
+  GemmParams p[LONG_GROUP];
+  int first[LONG_GROUP + 1];
+  int n;
+};
+
+__global__ void __launch_bounds__(THREADS, 1) k_tc_gemm_long_group(const __grid_constant__ LongGroup g) {
+  int i = 0;
+  while (i + 1 < g.n && (int)blockIdx.x >= g.first[i + 1]) ++i;
+  long_unit<0>(g.a[i], g.b[i], g.p[i], (int)blockIdx.x - g.first[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1625,10 +1647,9 @@ static bool takes_long_tiles(int64_t m_tiles, int64_t n_valid, int64_t k_bytes) 
   return k_bytes >= 4096 && m_tiles * ceil_div(n_valid, 256) <= device_sm_count() / 2;
 }
 
-template <int KIND>
-static int launch_long(const void* A, const void* B, int lp_dtype, int64_t m_pad, int64_t n_pad, int64_t k_pad,
-                       const GemmParams& p_in, cudaStream_t s) {
-  GemmParams p = p_in;
+// Completes the parameters and tensor maps of one product; units: its CTAs.
+static int plan_long(const void* A, const void* B, int lp_dtype, int64_t m_pad, int64_t n_pad, int64_t k_pad,
+                     GemmParams& p, CUtensorMap* ta, CUtensorMap* tb, int* units) {
   const int64_t m_tiles = ceil_div(p.m_valid, BM);
   p.a_rows = m_tiles > 1 || p.m_valid > 64 ? 128 : p.m_valid > 32 ? 64 : 32;
   p.tile_n = m_tiles * ceil_div(p.n_valid, 32) <= device_sm_count() / 2 ? 16 : 32;
@@ -1637,12 +1658,59 @@ static int launch_long(const void* A, const void* B, int lp_dtype, int64_t m_pad
   const int half = long_half_bytes(p.a_rows, p.tile_n);
   p.stages = std::min(LONG_MAX_STAGES, (LONG_DATA_BYTES - A_BYTES + half) / (2 * half));
   p.wait_ns = wait_limit_ns();
+  *units = (int)(m_tiles * p.n_tiles);
+  if (int rc = make_tmap(ta, A, lp_dtype, m_pad, k_pad, p.a_rows)) return rc;
+  return make_tmap(tb, B, lp_dtype, n_pad, k_pad, p.tile_n);
+}
+
+template <int KIND>
+static int launch_long(const void* A, const void* B, int lp_dtype, int64_t m_pad, int64_t n_pad, int64_t k_pad,
+                       const GemmParams& p_in, cudaStream_t s) {
+  GemmParams p = p_in;
   CUtensorMap ta, tb;
-  if (int rc = make_tmap(&ta, A, lp_dtype, m_pad, k_pad, p.a_rows)) return rc;
-  if (int rc = make_tmap(&tb, B, lp_dtype, n_pad, k_pad, p.tile_n)) return rc;
+  int units;
+  if (int rc = plan_long(A, B, lp_dtype, m_pad, n_pad, k_pad, p, &ta, &tb, &units)) return rc;
   const auto kern = k_tc_gemm_long<KIND>;
   EBSD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LONG_SMEM_BYTES));
-  kern<<<(unsigned)(m_tiles * p.n_tiles), THREADS, LONG_SMEM_BYTES, s>>>(ta, tb, p);
+  kern<<<units, THREADS, LONG_SMEM_BYTES, s>>>(ta, tb, p);
+  EBSD_LAUNCH_CHECK();
+  return 0;
+}
+
+extern "C" int ebsd_gemm_nt_group(int n, const void* const* A, const int64_t* m_pad, const void* const* B,
+                                  const int64_t* n_pad, const int64_t* k_pad, float* const* C, const int64_t* ldc,
+                                  const int64_t* m_valid, const int64_t* n_valid, int* d_status, void* stream) {
+  EBSD_ARG_CHECK(n >= 0 && n <= LONG_GROUP, "ebsd_gemm_nt_group: 0..%d products", LONG_GROUP);
+  EBSD_ARG_CHECK(n == 0 || (A && m_pad && B && n_pad && k_pad && C && ldc && m_valid && n_valid),
+                 "ebsd_gemm_nt_group: null array");
+  if (n == 0) return 0;
+  LongGroup g{};
+  g.n = n;
+  int order[LONG_GROUP];
+  for (int i = 0; i < n; ++i) order[i] = i;
+  std::sort(order, order + n, [&](int i, int j) { return k_pad[i] > k_pad[j]; });
+  for (int j = 0; j < n; ++j) {
+    const int i = order[j];
+    if (int rc = check_operands(A[i], m_pad[i], B[i], n_pad[i], k_pad[i], EBSD_DT_BF16, d_status)) return rc;
+    EBSD_ARG_CHECK(C[i] != nullptr && m_valid[i] > 0 && m_valid[i] <= m_pad[i] && n_valid[i] > 0 &&
+                       n_valid[i] <= n_pad[i] && ldc[i] >= n_valid[i],
+                   "ebsd_gemm_nt_group: product %d: extents out of range", i);
+    GemmParams& p = g.p[j];
+    p.k_iters = (int)(k_pad[i] * 2 / BKB);
+    p.n_valid = n_valid[i];
+    p.C = C[i];
+    p.ldc = ldc[i];
+    p.m_valid = m_valid[i];
+    p.alpha = 1.0f;
+    p.status = d_status;
+    int units;
+    if (int rc = plan_long(A[i], B[i], EBSD_DT_BF16, m_pad[i], n_pad[i], k_pad[i], p, &g.a[j], &g.b[j], &units))
+      return rc;
+    g.first[j + 1] = g.first[j] + units;
+  }
+  EBSD_CUDA_CHECK(cudaFuncSetAttribute(k_tc_gemm_long_group, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       LONG_SMEM_BYTES));
+  k_tc_gemm_long_group<<<g.first[n], THREADS, LONG_SMEM_BYTES, as_stream(stream)>>>(g);
   EBSD_LAUNCH_CHECK();
   return 0;
 }

@@ -312,6 +312,32 @@ def gemm_nt(A, B, out, alpha: float = 1.0, accumulate: bool = False, m_valid=Non
     return status
 
 
+def gemm_nt_group(products, status: torch.Tensor) -> None:
+    """out = A @ B.T for up to 8 (A, B, out) products of bf16 rows with a long
+    K, in one launch (ebsd_gemm_nt_group): out (m, n), A with at least m rows
+    (a multiple of 128), B with at least n (a multiple of 256). Rows beyond m
+    and n need not be written."""
+    n = len(products)
+    if not n:
+        return
+    import ctypes
+
+    def arr(ctype, values):
+        return (ctype * n)(*values)
+
+    for A, B, out in products:
+        _cuda(A, "A", torch.bfloat16)
+        _cuda(B, "B", torch.bfloat16)
+        _cuda(out, "out", torch.float32)
+    i64, vp = ctypes.c_int64, ctypes.c_void_p
+    call("ebsd_gemm_nt_group", n, arr(vp, [A.data_ptr() for A, _, _ in products]),
+         arr(i64, [A.shape[0] for A, _, _ in products]), arr(vp, [B.data_ptr() for _, B, _ in products]),
+         arr(i64, [B.shape[0] for _, B, _ in products]), arr(i64, [A.shape[1] for A, _, _ in products]),
+         arr(vp, [o.data_ptr() for _, _, o in products]), arr(i64, [o.stride(0) for _, _, o in products]),
+         arr(i64, [o.shape[0] for _, _, o in products]), arr(i64, [o.shape[1] for _, _, o in products]), ptr(status),
+         _stream(products[0][0].device))
+
+
 def gemm_f32(A: torch.Tensor, B: torch.Tensor, out: torch.Tensor, alpha: float = 1.0, accumulate: bool = False,
              status=None, splits: int = 0) -> torch.Tensor:
     """out[:m, :n] = alpha * A @ B.T (+ out) from FP32 rows read as TF32

@@ -93,27 +93,32 @@ class _Conv:
         keep.update(out=out, M=M, H=H, W=W, B=B)
         return out, out32, Ho, Wo
 
-    def backward(self, dout: torch.Tensor, keep: dict, need_dx: bool) -> Optional[torch.Tensor]:
+    def backward(self, dout: torch.Tensor, keep: dict, need_dx: bool, products: list) -> Optional[torch.Tensor]:
+        """Gradient of the input (need_dx) and of the bias; the weight
+        gradient's product is appended to `products` (a network launches those
+        of its layers together)."""
         M, B, H, W = keep["M"], keep["B"], keep["H"], keep["W"]
         dev = dout.device
         s = _stream(dout)
-        g32 = torch.empty((M, self.cout), dtype=torch.float32, device=dev)
+        # ReLU gradient: rows for the column gradient, their transpose for the
+        # weight gradient, column sums for the bias
         ld16 = round_up(self.cout, 64)
-        g16 = torch.empty((M, ld16), dtype=torch.bfloat16, device=dev)
-        call("ebsd_cnn_relu_grad", ptr(dout), self.cout, ptr(keep["out"]), self.cout, M, self.cout, ptr(g32),
-             ptr(g16), ld16, s)
-        call("ebsd_cnn_col_sum", ptr(g32), M, self.cout, ptr(self.gb), s)
-        # weight gradient: (cout x K) = g^T (cout x M) . cols (M x K)
+        g16 = torch.empty((M, ld16), dtype=torch.bfloat16, device=dev) if need_dx else None
         gT = torch.empty((round_up(self.cout, 128), M), dtype=torch.bfloat16, device=dev)
-        call("ebsd_cnn_transpose", ptr(g16), 0, M, self.cout, ld16, ptr(gT), gT.shape[0], M, s)
-        colsT = torch.empty((round_up(self.K_pad, 256), M), dtype=torch.bfloat16, device=dev)
-        cols = keep["cols"] if "cols" in keep else self._im2col(keep["x"], B, H, W)
-        call("ebsd_cnn_transpose", ptr(cols), 0, M, self.K_pad, self.K_pad, ptr(colsT), colsT.shape[0], M, s)
-        kernels.gemm_nt(gT, colsT, self.gw, m_valid=self.cout, n_valid=self.K)
+        call("ebsd_cnn_relu_grad_t", ptr(dout.contiguous()), ptr(keep["out"]), M, self.cout, ptr(g16), ld16, ptr(gT), M,
+             ptr(self.gb), s)
+        # weight gradient: (cout x K) = g^T (cout x M) . cols (M x K)
+        colsT = torch.empty((round_up(self.K, 256), M), dtype=torch.bfloat16, device=dev)
+        if "cols" in keep:
+            call("ebsd_cnn_transpose", ptr(keep["cols"]), 0, M, self.K_pad, self.K_pad, ptr(colsT), colsT.shape[0], M,
+                 s)
+        else:
+            call("ebsd_cnn_im2col_t", ptr(keep["x"]), B, H, W, self.cin, ptr(colsT), M, s)
+        products.append((gT, colsT, self.gw))
         if not need_dx:
             return None
         dcols = torch.empty((M, self.K), dtype=torch.float32, device=dev)
-        kernels.gemm_nt(g16, self.w16t, dcols, m_valid=M, n_valid=self.K)
+        kernels.gemm_nt(g16, self.w16t, dcols, m_valid=M, n_valid=self.K, status=self.status)
         dx = torch.empty((B, H, W, self.cin), dtype=torch.float32, device=dev)
         call("ebsd_cnn_col2im", ptr(dcols), self.K, B, H, W, self.cin, ptr(dx), s)
         return dx
@@ -229,10 +234,12 @@ class OrientationCNN:
         dh = self.fc2.backward(dout, k2, need_dx=True)
         dfeat = self.fc1.backward(dh, k1, need_dx=True)
         d = dfeat
+        products: list = []
         for i in range(len(self.convs) - 1, -1, -1):
             conv = self.convs[i]
             keep = self._keep[i]
-            d = conv.backward(d.reshape(keep["M"], conv.cout), keep, need_dx=(i > 0))
+            d = conv.backward(d.reshape(keep["M"], conv.cout), keep, i > 0, products)
+        kernels.gemm_nt_group(products, self.convs[0].status)
 
     def adam_step(self, lr: float = 1e-3, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8, wd: float = 0.0):
         self.step_count += 1

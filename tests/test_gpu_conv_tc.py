@@ -93,3 +93,45 @@ def test_first_layer_rounds_fp32_pixels_as_the_cast_does(B, H, W, cout):
                                      b.double(), stride=2, padding=1)
     ref = torch.relu(ref).permute(0, 2, 3, 1).reshape(M, cout)
     assert (o32.double() - ref).abs().max() <= 16 * 2.0 ** -24 * 9 * 16
+
+
+@pytest.mark.parametrize("C", [1, 32, 64, 128])
+@pytest.mark.parametrize("B,H,W", [(8, 1, 1), (8, 5, 7), (16, 6, 6), (8, 16, 15)])
+def test_backward_operands(C, B, H, W):
+    """Transposed columns, the fused ReLU gradient and the column gradient's
+    scatter against torch, padding included."""
+    from ebsdtorch_b200._capi import call, ptr
+
+    Ho, Wo = (H + 1) // 2, (W + 1) // 2
+    M = B * Ho * Wo
+    g = torch.Generator().manual_seed(C + H)
+    x = torch.randn((B, H, W, C), generator=g).to(DEV).bfloat16()
+    pad = torch.nn.functional.pad(x, (0, 0, 1, 2, 1, 2))
+    taps = [pad[:, ky:ky + 2 * Ho:2, kx:kx + 2 * Wo:2] for ky in range(3) for kx in range(3)]
+    ref = torch.stack(taps, 3).reshape(M, 9 * C).t()
+    out = torch.full((9 * C + 1, M + 8), 7.0, device=DEV).bfloat16()
+    call("ebsd_cnn_im2col_t", ptr(x), B, H, W, C, ptr(out), M + 8, None)
+    assert torch.equal(out[:9 * C, :M], ref) and (out[9 * C] == 7).all() and (out[:, M:] == 7).all()
+    dcols = torch.randn((M, 9 * C), generator=g).to(DEV)
+    dx = torch.empty((B, H, W, C), device=DEV)
+    call("ebsd_cnn_col2im", ptr(dcols), 9 * C, B, H, W, C, ptr(dx), None)
+    acc = torch.zeros((B, H + 3, W + 3, C), device=DEV, dtype=torch.float64)
+    for i in range(9):
+        acc[:, i // 3:i // 3 + 2 * Ho:2, i % 3:i % 3 + 2 * Wo:2] += dcols[:, i * C:(i + 1) * C].double().view(B, Ho, Wo, C)
+    assert (dx.double() - acc[:, 1:H + 1, 1:W + 1]).abs().max() <= 8 * 4 * 2.0 ** -23 * 4
+    if C % 4:
+        return
+    dy = torch.randn((M, C), generator=g).to(DEV)
+    act = torch.relu(torch.randn((M, C), generator=g)).to(DEV).bfloat16()
+    ld16 = -(-C // 64) * 64
+    want = torch.where(act.float() > 0, dy, torch.zeros_like(dy))
+    for keep in (True, False):
+        g16 = torch.full((M, ld16), 5.0, device=DEV).bfloat16()
+        gT = torch.full((C + 1, M), 5.0, device=DEV).bfloat16()
+        db = torch.full((C,), 5.0, device=DEV)
+        call("ebsd_cnn_relu_grad_t", ptr(dy), ptr(act), M, C, ptr(g16) if keep else None, ld16, ptr(gT), M, ptr(db),
+             None)
+        if keep:
+            assert torch.equal(g16[:, :C], want.bfloat16()) and (g16[:, C:] == 0).all()
+        assert torch.equal(gT[:C], want.bfloat16().t()) and (gT[C] == 5).all()
+        assert (db.double() - want.double().sum(0)).abs().max() <= M * 2.0 ** -23 * 4

@@ -54,3 +54,26 @@ def test_store_epilogue_alignments(ldc):
             kernels.gemm_nt(A, B, out, accumulate=True, m_valid=200, n_valid=min(n, ldc))
             assert (out[:, :n].double() - 2 * ref[:, :n]).abs().max() < 1e-3
             assert (out[:, n:] == 0).all()
+
+
+def test_grouped_products_give_the_same_bits():
+    from ebsdtorch_b200 import kernels
+
+    g = torch.Generator(device=DEV).manual_seed(3)
+    shapes = [(32, 9, 8192), (64, 288, 4096), (256, 40, 64), (129, 257, 128), (1, 1, 192), (128, 16, 2112)]
+    prods, refs = [], []
+    for m, n, k in shapes:
+        A = torch.randn((-(-m // 128) * 128, k), generator=g, device=DEV).bfloat16()
+        B = torch.randn((-(-n // 256) * 256, k), generator=g, device=DEV).bfloat16()
+        prods.append((A, B, torch.zeros((m, n), device=DEV)))
+        ref = torch.zeros((m, n), device=DEV)
+        kernels.gemm_nt(A, B, ref, m_valid=m, n_valid=n, splits=B.shape[0] // 256)
+        refs.append(ref)
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    kernels.gemm_nt_group(prods, st)
+    kernels.gemm_nt_group([], st)
+    assert int(st.item()) == 0
+    for (_, _, out), ref in zip(prods, refs):
+        assert torch.equal(out, ref)
+    with pytest.raises(Exception):
+        kernels.gemm_nt_group(prods * 2, st)
