@@ -75,8 +75,11 @@ SIGNATURES = {
     "ebsd_pcfit_xcorr_table_bytes": (i64, [i32, i32]),
     "ebsd_pcfit_xcorr_tables": (i32, [i32, i32, vp, i64, vp]),
     "ebsd_pcfit_spectra": (i32, [vp, i64, i64, i32, i32, vp, vp, vp, vp]),
+    "ebsd_pcfit_spectra_quads": (i32, [vp, i64, i64, i32, i32, vp, vp, vp, vp]),
     "ebsd_pcfit_pattern_terms": (i32, [vp, i64, i32, i32, vp, vp]),
+    "ebsd_pcfit_pattern_terms_quads": (i32, [vp, i64, i32, i32, vp, vp]),
     "ebsd_pcfit_xcorr_max": (i32, [vp, i64, vp, i32, i32, i32, vp, vp, i64, vp, vp]),
+    "ebsd_pcfit_xcorr_max_quads": (i32, [vp, i64, vp, i32, i32, i32, vp, vp, i64, vp, vp]),
     "ebsd_pcfit_fold": (i32, [vp, i64, vp, vp, vp]),
     "ebsd_nlpar_weights": (i32, [vp, i32, i32, i32, vp, i32, f32, f32, f32, vp, sz, vp]),
     "ebsd_local_search": (i32, [vp, i64, i64, vp, i32, i32, vp, vp, vp, i64, vp, i32, i64, vp, vp, i32, i64, i32,
@@ -120,8 +123,8 @@ LAUNCHES_PER_CALL = {
     "ebsd_pattern_mean": 2, "ebsd_subtract_pattern": 1, "ebsd_normalize_patterns": 1, "ebsd_clahe": 1,
     "ebsd_nlpar_dists": 1, "ebsd_nlpar_average": 1,
     "ebsd_nlpar_dists_window": 1, "ebsd_nlpar_average_window": 1, "ebsd_nlpar_weights": 14,
-    "ebsd_pcfit_prep": 1, "ebsd_pcfit_reduce": 1, "ebsd_pcfit_xcorr_tables": 1, "ebsd_pcfit_spectra": 1,
-    "ebsd_pcfit_pattern_terms": 1, "ebsd_pcfit_xcorr_max": 1, "ebsd_pcfit_fold": 1,
+    "ebsd_pcfit_prep": 1, "ebsd_pcfit_reduce": 1, "ebsd_pcfit_xcorr_tables": 1, "ebsd_pcfit_spectra": 1, "ebsd_pcfit_spectra_quads": 1,
+    "ebsd_pcfit_pattern_terms": 1, "ebsd_pcfit_pattern_terms_quads": 1, "ebsd_pcfit_xcorr_max": 1, "ebsd_pcfit_xcorr_max_quads": 1, "ebsd_pcfit_fold": 1,
     "ebsd_rot6d_sym_loss": 1, "ebsd_cnn_im2col": 1, "ebsd_cnn_col2im": 1, "ebsd_cnn_bias_act": 1,
     "ebsd_cnn_conv_fwd": 1, "ebsd_cnn_im2col_t": 1, "ebsd_cnn_relu_grad_t": 1, "ebsd_gemm_nt_group": 1, "ebsd_cnn_conv_tc": 1, "ebsd_cnn_conv_c1": 1, "ebsd_cnn_conv_c1_f32": 1, "ebsd_cnn_relu_grad": 1, "ebsd_cnn_col_sum": 1,
     "ebsd_cnn_transpose": 1, "ebsd_cnn_scale_cast": 1,

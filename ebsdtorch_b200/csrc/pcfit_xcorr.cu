@@ -369,6 +369,9 @@ struct XcParams {
   int n_pats;
   int slices;
   int pp_tm;  // TMEM kernel: pairs per pass
+  // spectrum element (trig, part, ky, kx) at (2 trig + part) * part_step +
+  // (ky * WF + kx) * elem_step: planes, or quads of one (ky, kx)
+  int part_step, elem_step;
   int64_t index_base;
   unsigned long long* keys;
   int* status;
@@ -526,7 +529,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_xc_forward(const XcParams p) {
       const int im = r / g.RW, c = r - im * g.RW;
       const int part = c >= g.KOB, kx = c - part * g.KOB;
       const bool valid = r < ni * g.RW && kx < g.WF;
-      float* out = p.spec_out + (i0 + im) * (int64_t)g.spec + (int64_t)part * g.H2 * g.WF + kx;
+      float* out = p.spec_out + (i0 + im) * (int64_t)g.spec + part * p.part_step + kx * p.elem_step;
       if (t_of_warp * 128 < ni * g.RW) {
         for (int c8 = cg; c8 < g.N2 / 8; c8 += n_cg) {
           float v[8];
@@ -536,7 +539,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_xc_forward(const XcParams p) {
             for (int j = 0; j < 8; ++j) {
               const int n2 = c8 * 8 + j;
               const int trig = n2 >= g.KOA, ky = n2 - trig * g.KOA;
-              if (ky < g.H2 && trig < 2) out[((int64_t)trig * 2 * g.H2 + ky) * g.WF] = v[j];
+              if (ky < g.H2 && trig < 2) out[2 * trig * p.part_step + ky * g.WF * p.elem_step] = v[j];
             }
           }
         }
@@ -588,7 +591,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_xc_max(const XcParams p) {
   const uint32_t ca_hi = smem_u32(s.c0), ca_lo = ca_hi + p.tb.inv_a;
   const uint32_t cb_hi = smem_u32(s.c1), cb_lo = cb_hi + p.tb.inv_b;
   float* scratch = reinterpret_cast<float*>(s.a_hi);  // the pass's maps, [pair][y][x]
-  const int hw = g.H * g.W, ng = g.KOA / 8, hwf = g.H2 * g.WF;
+  const int hw = g.H * g.W, ng = g.KOA / 8, ps = p.part_step, es = p.elem_step;
   const float* pt = p.pat_terms + (int64_t)b * g.spec;
 
   float best_v[POS];
@@ -605,18 +608,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_xc_max(const XcParams p) {
     // stage A operand: rows (pair, part, kx), K = [E part | O part] over ky
     for (int it = tid; it < np * g.WF * ng; it += THREADS) {
       const int pr = it / (g.WF * ng), rem = it - pr * g.WF * ng, grp = rem / g.WF, kx = rem - grp * g.WF;
-      const float* cs = p.sim_spec + (s0 + pr) * (int64_t)g.spec + kx;
+      const float* cs = p.sim_spec + (s0 + pr) * (int64_t)g.spec + kx * es;
       float er[8], ei[8], orr[8], oi[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int ky = grp * 8 + j;
         er[j] = ei[j] = orr[j] = oi[j] = 0.0f;
         if (ky < g.H2) {
-          const int o = ky * g.WF;
-          const float a = __ldg(cs + o), bi = __ldg(cs + hwf + o);                // Cc
-          const float c = __ldg(cs + 2 * hwf + o), d = __ldg(cs + 3 * hwf + o);   // Ss
-          const float e = __ldg(pt + o + kx), f = __ldg(pt + hwf + o + kx);       // Pe
-          const float gg = __ldg(pt + 2 * hwf + o + kx), h = __ldg(pt + 3 * hwf + o + kx);  // Po
+          const int o = ky * g.WF * es, ot = o + kx * es;
+          const float a = __ldg(cs + o), bi = __ldg(cs + ps + o);              // Cc
+          const float c = __ldg(cs + 2 * ps + o), d = __ldg(cs + 3 * ps + o);  // Ss
+          const float e = __ldg(pt + ot), f = __ldg(pt + ps + ot);             // Pe
+          const float gg = __ldg(pt + 2 * ps + ot), h = __ldg(pt + 3 * ps + ot);  // Po
           er[j] = a * e - bi * f + c * h + d * gg;
           ei[j] = a * f + bi * e - c * gg + d * h;
           orr[j] = a * gg - bi * h + c * f + d * e;
@@ -722,7 +725,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_xc_max(const XcParams p) {
 //            chunk's 8 K elements: hi Bhi + lo Bhi + hi Blo, the 3-term split;
 //   epilogue each thread owns lane y and CPT x chunks; the max over the
 //            pass's pairs and over passes stays in its registers.
-template <int CPT>  // x chunks of 8 per thread: NB / 8 <= 4 CPT
+// QUADS: the four values of a (ky, kx) are one 16-byte load. Operand formation
+// waits on its loads (16 lines of spectrum and terms per thread, from L2), so
+// their number counts: 64 loads of 4 bytes took about 0.20 of a batch's 0.507 ms
+// (16 patterns, 78 x 78 px, 1,024 simulated ones); 16 of 16 bytes: 0.465 in all.
+template <int CPT, bool QUADS>  // x chunks of 8 per thread: NB / 8 <= 4 CPT
 __global__ void __launch_bounds__(THREADS, 1) k_xc_max_tm(const XcParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_s = smem_u32(smem_raw);
@@ -793,7 +800,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_xc_max_tm(const XcParams p) {
     for (int k = 0; k < 2; ++k) {
       if (it_pr[k] >= np) continue;
       const int pr = it_pr[k], grp = it_grp[k], kx = it_kx[k];
-      const float* cs = p.sim_spec + (s0 + pr) * (int64_t)g.spec + kx;
+      const float* cs = p.sim_spec + (s0 + pr) * (int64_t)g.spec + (QUADS ? 4 * kx : kx);
       float er[8], ei[8], orr[8], noi[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -801,10 +808,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_xc_max_tm(const XcParams p) {
         er[j] = ei[j] = orr[j] = noi[j] = 0.0f;
         if (ky < g.H2) {
           const int o = ky * g.WF;
-          const float a = __ldg(cs + o), bi = __ldg(cs + hwf + o);                // Cc
-          const float c = __ldg(cs + 2 * hwf + o), d = __ldg(cs + 3 * hwf + o);   // Ss
-          const float e = __ldg(pt + o + kx), f = __ldg(pt + hwf + o + kx);       // Pe
-          const float gg = __ldg(pt + 2 * hwf + o + kx), h = __ldg(pt + 3 * hwf + o + kx);  // Po
+          float4 cv, pv;  // (Cc, Ss) of the simulated pattern, (Pe, Po) of the experimental one
+          if constexpr (QUADS) {
+            cv = __ldg(reinterpret_cast<const float4*>(cs) + o);
+            pv = __ldg(reinterpret_cast<const float4*>(pt) + o + kx);
+          } else {
+            cv = make_float4(__ldg(cs + o), __ldg(cs + hwf + o), __ldg(cs + 2 * hwf + o), __ldg(cs + 3 * hwf + o));
+            pv = make_float4(__ldg(pt + o + kx), __ldg(pt + hwf + o + kx), __ldg(pt + 2 * hwf + o + kx),
+                             __ldg(pt + 3 * hwf + o + kx));
+          }
+          const float a = cv.x, bi = cv.y, c = cv.z, d = cv.w, e = pv.x, f = pv.y, gg = pv.z, h = pv.w;
           er[j] = a * e - bi * f + c * h + d * gg;
           ei[j] = a * f + bi * e - c * gg + d * h;
           orr[j] = a * gg - bi * h + c * f + d * e;
@@ -819,25 +832,37 @@ __global__ void __launch_bounds__(THREADS, 1) k_xc_max_tm(const XcParams p) {
       put8(s.a_hi, s.a_lo, p.buf_rows, row_im, g.KOA + grp * 8, orr);
     }
   };
+  // Descriptors advance by additions to their address field (16-byte units);
+  // one thread issues, and its instructions per MMA add up.
+  const uint64_t ca_hi_d = smem_desc_sw128(ca_hi), ca_lo_d = smem_desc_sw128(ca_lo);
+  const uint64_t d_hi_d = smem_desc_sw128(d_hi), d_lo_d = smem_desc_sw128(d_lo);
+  const uint64_t cp_d = smem_desc_sw128(cp), cq_d = smem_desc_sw128(cq);
   auto issue_a = [&](int np) {
     const int n = np * g.RW;
     const uint32_t idesc = xc_idesc(n);
+    const uint32_t plane = (uint32_t)p.buf_rows * 8u;
+    uint32_t acc = 0;
     for (int ks = 0; ks < g.KSA; ++ks) {
-      const uint32_t aoff = (uint32_t)(ks >> 2) * 128u * 128u + (uint32_t)(ks & 3) * 32u;
-      const uint32_t boff = (uint32_t)(ks >> 2) * (uint32_t)p.buf_rows * 128u + (uint32_t)(ks & 3) * 32u;
-      tc_mma<0>(da, smem_desc_sw128(ca_hi + aoff), smem_desc_sw128(d_hi + boff), idesc, ks > 0 ? 1u : 0u);
-      tc_mma<0>(da, smem_desc_sw128(ca_hi + aoff), smem_desc_sw128(d_lo + boff), idesc, 1u);
-      tc_mma<0>(da, smem_desc_sw128(ca_lo + aoff), smem_desc_sw128(d_hi + boff), idesc, 1u);
+      const uint32_t aoff = (uint32_t)(ks >> 2) * (128u * 8u) + (uint32_t)(ks & 3) * 2u;
+      const uint32_t boff = (uint32_t)(ks >> 2) * plane + (uint32_t)(ks & 3) * 2u;
+      tc_mma<0>(da, ca_hi_d + aoff, d_hi_d + boff, idesc, acc);
+      tc_mma<0>(da, ca_hi_d + aoff, d_lo_d + boff, idesc, 1u);
+      tc_mma<0>(da, ca_lo_d + aoff, d_hi_d + boff, idesc, 1u);
+      acc = 1;
     }
   };
   auto issue_b = [&](int np) {
-    const uint32_t idesc = xc_idesc(g.NB);
+    const uint32_t idesc = xc_idesc(g.NB), plane = (uint32_t)g.NB * 8u;
     for (int pr = 0; pr < np; ++pr) {
+      const uint32_t d = db + (uint32_t)(pr * g.NB);
+      uint32_t a = da + (uint32_t)(pr * g.RW), acc = 0;
+#pragma unroll 2
       for (int q = 0; q < rw8; ++q) {
-        const uint32_t boff = (uint32_t)((16 * q) >> 6) * (uint32_t)g.NB * 128u + (uint32_t)(q & 3) * 32u;
-        const uint32_t a = da + (uint32_t)(pr * g.RW + 8 * q);
-        tc_mma_ta(db + (uint32_t)(pr * g.NB), a, smem_desc_sw128(cp + boff), idesc, q > 0 ? 1u : 0u);
-        tc_mma_ta(db + (uint32_t)(pr * g.NB), a, smem_desc_sw128(cq + boff), idesc, 1u);
+        const uint32_t boff = (uint32_t)(q >> 2) * plane + (uint32_t)(q & 3) * 2u;
+        tc_mma_ta(d, a, cp_d + boff, idesc, acc);
+        tc_mma_ta(d, a, cq_d + boff, idesc, 1u);
+        acc = 1;
+        a += 8;
       }
     }
   };
@@ -967,7 +992,8 @@ __global__ void k_xc_fold(unsigned long long* __restrict__ keys, int64_t n, floa
 // Pattern terms from pattern spectra: Pe = 2 conj(Cc), Po = 2 i conj(Ss),
 // with weight 1 instead of 2 at ky = 0 and at ky = H/2 (H even), where the
 // pair (ky, H - ky) is a single frequency.
-__global__ void k_xc_pattern_terms(const float* __restrict__ spec, int64_t n, Geo g, float* __restrict__ out) {
+__global__ void k_xc_pattern_terms(const float* __restrict__ spec, int64_t n, Geo g, int ps, int es,
+                                   float* __restrict__ out) {
   const int64_t hwf = (int64_t)g.H2 * g.WF;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n * hwf) return;
@@ -976,11 +1002,12 @@ __global__ void k_xc_pattern_terms(const float* __restrict__ spec, int64_t n, Ge
   const float w = (ky == 0 || 2 * ky == g.H) ? 1.0f : 2.0f;
   const float* sp = spec + im * g.spec;
   float* o = out + im * g.spec;
-  const float ccr = sp[e], cci = sp[hwf + e], ssr = sp[2 * hwf + e], ssi = sp[3 * hwf + e];
-  o[e] = w * ccr;
-  o[hwf + e] = -w * cci;
-  o[2 * hwf + e] = w * ssi;
-  o[3 * hwf + e] = w * ssr;
+  const int64_t q = e * es;
+  const float ccr = sp[q], cci = sp[ps + q], ssr = sp[2 * ps + q], ssi = sp[3 * ps + q];
+  o[q] = w * ccr;
+  o[ps + q] = -w * cci;
+  o[2 * ps + q] = w * ssi;
+  o[3 * ps + q] = w * ssr;
 }
 
 }  // namespace xc
@@ -1051,7 +1078,7 @@ int sm_count() {
   return n;
 }
 
-XcParams base_params(const Plan& pl, const void* tables, int* status) {
+XcParams base_params(const Plan& pl, const void* tables, int* status, bool quads) {
   XcParams p{};
   p.g = pl.g;
   p.mt = pl.mt;
@@ -1063,6 +1090,8 @@ XcParams base_params(const Plan& pl, const void* tables, int* status) {
   p.tables = static_cast<const uint8_t*>(tables);
   p.status = status;
   p.wait_ns = wait_limit_ns();
+  p.part_step = quads ? 1 : pl.g.H2 * pl.g.WF;
+  p.elem_step = quads ? 4 : 1;
   return p;
 }
 
@@ -1089,15 +1118,15 @@ extern "C" int ebsd_pcfit_xcorr_tables(int hp, int wp, void* tables, int64_t byt
   return 0;
 }
 
-extern "C" int ebsd_pcfit_spectra(const float* images, int64_t ld, int64_t n, int hp, int wp, const void* tables,
-                                  float* spectra, int* status, void* stream) {
+static int run_spectra(const float* images, int64_t ld, int64_t n, int hp, int wp, const void* tables, float* spectra,
+                       bool quads, int* status, void* stream) {
   Plan pl;
   EBSD_ARG_CHECK(make_plan(hp, wp, pl), "enlarged detector %d x %d not supported (2..%d each)", hp, wp, MAX_HW);
   EBSD_ARG_CHECK(images && tables && spectra && status, "ebsd_pcfit_spectra: null pointer");
   EBSD_ARG_CHECK(n >= 0 && ld >= (int64_t)hp * wp, "bad image count or leading dimension");
   EBSD_ARG_CHECK(((uintptr_t)tables & 15) == 0, "tables must be 16-byte aligned");
   if (n == 0) return 0;
-  XcParams p = base_params(pl, tables, status);
+  XcParams p = base_params(pl, tables, status, quads);
   p.img = images;
   p.ld_img = ld;
   p.n_img = n;
@@ -1110,22 +1139,23 @@ extern "C" int ebsd_pcfit_spectra(const float* images, int64_t ld, int64_t n, in
   return 0;
 }
 
-extern "C" int ebsd_pcfit_pattern_terms(const float* spectra, int64_t n, int hp, int wp, float* terms,
-                                        void* stream) {
+static int run_pattern_terms(const float* spectra, int64_t n, int hp, int wp, float* terms, bool quads,
+                             void* stream) {
   Plan pl;
   EBSD_ARG_CHECK(make_plan(hp, wp, pl), "enlarged detector %d x %d not supported (2..%d each)", hp, wp, MAX_HW);
   EBSD_ARG_CHECK(spectra && terms, "ebsd_pcfit_pattern_terms: null pointer");
   EBSD_ARG_CHECK(n >= 0, "bad pattern count");
   const int64_t e = n * pl.g.H2 * pl.g.WF;
   if (e == 0) return 0;
-  k_xc_pattern_terms<<<(unsigned)((e + 255) / 256), 256, 0, as_stream(stream)>>>(spectra, n, pl.g, terms);
+  k_xc_pattern_terms<<<(unsigned)((e + 255) / 256), 256, 0, as_stream(stream)>>>(spectra, n, pl.g, quads ? 1 : pl.g.H2 * pl.g.WF,
+                                                                                    quads ? 4 : 1, terms);
   EBSD_LAUNCH_CHECK();
   return 0;
 }
 
-extern "C" int ebsd_pcfit_xcorr_max(const float* sim_spectra, int64_t n_sims, const float* pat_terms, int n_pats,
-                                    int hp, int wp, const void* tables, unsigned long long* keys,
-                                    int64_t index_base, int* status, void* stream) {
+static int run_xcorr_max(const float* sim_spectra, int64_t n_sims, const float* pat_terms, int n_pats, int hp, int wp,
+                         const void* tables, unsigned long long* keys, int64_t index_base, bool quads, int* status,
+                         void* stream) {
   Plan pl;
   EBSD_ARG_CHECK(make_plan(hp, wp, pl), "enlarged detector %d x %d not supported (2..%d each)", hp, wp, MAX_HW);
   EBSD_ARG_CHECK(sim_spectra && pat_terms && tables && keys && status, "ebsd_pcfit_xcorr_max: null pointer");
@@ -1133,7 +1163,9 @@ extern "C" int ebsd_pcfit_xcorr_max(const float* sim_spectra, int64_t n_sims, co
   EBSD_ARG_CHECK(index_base >= 0 && index_base + n_sims < (int64_t)UINT32_MAX, "index range exceeds 32 bits");
   EBSD_ARG_CHECK(((uintptr_t)tables & 15) == 0, "tables must be 16-byte aligned");
   if (n_sims == 0 || n_pats == 0) return 0;
-  XcParams p = base_params(pl, tables, status);
+  EBSD_ARG_CHECK(!quads || (((uintptr_t)sim_spectra | (uintptr_t)pat_terms) & 15) == 0,
+                 "ebsd_pcfit_xcorr_max_quads: spectra must be 16-byte aligned");
+  XcParams p = base_params(pl, tables, status, quads);
   p.sim_spec = sim_spectra;
   p.n_sims = n_sims;
   p.pat_terms = pat_terms;
@@ -1152,11 +1184,13 @@ extern "C" int ebsd_pcfit_xcorr_max(const float* sim_spectra, int64_t n_sims, co
     p.buf_planes = pl.g.KPA;
     p.buf_bytes = p.buf_rows * 128 * p.buf_planes;
     switch (pl.cpt) {
-#define EBSD_XC_TM_CASE(CPT)                                                                                       \
-  case CPT:                                                                                                         \
-    EBSD_CUDA_CHECK(cudaFuncSetAttribute(k_xc_max_tm<CPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem_tm)); \
-    k_xc_max_tm<CPT><<<(int)grid, THREADS, pl.smem_tm, s>>>(p);                                                     \
-    break;
+#define EBSD_XC_TM_CASE(CPT)                                                                                  \
+  case CPT: {                                                                                                  \
+    const auto fn = quads ? k_xc_max_tm<CPT, true> : k_xc_max_tm<CPT, false>;                                  \
+    EBSD_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem_tm));        \
+    fn<<<(int)grid, THREADS, pl.smem_tm, s>>>(p);                                                              \
+    break;                                                                                                     \
+  }
       EBSD_XC_TM_CASE(1)
       EBSD_XC_TM_CASE(2)
       EBSD_XC_TM_CASE(3)
@@ -1185,6 +1219,39 @@ extern "C" int ebsd_pcfit_xcorr_max(const float* sim_spectra, int64_t n_sims, co
   }
   EBSD_LAUNCH_CHECK();
   return 0;
+}
+
+extern "C" int ebsd_pcfit_spectra(const float* images, int64_t ld, int64_t n, int hp, int wp, const void* tables,
+                                  float* spectra, int* status, void* stream) {
+  return run_spectra(images, ld, n, hp, wp, tables, spectra, false, status, stream);
+}
+
+extern "C" int ebsd_pcfit_spectra_quads(const float* images, int64_t ld, int64_t n, int hp, int wp,
+                                        const void* tables, float* spectra, int* status, void* stream) {
+  return run_spectra(images, ld, n, hp, wp, tables, spectra, true, status, stream);
+}
+
+extern "C" int ebsd_pcfit_pattern_terms(const float* spectra, int64_t n, int hp, int wp, float* terms,
+                                        void* stream) {
+  return run_pattern_terms(spectra, n, hp, wp, terms, false, stream);
+}
+
+extern "C" int ebsd_pcfit_pattern_terms_quads(const float* spectra, int64_t n, int hp, int wp, float* terms,
+                                              void* stream) {
+  return run_pattern_terms(spectra, n, hp, wp, terms, true, stream);
+}
+
+extern "C" int ebsd_pcfit_xcorr_max(const float* sim_spectra, int64_t n_sims, const float* pat_terms, int n_pats,
+                                    int hp, int wp, const void* tables, unsigned long long* keys,
+                                    int64_t index_base, int* status, void* stream) {
+  return run_xcorr_max(sim_spectra, n_sims, pat_terms, n_pats, hp, wp, tables, keys, index_base, false, status,
+                       stream);
+}
+
+extern "C" int ebsd_pcfit_xcorr_max_quads(const float* sim_spectra, int64_t n_sims, const float* pat_terms,
+                                          int n_pats, int hp, int wp, const void* tables, unsigned long long* keys,
+                                          int64_t index_base, int* status, void* stream) {
+  return run_xcorr_max(sim_spectra, n_sims, pat_terms, n_pats, hp, wp, tables, keys, index_base, true, status, stream);
 }
 
 extern "C" int ebsd_pcfit_fold(unsigned long long* keys, int64_t n, float* best, int64_t* best_idx, void* stream) {

@@ -221,8 +221,8 @@ MAX_SIM_BYTES = 2 << 30
 def _search_dft(mp_t, padded, quats, pix64, z_vals, tilt, sec_tilt, det, bs, batch_local, best, best_idx, stream):
     """The search with the correlation in the project's kernels: spectra of
     the patterns and of each projected dictionary sub-batch
-    (ebsd_pcfit_spectra), the per-batch max over all shifts
-    (ebsd_pcfit_xcorr_max) and the running best (ebsd_pcfit_fold)."""
+    (ebsd_pcfit_spectra_quads), the per-batch max over all shifts
+    (ebsd_pcfit_xcorr_max_quads) and the running best (ebsd_pcfit_fold)."""
     dev = padded.device
     B, hp, wp = padded.shape
     n_dict = quats.shape[0]
@@ -231,9 +231,9 @@ def _search_dft(mp_t, padded, quats, pix64, z_vals, tilt, sec_tilt, det, bs, bat
     call("ebsd_pcfit_xcorr_tables", hp, wp, ptr(tables), tables.numel(), stream)
     status = torch.zeros(1, dtype=torch.int32, device=dev)
     pspec = torch.empty((B, spec_len), dtype=torch.float32, device=dev)
-    call("ebsd_pcfit_spectra", ptr(padded), hp * wp, B, hp, wp, ptr(tables), ptr(pspec), ptr(status), stream)
+    call("ebsd_pcfit_spectra_quads", ptr(padded), hp * wp, B, hp, wp, ptr(tables), ptr(pspec), ptr(status), stream)
     terms = torch.empty_like(pspec)
-    call("ebsd_pcfit_pattern_terms", ptr(pspec), B, hp, wp, ptr(terms), stream)
+    call("ebsd_pcfit_pattern_terms_quads", ptr(pspec), B, hp, wp, ptr(terms), stream)
     keys = torch.zeros((B * hp * wp,), dtype=torch.int64, device=dev)
     sub = max(1, min(bs, n_dict, MAX_SIM_BYTES // (hp * wp * 4)))
     sims = torch.empty((sub, hp * wp), dtype=torch.float32, device=dev)
@@ -247,8 +247,8 @@ def _search_dft(mp_t, padded, quats, pix64, z_vals, tilt, sec_tilt, det, bs, bat
                 n = min(sub, j_end - s)
                 kernels.project(mp_t, rays, quats[s:s + n], RowBuffers(f32=sims[:n]), subtract_mean=False,
                                quads=quads)
-                call("ebsd_pcfit_spectra", ptr(sims), hp * wp, n, hp, wp, ptr(tables), ptr(spec), ptr(status), stream)
-                call("ebsd_pcfit_xcorr_max", ptr(spec), n, ptr(terms), B, hp, wp, ptr(tables), ptr(keys),
+                call("ebsd_pcfit_spectra_quads", ptr(sims), hp * wp, n, hp, wp, ptr(tables), ptr(spec), ptr(status), stream)
+                call("ebsd_pcfit_xcorr_max_quads", ptr(spec), n, ptr(terms), B, hp, wp, ptr(tables), ptr(keys),
                      (s - j) if batch_local else s, ptr(status), stream)
             call("ebsd_pcfit_fold", ptr(keys), keys.numel(), ptr(best[zi]), ptr(best_idx[zi]), stream)
     if int(status.item()) != 0:

@@ -350,11 +350,13 @@ int ebsd_match_topk_noalloc(const void* queries_lp, int64_t n_queries, int64_t n
 int ebsd_gemm_nt(const void* A, int64_t m_pad, const void* B, int64_t n_pad, int64_t k_pad,
                  int lp_dtype, float alpha, int accumulate, float* C, int64_t ldc, int64_t m_valid,
                  int64_t n_valid, int splits, int* d_status, void* stream);
-/* Up to 8 such bf16 products with a long K in one launch (alpha 1, no
- * accumulation): C[i] (m_valid[i] x n_valid[i], row stride ldc[i]). */
-int ebsd_gemm_nt_group(int n, const void* const* A, const int64_t* m_pad, const void* const* B, const int64_t* n_pad,
-                       const int64_t* k_pad, float* const* C, const int64_t* ldc, const int64_t* m_valid,
-                       const int64_t* n_valid, int* d_status, void* stream);
+/* Up to 8 bf16 products A B^T with a long K in one launch, from operands
+ * blocked by 64 of K: A[i] is (k / 64) x a_rows x 64, B[i] (k / 64) x b_rows x
+ * 64, 16-byte aligned, C[i] (m x n_cols, row stride ldc); the sums run in the
+ * order of ebsd_gemm_nt. */
+int ebsd_gemm_nt_group(int n, const void* const* A, const int64_t* a_rows, const void* const* B,
+                       const int64_t* b_rows, const int64_t* k, float* const* C, const int64_t* ldc, const int64_t* m,
+                       const int64_t* n_cols, int* d_status, void* stream);
 
 /* C (m x n, row stride ldc) = alpha * A B^T (+ C if accumulate) from FP32
  * rows A (m x k, stride lda) and B (n x k, stride ldb), read as TF32
@@ -518,6 +520,15 @@ int ebsd_pcfit_pattern_terms(const float* spectra, int64_t n, int padded_h, int 
 int ebsd_pcfit_xcorr_max(const float* sim_spectra, int64_t n_sims, const float* pattern_terms, int n_patterns,
                          int padded_h, int padded_w, const void* tables, unsigned long long* keys,
                          int64_t index_base, int* status, void* stream);
+/* The same three with quads: [ky][kx][trig][part], so that the correlation
+ * reads 16 bytes at a time (spectra and terms 16-byte aligned). */
+int ebsd_pcfit_spectra_quads(const float* images, int64_t ld, int64_t n, int padded_h, int padded_w,
+                             const void* tables, float* spectra, int* status, void* stream);
+int ebsd_pcfit_pattern_terms_quads(const float* spectra, int64_t n, int padded_h, int padded_w, float* terms,
+                                   void* stream);
+int ebsd_pcfit_xcorr_max_quads(const float* sim_spectra, int64_t n_sims, const float* pat_terms, int n_patterns,
+                               int padded_h, int padded_w, const void* tables, unsigned long long* keys,
+                               int64_t index_base, int* status, void* stream);
 int ebsd_pcfit_fold(unsigned long long* keys, int64_t n, float* best, int64_t* best_index, void* stream);
 
 /* ---- local dictionary search around orientation proposals --------------------
@@ -590,14 +601,16 @@ int ebsd_cnn_conv_fwd(const void* w16, int64_t cout_pad, const void* cols, int64
 int ebsd_cnn_conv_supported(int cin, int cout, int width);
 int ebsd_cnn_conv_tc(const void* x, int batch, int height, int width, int cin, const void* w16, int64_t ldw,
                      const float* bias, int cout, int relu, void* out16, float* out32, int* d_status, void* stream);
-/* The columns transposed, (9 C) x M with row stride ld (M = B Ho Wo pixels, a
- * multiple of 8): C = 1, 32 or a multiple of 64, 16-byte aligned pointers. */
-int ebsd_cnn_im2col_t(const void* x, int B, int H, int W, int C, void* out, int64_t ld, void* stream);
+/* The columns transposed and blocked by 64 pixels: out[m / 64][9 C rows of
+ * `rows`][m % 64] for M = B Ho Wo pixels, a multiple of 64; C = 1, 32 or a
+ * multiple of 64, 16-byte aligned pointers. */
+int ebsd_cnn_im2col_t(const void* x, int B, int H, int W, int C, void* out, int64_t rows, void* stream);
 /* g = dy * (act > 0) of a layer of C channels (a multiple of 4) in one pass:
  * bf16 rows g16 (may be null; row stride ld16, zero beyond C), the bf16
- * transpose gT (C x M, row stride ld_t) and the column sums db. */
+ * transpose blocked by 64 pixels gT[m / 64][C of `rows`][m % 64] (M a multiple
+ * of 64) and the column sums db. */
 int ebsd_cnn_relu_grad_t(const float* dy, const void* act, int64_t M, int C, void* g16, int64_t ld16, void* gT,
-                         int64_t ld_t, float* db, void* stream);
+                         int64_t rows, float* db, void* stream);
 int ebsd_cnn_bias_act(const float* y, int64_t ldy, const float* bias, int64_t M, int C, int relu, void* out,
                       int64_t ld_out, float* out32, void* stream);
 int ebsd_cnn_relu_grad(const float* dy, int64_t ldy, const void* act, int64_t lda, int64_t M, int C, float* g32,
