@@ -181,14 +181,16 @@ __global__ void __launch_bounds__(256) k_conv_c1(const T* __restrict__ x, int H,
   }
 }
 
-// out[(ky, kx, c), m] = x[b, 2 oy - 1 + ky, 2 ox - 1 + kx, c] for output pixel
-// m = (b, oy, ox): the columns of k_im2col, transposed (a weight gradient's
-// operand), straight from the activations. Block: 64 pixels x up to 64 channels
-// of one tap through shared memory, 16-byte loads and stores.
+// out[m / 64][(ky, kx, c)][m % 64] = x[b, 2 oy - 1 + ky, 2 ox - 1 + kx, c] for
+// output pixel m = (b, oy, ox): the columns of k_im2col, transposed (a weight
+// gradient's operand) and blocked by 64 pixels, so that a stage of the product
+// is one piece of memory (as rows of M pixels, 2 MB apart, its copies took 7
+// cycles a row). Straight from the activations. Block: 64 pixels x up to 64
+// channels of one tap through shared memory, 16-byte loads and stores.
 constexpr int kTrPix = 64, kTrPitch = kTrPix + 8;
 
 __global__ void __launch_bounds__(256) k_im2col_t(const __nv_bfloat16* __restrict__ x, int H, int W, int C, int Ho,
-                                                  int Wo, int64_t M, __nv_bfloat16* __restrict__ out, int64_t ld) {
+                                                  int Wo, int64_t M, __nv_bfloat16* __restrict__ out, int64_t rows) {
   __shared__ __align__(16) __nv_bfloat16 tile[64 * kTrPitch];
   const int cw = min(C, 64), blocks_c = C / cw;
   const int tap = blockIdx.y / blocks_c, c0 = (blockIdx.y % blocks_c) * cw;
@@ -215,15 +217,14 @@ __global__ void __launch_bounds__(256) k_im2col_t(const __nv_bfloat16* __restric
   __syncthreads();
   for (int i = threadIdx.x; i < cw * 8; i += 256) {
     const int c = i >> 3, j = i & 7;
-    if (m0 + 8 * j < M)
-      *reinterpret_cast<uint4*>(out + ((int64_t)tap * C + c0 + c) * ld + m0 + 8 * j) =
-          *reinterpret_cast<const uint4*>(tile + c * kTrPitch + 8 * j);
+    *reinterpret_cast<uint4*>(out + ((int64_t)blockIdx.x * rows + (int64_t)tap * C + c0 + c) * 64 + 8 * j) =
+        *reinterpret_cast<const uint4*>(tile + c * kTrPitch + 8 * j);
   }
 }
 
 // The same for a single channel: eight pixels of a tap per thread.
 __global__ void k_im2col_t1(const __nv_bfloat16* __restrict__ x, int H, int W, int Ho, int Wo, int64_t M,
-                            __nv_bfloat16* __restrict__ out, int64_t ld) {
+                            __nv_bfloat16* __restrict__ out, int64_t rows) {
   const int tap = blockIdx.y, hw = Ho * Wo;
   const int64_t m0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (m0 >= M) return;
@@ -237,17 +238,17 @@ __global__ void k_im2col_t1(const __nv_bfloat16* __restrict__ x, int H, int W, i
     v[e] = (m < M && iy >= 0 && iy < H && ix >= 0 && ix < W) ? x[((int64_t)b * H + iy) * W + ix]
                                                              : __float2bfloat16_rn(0.f);
   }
-  *reinterpret_cast<uint4*>(out + tap * ld + m0) = *reinterpret_cast<const uint4*>(v);
+  *reinterpret_cast<uint4*>(out + ((m0 >> 6) * rows + tap) * 64 + (m0 & 63)) = *reinterpret_cast<const uint4*>(v);
 }
 
 // g = dy * (act > 0) of a convolution layer in one pass over its pixels: bf16
 // rows g16 (optional, row stride ld16, columns C .. ld16 zero), the bf16
-// transpose gT (C rows of ld_t) and the column sums added to db. Block: 64
+// transpose gT (blocked as in k_im2col_t) and the column sums added to db. Block: 64
 // pixels x 64 channels through shared memory, several pixel tiles per block.
 __global__ void __launch_bounds__(256) k_relu_grad_t(const float* __restrict__ dy,
                                                      const __nv_bfloat16* __restrict__ act, int64_t M, int C,
                                                      __nv_bfloat16* __restrict__ g16, int64_t ld16,
-                                                     __nv_bfloat16* __restrict__ gT, int64_t ld_t,
+                                                     __nv_bfloat16* __restrict__ gT, int64_t rows,
                                                      float* __restrict__ db) {
   __shared__ __align__(16) __nv_bfloat16 tile[64 * kTrPitch];
   __shared__ float sums[64];
@@ -283,9 +284,8 @@ __global__ void __launch_bounds__(256) k_relu_grad_t(const float* __restrict__ d
     __syncthreads();
     for (int i = threadIdx.x; i < cw * 8; i += 256) {
       const int c = i >> 3, j = i & 7;
-      if (m0 + 8 * j < M)
-        *reinterpret_cast<uint4*>(gT + (int64_t)(c0 + c) * ld_t + m0 + 8 * j) =
-            *reinterpret_cast<const uint4*>(tile + c * kTrPitch + 8 * j);
+      *reinterpret_cast<uint4*>(gT + ((m0 >> 6) * rows + c0 + c) * 64 + 8 * j) =
+          *reinterpret_cast<const uint4*>(tile + c * kTrPitch + 8 * j);
     }
   }
   __syncthreads();
@@ -585,38 +585,38 @@ extern "C" int ebsd_cnn_col2im(const float* dcols, int64_t ld, int B, int H, int
   return 0;
 }
 
-extern "C" int ebsd_cnn_im2col_t(const void* x, int B, int H, int W, int C, void* out, int64_t ld, void* stream) {
+extern "C" int ebsd_cnn_im2col_t(const void* x, int B, int H, int W, int C, void* out, int64_t rows, void* stream) {
   const int Ho = (H + 1) / 2, Wo = (W + 1) / 2;
   const int64_t M = (int64_t)B * Ho * Wo;
   EBSD_ARG_CHECK(x && out && B > 0 && H > 0 && W > 0, "ebsd_cnn_im2col_t: bad arguments");
   EBSD_ARG_CHECK(C == 1 || C == 32 || C % 64 == 0, "ebsd_cnn_im2col_t: %d channels not 1, 32 or a multiple of 64", C);
-  EBSD_ARG_CHECK(M % 8 == 0 && ld >= M && ld % 8 == 0, "ebsd_cnn_im2col_t: pixel counts must be multiples of 8");
+  EBSD_ARG_CHECK(M % 64 == 0 && rows >= 9 * C, "ebsd_cnn_im2col_t: pixels must be a multiple of 64, rows at least 9 C");
   EBSD_ARG_CHECK(((uintptr_t)x & 15) == 0 && ((uintptr_t)out & 15) == 0, "ebsd_cnn_im2col_t: pointers not 16-byte aligned");
   EBSD_ARG_CHECK(ceil_div(M, kTrPix) < INT32_MAX, "ebsd_cnn_im2col_t: too many pixels");
   const auto* xb = reinterpret_cast<const __nv_bfloat16*>(x);
   auto* ob = reinterpret_cast<__nv_bfloat16*>(out);
   if (C == 1)
-    k_im2col_t1<<<dim3(ceil_div(M, 8 * 256), 9), 256, 0, CNN_STREAM>>>(xb, H, W, Ho, Wo, M, ob, ld);
+    k_im2col_t1<<<dim3(ceil_div(M, 8 * 256), 9), 256, 0, CNN_STREAM>>>(xb, H, W, Ho, Wo, M, ob, rows);
   else
     k_im2col_t<<<dim3(ceil_div(M, kTrPix), 9 * (C / std::min(C, 64))), 256, 0, CNN_STREAM>>>(xb, H, W, C, Ho, Wo, M,
-                                                                                            ob, ld);
+                                                                                            ob, rows);
   EBSD_LAUNCH_CHECK();
   return 0;
 }
 
 extern "C" int ebsd_cnn_relu_grad_t(const float* dy, const void* act, int64_t M, int C, void* g16, int64_t ld16,
-                                    void* gT, int64_t ld_t, float* db, void* stream) {
+                                    void* gT, int64_t rows, float* db, void* stream) {
   EBSD_ARG_CHECK(dy && act && gT && db && M > 0 && C > 0 && C % 4 == 0, "ebsd_cnn_relu_grad_t: bad arguments");
-  EBSD_ARG_CHECK(M % 8 == 0 && ld_t >= M && ld_t % 8 == 0, "ebsd_cnn_relu_grad_t: pixel counts must be multiples of 8");
+  EBSD_ARG_CHECK(M % 64 == 0 && rows >= C, "ebsd_cnn_relu_grad_t: pixels must be a multiple of 64, rows at least C");
   EBSD_ARG_CHECK(!g16 || (ld16 >= C && ld16 % 4 == 0), "ebsd_cnn_relu_grad_t: bad ld16");
   EBSD_ARG_CHECK((((uintptr_t)dy | (uintptr_t)act | (uintptr_t)g16 | (uintptr_t)gT) & 15) == 0,
                  "ebsd_cnn_relu_grad_t: pointers not 16-byte aligned");
   EBSD_CUDA_CHECK(cudaMemsetAsync(db, 0, sizeof(float) * C, CNN_STREAM));
   const int cols = ceil_div(std::max<int64_t>(C, g16 ? ld16 : C), 64);
-  const int rows = (int)std::min<int64_t>((M + kTrPix - 1) / kTrPix, std::max(1, device_sm_count() * 8 / cols));
-  k_relu_grad_t<<<dim3(rows, cols), 256, 0, CNN_STREAM>>>(
+  const int tiles = (int)std::min<int64_t>(M / kTrPix, std::max(1, device_sm_count() * 8 / cols));
+  k_relu_grad_t<<<dim3(tiles, cols), 256, 0, CNN_STREAM>>>(
       dy, reinterpret_cast<const __nv_bfloat16*>(act), M, C, reinterpret_cast<__nv_bfloat16*>(g16), ld16,
-      reinterpret_cast<__nv_bfloat16*>(gT), ld_t, db);
+      reinterpret_cast<__nv_bfloat16*>(gT), rows, db);
   EBSD_LAUNCH_CHECK();
   return 0;
 }

@@ -74,6 +74,7 @@ struct GemmParams {
   int a_rows;            // k_tc_gemm_long: rows of A staged (32, 64 or 128)
   int tile_n;            // k_tc_gemm_long: columns of a unit (16 or 32)
   int stages;            // k_tc_gemm_long
+  int chunks;            // k_tc_gemm_long: 128-byte slices of K in a stage
   const float* bias;     // MODE 2: per-row (output channel) bias
   __nv_bfloat16* out16;  // MODE 2: bf16 activations, (n_valid x ld_out)
   float* out32;          // MODE 2: optional FP32 copy, same layout
@@ -490,12 +491,14 @@ __global__ void __launch_bounds__(THREADS, 1)
 // outputs). With 128 x 256 tiles they ran in 1 to 18 CTAs that staged mostly
 // padding (48 KB per 64 of K) and took 5.6 of a training step's 12.7 ms. A unit
 // is 128 rows x 16 or 32 columns, only the rows of A that exist are staged, and
-// a stage holds 128 of K, so many stages are in flight and the chain of
-// dependent MMAs is the bound (60 ns each on one accumulator). K is not split:
-// every output keeps its one chain of accumulations in the order of k_tc_gemm,
-// and with it its value (the FP32 accumulators truncate, so a split sum of 10^6
-// terms differs by 10^-3). 32 x 9 x 1,048,576: 6.16 -> 3.97 ms, 64 x 288 x
-// 262,144: 1.53 -> 1.00, 256 x 1,152 x 16,384: 0.12 -> 0.07.
+// a stage holds 128 or 256 of K. K is not split: every output keeps its one
+// chain of accumulations in the order of k_tc_gemm, and with it its value (the
+// FP32 accumulators truncate, so a split sum of 10^6 terms differs by 10^-3).
+// Bound by the pace of the two single threads that issue: 32 x 9 x 1,048,576
+// (one CTA, 65,536 MMAs) 6.16 ms in a wide tile; 3.97 with narrow tiles; 3.21
+// with descriptors advanced by additions; 2.78 with one copy per operand and
+// stage; 2.66 from operands blocked by 64 of K (two accumulators in turn, or
+// M = 64, change nothing). 64 x 288 x 262,144: 1.53 -> 0.70 ms.
 //   warp 0 TMA producer, warp 1 TMEM (32 columns) and the MMAs, warps 2-5
 //   epilogue; waits and give-up as in k_tc_gemm.
 // ---------------------------------------------------------------------------
@@ -505,8 +508,9 @@ constexpr int LONG_DATA_BYTES = 216 * 1024;
 constexpr int LONG_SMEM_BYTES = 1024 + LONG_DATA_BYTES + LONG_BAR_BYTES;
 static_assert(LONG_SMEM_BYTES <= 232448, "shared memory budget");
 
-// Bytes of one 128-byte-wide half of a stage.
-__host__ __device__ inline int long_half_bytes(int a_rows, int tile_n) { return (a_rows + tile_n) * BKB; }
+// A stage holds p.chunks slices of 128 bytes of K, [slice][row of A] then
+// [slice][row of B], each operand one 3-D copy: a copy takes about 100 ns of the
+// producer whatever its size, so few and large ones.
 
 template <int KIND>
 __device__ __forceinline__ void long_unit(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p,
@@ -526,7 +530,9 @@ __device__ __forceinline__ void long_unit(const CUtensorMap& tmA, const CUtensor
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int stages = p.stages, k_iters = p.k_iters, tile_n = p.tile_n;
   const int m_tile = unit / p.n_tiles, n_tile = unit % p.n_tiles;
-  const uint32_t a_bytes = (uint32_t)p.a_rows * BKB, half = (uint32_t)long_half_bytes(p.a_rows, tile_n);
+  const int chunks = p.chunks;
+  const uint32_t a_bytes = (uint32_t)p.a_rows * BKB, b_bytes = (uint32_t)tile_n * BKB;
+  const uint32_t stage_bytes = (uint32_t)chunks * (a_bytes + b_bytes);
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
       mbar_init(full_bar(s), 1);
@@ -547,7 +553,6 @@ __device__ __forceinline__ void long_unit(const CUtensorMap& tmA, const CUtensor
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
   const uint64_t wait_ns = p.wait_ns;
-  constexpr int kx_step = BKB / kind_elem_bytes<KIND>();
   int prod_stage = 0;
   uint32_t prod_phase = 0;
   int64_t issued = 0;
@@ -558,18 +563,16 @@ __device__ __forceinline__ void long_unit(const CUtensorMap& tmA, const CUtensor
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int k = 0; k < k_iters; k += 2) {
+      for (int k = 0; k < k_iters; k += chunks) {
         if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, wait_ns)) {
           ok = false;
           break;
         }
-        const int halves = min(2, k_iters - k);
-        const uint32_t dst = sbase + (uint32_t)stage * 2u * half;
-        mbar_arrive_expect_tx(full_bar(stage), (uint32_t)halves * half);
-        for (int h = 0; h < halves; ++h) {
-          tma_load_2d(dst + h * half, &tmA, (k + h) * kx_step, m_tile * BM, full_bar(stage));
-          tma_load_2d(dst + h * half + a_bytes, &tmB, (k + h) * kx_step, n_tile * tile_n, full_bar(stage));
-        }
+        const uint32_t dst = sbase + (uint32_t)stage * stage_bytes;
+        // slices beyond the last arrive as zeros and are not used
+        mbar_arrive_expect_tx(full_bar(stage), stage_bytes);
+        tma_load_3d(dst, &tmA, 0, m_tile * BM, k, full_bar(stage));
+        tma_load_3d(dst + chunks * a_bytes, &tmB, 0, n_tile * tile_n, k, full_bar(stage));
         ++issued;
         if (++stage == stages) {
           stage = 0;
@@ -587,20 +590,24 @@ __device__ __forceinline__ void long_unit(const CUtensorMap& tmA, const CUtensor
       uint32_t phase = 0;
       bool ok = true;
       const uint32_t idesc = (make_idesc<KIND, 256>() & ~(0x3Fu << 17)) | ((uint32_t)(tile_n >> 3) << 17);
-      for (int k = 0; k < k_iters; k += 2) {
+      // descriptors advance by additions to their address field (16-byte units):
+      // this one thread's instructions per MMA pace the chain
+      const uint64_t a0 = smem_desc_sw128(sbase), b0 = smem_desc_sw128(sbase + chunks * a_bytes);
+      const uint32_t stage16 = stage_bytes >> 4, a16 = a_bytes >> 4, b16 = b_bytes >> 4;
+      uint32_t accumulate = 0;
+      for (int k = 0; k < k_iters; k += chunks) {
         if (!mbar_wait(full_bar(stage), phase, abort_flag, wait_ns)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t base = sbase + (uint32_t)stage * 2u * half;
-        const int halves = min(2, k_iters - k);
-        for (int h = 0; h < halves; ++h) {
-          const uint32_t a_addr = base + h * half, b_addr = a_addr + a_bytes;
+        uint64_t a = a0 + (uint32_t)stage * stage16, b = b0 + (uint32_t)stage * stage16;
+        const int n = min(chunks, k_iters - k);
+        for (int c = 0; c < n; ++c, a += a16, b += b16) {
+          tc_mma<KIND>(tmem_base, a, b, idesc, accumulate);
+          accumulate = 1;
 #pragma unroll
-          for (int kk = 0; kk < BKB / 32; ++kk)
-            tc_mma<KIND>(tmem_base, smem_desc_sw128(a_addr + kk * 32), smem_desc_sw128(b_addr + kk * 32), idesc,
-                         (k | h | kk) != 0 ? 1u : 0u);
+          for (int kk = 1; kk < BKB / 32; ++kk) tc_mma<KIND>(tmem_base, a + 2 * kk, b + 2 * kk, idesc, 1u);
         }
         any_mma = true;
         tc_commit(empty_bar(stage));
@@ -1642,25 +1649,38 @@ extern "C" int ebsd_match_topk(const void* queries_lp, int64_t n_queries_pad, co
 // Whether a product runs k_tc_gemm_long: K long enough that one unit's chain
 // outlasts its set-up, and too few 128 x 256 tiles to occupy half of the SMs
 // (with more, the wide tiles re-read A less often). At K = 4,096 and 18 wide
-// tiles the two take 0.030 and 0.033 ms, at K = 262,144 and 2 tiles 1.0 and 1.5.
+// tiles the two take 0.030 and 0.034 ms, at K = 262,144 and 2 tiles 0.70 and 1.51.
 static bool takes_long_tiles(int64_t m_tiles, int64_t n_valid, int64_t k_bytes) {
   return k_bytes >= 4096 && m_tiles * ceil_div(n_valid, 256) <= device_sm_count() / 2;
 }
 
 // Completes the parameters and tensor maps of one product; units: its CTAs.
+// blocked: operands as [slice of 128 bytes of K][row], else row-major.
 static int plan_long(const void* A, const void* B, int lp_dtype, int64_t m_pad, int64_t n_pad, int64_t k_pad,
-                     GemmParams& p, CUtensorMap* ta, CUtensorMap* tb, int* units) {
+                     bool blocked, GemmParams& p, CUtensorMap* ta, CUtensorMap* tb, int* units) {
   const int64_t m_tiles = ceil_div(p.m_valid, BM);
   p.a_rows = m_tiles > 1 || p.m_valid > 64 ? 128 : p.m_valid > 32 ? 64 : 32;
   p.tile_n = m_tiles * ceil_div(p.n_valid, 32) <= device_sm_count() / 2 ? 16 : 32;
   p.n_tiles = (int)ceil_div(p.n_valid, p.tile_n);
-  // the MMA reads 128 rows of A wherever its tile starts: keep the last one inside
-  const int half = long_half_bytes(p.a_rows, p.tile_n);
-  p.stages = std::min(LONG_MAX_STAGES, (LONG_DATA_BYTES - A_BYTES + half) / (2 * half));
+  const int slice = (p.a_rows + p.tile_n) * BKB;
+  p.chunks = slice <= 10 * 1024 ? 4 : 2;
+  // the MMA reads 128 rows of A wherever a slice starts: keep the last one inside
+  const int last = (p.chunks - 1) * p.a_rows * BKB + A_BYTES;
+  p.stages = std::min(LONG_MAX_STAGES, (LONG_DATA_BYTES - last) / (p.chunks * slice) + 1);
+  while (p.stages * p.chunks * slice > LONG_DATA_BYTES) --p.stages;
   p.wait_ns = wait_limit_ns();
   *units = (int)(m_tiles * p.n_tiles);
-  if (int rc = make_tmap(ta, A, lp_dtype, m_pad, k_pad, p.a_rows)) return rc;
-  return make_tmap(tb, B, lp_dtype, n_pad, k_pad, p.tile_n);
+  const int esz = lp_dtype == EBSD_DT_BF16 ? 2 : 1;
+  const CUtensorMapDataType type = esz == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+  const cuuint64_t sa[2] = {(cuuint64_t)(blocked ? BKB : k_pad * esz), (cuuint64_t)(blocked ? m_pad * BKB : BKB)};
+  const cuuint64_t sb[2] = {(cuuint64_t)(blocked ? BKB : k_pad * esz), (cuuint64_t)(blocked ? n_pad * BKB : BKB)};
+  const cuuint32_t steps[3] = {1, 1, 1};
+  const cuuint64_t da[3] = {(cuuint64_t)(BKB / esz), (cuuint64_t)m_pad, (cuuint64_t)p.k_iters};
+  const cuuint64_t db[3] = {(cuuint64_t)(BKB / esz), (cuuint64_t)n_pad, (cuuint64_t)p.k_iters};
+  const cuuint32_t ba[3] = {(cuuint32_t)(BKB / esz), (cuuint32_t)p.a_rows, (cuuint32_t)p.chunks};
+  const cuuint32_t bb[3] = {(cuuint32_t)(BKB / esz), (cuuint32_t)p.tile_n, (cuuint32_t)p.chunks};
+  if (int rc = encode_tensor_map(ta, type, 3, A, da, sa, ba, steps, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+  return encode_tensor_map(tb, type, 3, B, db, sb, bb, steps, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 template <int KIND>
@@ -1669,7 +1689,7 @@ static int launch_long(const void* A, const void* B, int lp_dtype, int64_t m_pad
   GemmParams p = p_in;
   CUtensorMap ta, tb;
   int units;
-  if (int rc = plan_long(A, B, lp_dtype, m_pad, n_pad, k_pad, p, &ta, &tb, &units)) return rc;
+  if (int rc = plan_long(A, B, lp_dtype, m_pad, n_pad, k_pad, false, p, &ta, &tb, &units)) return rc;
   const auto kern = k_tc_gemm_long<KIND>;
   EBSD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LONG_SMEM_BYTES));
   kern<<<units, THREADS, LONG_SMEM_BYTES, s>>>(ta, tb, p);
@@ -1677,34 +1697,37 @@ static int launch_long(const void* A, const void* B, int lp_dtype, int64_t m_pad
   return 0;
 }
 
-extern "C" int ebsd_gemm_nt_group(int n, const void* const* A, const int64_t* m_pad, const void* const* B,
-                                  const int64_t* n_pad, const int64_t* k_pad, float* const* C, const int64_t* ldc,
-                                  const int64_t* m_valid, const int64_t* n_valid, int* d_status, void* stream) {
+extern "C" int ebsd_gemm_nt_group(int n, const void* const* A, const int64_t* a_rows, const void* const* B,
+                                  const int64_t* b_rows, const int64_t* k, float* const* C, const int64_t* ldc,
+                                  const int64_t* m, const int64_t* n_cols, int* d_status, void* stream) {
   EBSD_ARG_CHECK(n >= 0 && n <= LONG_GROUP, "ebsd_gemm_nt_group: 0..%d products", LONG_GROUP);
-  EBSD_ARG_CHECK(n == 0 || (A && m_pad && B && n_pad && k_pad && C && ldc && m_valid && n_valid),
+  EBSD_ARG_CHECK(n == 0 || (A && a_rows && B && b_rows && k && C && ldc && m && n_cols && d_status),
                  "ebsd_gemm_nt_group: null array");
   if (n == 0) return 0;
   LongGroup g{};
   g.n = n;
   int order[LONG_GROUP];
   for (int i = 0; i < n; ++i) order[i] = i;
-  std::sort(order, order + n, [&](int i, int j) { return k_pad[i] > k_pad[j]; });
+  std::sort(order, order + n, [&](int i, int j) { return k[i] > k[j]; });
   for (int j = 0; j < n; ++j) {
     const int i = order[j];
-    if (int rc = check_operands(A[i], m_pad[i], B[i], n_pad[i], k_pad[i], EBSD_DT_BF16, d_status)) return rc;
-    EBSD_ARG_CHECK(C[i] != nullptr && m_valid[i] > 0 && m_valid[i] <= m_pad[i] && n_valid[i] > 0 &&
-                       n_valid[i] <= n_pad[i] && ldc[i] >= n_valid[i],
+    EBSD_ARG_CHECK(A[i] && B[i] && C[i] && (((uintptr_t)A[i] | (uintptr_t)B[i]) & 15) == 0,
+                   "ebsd_gemm_nt_group: product %d: null or unaligned operand", i);
+    EBSD_ARG_CHECK(k[i] >= 64 && k[i] % 64 == 0 && k[i] < ((int64_t)1 << 36),
+                   "ebsd_gemm_nt_group: product %d: K must be a multiple of 64", i);
+    EBSD_ARG_CHECK(m[i] > 0 && m[i] <= a_rows[i] && n_cols[i] > 0 && n_cols[i] <= b_rows[i] && ldc[i] >= n_cols[i] &&
+                       a_rows[i] < (1 << 24) && b_rows[i] < (1 << 24),
                    "ebsd_gemm_nt_group: product %d: extents out of range", i);
     GemmParams& p = g.p[j];
-    p.k_iters = (int)(k_pad[i] * 2 / BKB);
-    p.n_valid = n_valid[i];
+    p.k_iters = (int)(k[i] / 64);
+    p.n_valid = n_cols[i];
     p.C = C[i];
     p.ldc = ldc[i];
-    p.m_valid = m_valid[i];
+    p.m_valid = m[i];
     p.alpha = 1.0f;
     p.status = d_status;
     int units;
-    if (int rc = plan_long(A[i], B[i], EBSD_DT_BF16, m_pad[i], n_pad[i], k_pad[i], p, &g.a[j], &g.b[j], &units))
+    if (int rc = plan_long(A[i], B[i], EBSD_DT_BF16, a_rows[i], b_rows[i], k[i], true, p, &g.a[j], &g.b[j], &units))
       return rc;
     g.first[j + 1] = g.first[j] + units;
   }

@@ -9,6 +9,7 @@ except ``grid_fz`` (it must read the fundamental-zone point count).
 
 from __future__ import annotations
 
+import ctypes
 from typing import Optional
 
 import torch
@@ -313,14 +314,13 @@ def gemm_nt(A, B, out, alpha: float = 1.0, accumulate: bool = False, m_valid=Non
 
 
 def gemm_nt_group(products, status: torch.Tensor) -> None:
-    """out = A @ B.T for up to 8 (A, B, out) products of bf16 rows with a long
-    K, in one launch (ebsd_gemm_nt_group): out (m, n), A with at least m rows
-    (a multiple of 128), B with at least n (a multiple of 256). Rows beyond m
-    and n need not be written."""
+    """out = A @ B.T for up to 8 (A, B, out) products of bf16 operands with a
+    long K, in one launch (ebsd_gemm_nt_group): A (K / 64, rows, 64) and B
+    (K / 64, rows, 64) blocked by 64 of K, out (m, n) with m and n at most
+    their rows. Rows beyond m and n need not be written."""
     n = len(products)
     if not n:
         return
-    import ctypes
 
     def arr(ctype, values):
         return (ctype * n)(*values)
@@ -329,10 +329,12 @@ def gemm_nt_group(products, status: torch.Tensor) -> None:
         _cuda(A, "A", torch.bfloat16)
         _cuda(B, "B", torch.bfloat16)
         _cuda(out, "out", torch.float32)
+        if A.dim() != 3 or B.dim() != 3 or A.shape[2] != 64 or B.shape[2] != 64 or A.shape[0] != B.shape[0]:
+            raise ValueError("operands must be (K / 64, rows, 64) with the same K")
     i64, vp = ctypes.c_int64, ctypes.c_void_p
     call("ebsd_gemm_nt_group", n, arr(vp, [A.data_ptr() for A, _, _ in products]),
-         arr(i64, [A.shape[0] for A, _, _ in products]), arr(vp, [B.data_ptr() for _, B, _ in products]),
-         arr(i64, [B.shape[0] for _, B, _ in products]), arr(i64, [A.shape[1] for A, _, _ in products]),
+         arr(i64, [A.shape[1] for A, _, _ in products]), arr(vp, [B.data_ptr() for _, B, _ in products]),
+         arr(i64, [B.shape[1] for _, B, _ in products]), arr(i64, [64 * A.shape[0] for A, _, _ in products]),
          arr(vp, [o.data_ptr() for _, _, o in products]), arr(i64, [o.stride(0) for _, _, o in products]),
          arr(i64, [o.shape[0] for _, _, o in products]), arr(i64, [o.shape[1] for _, _, o in products]), ptr(status),
          _stream(products[0][0].device))

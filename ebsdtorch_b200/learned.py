@@ -104,16 +104,16 @@ class _Conv:
         # weight gradient, column sums for the bias
         ld16 = round_up(self.cout, 64)
         g16 = torch.empty((M, ld16), dtype=torch.bfloat16, device=dev) if need_dx else None
-        gT = torch.empty((round_up(self.cout, 128), M), dtype=torch.bfloat16, device=dev)
-        call("ebsd_cnn_relu_grad_t", ptr(dout.contiguous()), ptr(keep["out"]), M, self.cout, ptr(g16), ld16, ptr(gT), M,
-             ptr(self.gb), s)
-        # weight gradient: (cout x K) = g^T (cout x M) . cols (M x K)
-        colsT = torch.empty((round_up(self.K, 256), M), dtype=torch.bfloat16, device=dev)
+        gT = torch.empty((M // 64, round_up(self.cout, 16), 64), dtype=torch.bfloat16, device=dev)
+        call("ebsd_cnn_relu_grad_t", ptr(dout.contiguous()), ptr(keep["out"]), M, self.cout, ptr(g16), ld16, ptr(gT),
+             gT.shape[1], ptr(self.gb), s)
+        # weight gradient: (cout x K) = g^T (cout x M) . cols (M x K), both
+        # operands transposed and blocked by 64 pixels
         if "cols" in keep:
-            call("ebsd_cnn_transpose", ptr(keep["cols"]), 0, M, self.K_pad, self.K_pad, ptr(colsT), colsT.shape[0], M,
-                 s)
+            colsT = keep["cols"][:M].view(M // 64, 64, self.K_pad).transpose(1, 2).contiguous()
         else:
-            call("ebsd_cnn_im2col_t", ptr(keep["x"]), B, H, W, self.cin, ptr(colsT), M, s)
+            colsT = torch.empty((M // 64, round_up(self.K, 16), 64), dtype=torch.bfloat16, device=dev)
+            call("ebsd_cnn_im2col_t", ptr(keep["x"]), B, H, W, self.cin, ptr(colsT), colsT.shape[1], s)
         products.append((gT, colsT, self.gw))
         if not need_dx:
             return None

@@ -96,7 +96,7 @@ def test_first_layer_rounds_fp32_pixels_as_the_cast_does(B, H, W, cout):
 
 
 @pytest.mark.parametrize("C", [1, 32, 64, 128])
-@pytest.mark.parametrize("B,H,W", [(8, 1, 1), (8, 5, 7), (16, 6, 6), (8, 16, 15)])
+@pytest.mark.parametrize("B,H,W", [(64, 1, 1), (16, 5, 7), (64, 6, 6), (8, 16, 15)])
 def test_backward_operands(C, B, H, W):
     """Transposed columns, the fused ReLU gradient and the column gradient's
     scatter against torch, padding included."""
@@ -109,9 +109,10 @@ def test_backward_operands(C, B, H, W):
     pad = torch.nn.functional.pad(x, (0, 0, 1, 2, 1, 2))
     taps = [pad[:, ky:ky + 2 * Ho:2, kx:kx + 2 * Wo:2] for ky in range(3) for kx in range(3)]
     ref = torch.stack(taps, 3).reshape(M, 9 * C).t()
-    out = torch.full((9 * C + 1, M + 8), 7.0, device=DEV).bfloat16()
-    call("ebsd_cnn_im2col_t", ptr(x), B, H, W, C, ptr(out), M + 8, None)
-    assert torch.equal(out[:9 * C, :M], ref) and (out[9 * C] == 7).all() and (out[:, M:] == 7).all()
+    out = torch.full((M // 64 + 1, 9 * C + 1, 64), 7.0, device=DEV).bfloat16()
+    call("ebsd_cnn_im2col_t", ptr(x), B, H, W, C, ptr(out), 9 * C + 1, None)
+    assert torch.equal(out[:-1, :9 * C].transpose(0, 1).reshape(9 * C, M), ref)
+    assert (out[-1] == 7).all() and (out[:, 9 * C] == 7).all()
     dcols = torch.randn((M, 9 * C), generator=g).to(DEV)
     dx = torch.empty((B, H, W, C), device=DEV)
     call("ebsd_cnn_col2im", ptr(dcols), 9 * C, B, H, W, C, ptr(dx), None)
@@ -127,11 +128,12 @@ def test_backward_operands(C, B, H, W):
     want = torch.where(act.float() > 0, dy, torch.zeros_like(dy))
     for keep in (True, False):
         g16 = torch.full((M, ld16), 5.0, device=DEV).bfloat16()
-        gT = torch.full((C + 1, M), 5.0, device=DEV).bfloat16()
+        gT = torch.full((M // 64 + 1, C + 1, 64), 5.0, device=DEV).bfloat16()
         db = torch.full((C,), 5.0, device=DEV)
-        call("ebsd_cnn_relu_grad_t", ptr(dy), ptr(act), M, C, ptr(g16) if keep else None, ld16, ptr(gT), M, ptr(db),
-             None)
+        call("ebsd_cnn_relu_grad_t", ptr(dy), ptr(act), M, C, ptr(g16) if keep else None, ld16, ptr(gT), C + 1,
+             ptr(db), None)
         if keep:
             assert torch.equal(g16[:, :C], want.bfloat16()) and (g16[:, C:] == 0).all()
-        assert torch.equal(gT[:C], want.bfloat16().t()) and (gT[C] == 5).all()
+        assert torch.equal(gT[:-1, :C].transpose(0, 1).reshape(C, M), want.bfloat16().t())
+        assert (gT[-1] == 5).all() and (gT[:, C] == 5).all()
         assert (db.double() - want.double().sum(0)).abs().max() <= M * 2.0 ** -23 * 4

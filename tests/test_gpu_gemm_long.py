@@ -65,7 +65,9 @@ def test_grouped_products_give_the_same_bits():
     for m, n, k in shapes:
         A = torch.randn((-(-m // 128) * 128, k), generator=g, device=DEV).bfloat16()
         B = torch.randn((-(-n // 256) * 256, k), generator=g, device=DEV).bfloat16()
-        prods.append((A, B, torch.zeros((m, n), device=DEV)))
+        ra, rb = -(-m // 16) * 16, -(-n // 16) * 16
+        prods.append((A[:ra].view(ra, k // 64, 64).transpose(0, 1).contiguous(),
+                      B[:rb].view(rb, k // 64, 64).transpose(0, 1).contiguous(), torch.zeros((m, n), device=DEV)))
         ref = torch.zeros((m, n), device=DEV)
         kernels.gemm_nt(A, B, ref, m_valid=m, n_valid=n, splits=B.shape[0] // 256)
         refs.append(ref)
