@@ -201,18 +201,6 @@ __global__ void k_sampling_quads(const float* __restrict__ mp, int h, int w, flo
   quads[(int64_t)y * w + x] = make_float4(__ldg(lo + x), __ldg(lo + x1), __ldg(hi + x), __ldg(hi + x1));
 }
 
-// The four taps of a sample: one float4 of a gather table, or four values of
-// the image (upper taps clamped to the border).
-template <bool QUADS>
-__device__ __forceinline__ float4 load_taps(const float* __restrict__ img, int mp_h, const LambertGrid& g, int i) {
-  if constexpr (QUADS) return __ldg(reinterpret_cast<const float4*>(img) + i);
-  const int y0 = i / (int)g.w, x0 = i - y0 * (int)g.w;
-  const float* lo = img + i;
-  const float* hi = y0 < mp_h - 1 ? lo + g.w : lo;
-  const int dx = x0 < (int)g.w - 1 ? 1 : 0;
-  return make_float4(__ldg(lo), __ldg(lo + dx), __ldg(hi), __ldg(hi + dx));
-}
-
 // One CTA per dictionary row, grid-stride; each thread computes the taps of
 // its next pixel while the gather of the current one is in flight. QUADS:
 // `img` holds the four taps of every pixel as one float4, so a sample is one
@@ -241,18 +229,18 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 2) k_project(
     const float3 q2 = make_float3(2.0f * q.y, 2.0f * q.z, 2.0f * q.w);
     float part = 0.0f, part_b = 0.0f;
     int p = threadIdx.x;
-    LambertTap t = {0, 0.0f, 0.0f};
+    LambertTap<QUADS> t{};
     float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (p < n_pix) {
-      t = lambert_tap(g, q, q2, __ldg(rx + p), __ldg(ry + p), __ldg(rz + p));
-      v = load_taps<QUADS>(img, mp_h, g, t.i);
+      t = lambert_tap<false, QUADS>(g, q, q2, __ldg(rx + p), __ldg(ry + p), __ldg(rz + p));
+      v = load_taps(img, mp_h, g, t);
     }
 #pragma unroll 2
     for (; p < n_pix; p += THREADS) {
       const int pn = min(p + THREADS, n_pix - 1);
-      const LambertTap tn = lambert_tap(g, q, q2, __ldg(rx + pn), __ldg(ry + pn), __ldg(rz + pn));
-      const float4 vn = load_taps<QUADS>(img, mp_h, g, tn.i);
-      const float val = blend(t, v.x, v.y, v.z, v.w);
+      const LambertTap<QUADS> tn = lambert_tap<false, QUADS>(g, q, q2, __ldg(rx + pn), __ldg(ry + pn), __ldg(rz + pn));
+      const float4 vn = load_taps(img, mp_h, g, tn);
+      const float val = blend(t, v);
       row[p] = val;
       if constexpr (THREADS == 512) {
         part += val;
@@ -406,6 +394,7 @@ static int project_rows(const float* img, int mp_h, int mp_w2, const float* rays
   EBSD_ARG_CHECK(n_rows >= 0, "n_rows < 0");
   EBSD_ARG_CHECK((reinterpret_cast<uintptr_t>(quats) & 15) == 0, "quats must be 16-byte aligned");
   EBSD_ARG_CHECK(!QUADS || (reinterpret_cast<uintptr_t>(img) & 15) == 0, "quads must be 16-byte aligned");
+  EBSD_ARG_CHECK(!QUADS || quads_fit(mp_h, mp_w2), "master pattern shape (%d, %d) too large for quads", mp_h, mp_w2);
   if (int rc = check_row_out(o, n_pix)) return rc;
   if (n_rows == 0) return 0;
   const float4* q = reinterpret_cast<const float4*>(quats);
@@ -426,7 +415,7 @@ extern "C" int ebsd_project_dictionary(const float* master_pattern, int mp_h, in
 
 extern "C" int ebsd_sampling_quads(const float* master_pattern, int mp_h, int mp_w2, float* quads, void* stream) {
   EBSD_ARG_CHECK(master_pattern && quads, "ebsd_sampling_quads: null pointer");
-  EBSD_ARG_CHECK(mp_h >= 1 && mp_h <= 65535 && mp_w2 >= 1, "master pattern shape (%d, %d) invalid", mp_h, mp_w2);
+  EBSD_ARG_CHECK(mp_h >= 1 && mp_w2 >= 1 && quads_fit(mp_h, mp_w2), "master pattern shape (%d, %d) invalid", mp_h, mp_w2);
   EBSD_ARG_CHECK((reinterpret_cast<uintptr_t>(quads) & 15) == 0, "quads must be 16-byte aligned");
   k_sampling_quads<<<dim3(ceil_div(mp_w2, 256), mp_h), 256, 0, as_stream(stream)>>>(
       master_pattern, mp_h, mp_w2, reinterpret_cast<float4*>(quads));

@@ -31,9 +31,14 @@
 namespace ebsd {
 
 constexpr int kRefThreads = 512;
-constexpr int kRefGroup = 16;      // candidates scored per pass over the pixels
-constexpr int kRefIlp = 4;         // candidates whose gathers are issued together
-constexpr int kMaxRefGrid = 343;   // (2 * 3 + 1)^3
+// Candidates scored per pass over the pixels, in threes whose gathers are issued
+// together. Cubes of odd side leave no slot idle (27, nearly 125 and 343), and the
+// 18 sums fit two CTAs of 512 threads on an SM: 27 candidates on 4,096 patterns of
+// 128^2 px take 24.3 ms, 16 in fours (one CTA) 30.5, 12 in twos 26.1, 8 in fours
+// 25.1, 4 27.0; 7 candidates 8.1 ms against 9.8 (16) and 6.9 (8 one by one).
+constexpr int kRefGroup = 9;
+constexpr int kRefIlp = 3;
+constexpr int kMaxRefGrid = 343;  // (2 * 3 + 1)^3
 constexpr int kMaxRefPix = 40960;  // FP32 pattern row in shared memory (160 KiB)
 
 __device__ __forceinline__ void qmul_d(const double a[4], const double b[4], double o[4]) {
@@ -48,8 +53,15 @@ __device__ __forceinline__ void qstd_d(double q[4]) {
     for (int k = 0; k < 4; ++k) q[k] = -q[k];
 }
 
-__global__ void __launch_bounds__(kRefThreads) k_refine(
-    const float* __restrict__ mp, int mp_h, int mp_w2, const float* __restrict__ coords, int n_pix,
+// Bound by instruction issue: the rotate / Lambert / blend chain of a sample (a
+// CTA's candidates fall on the same few lines of the master pattern). QUADS: mp
+// is a gather table, one 16-byte load per sample in place of four of 4 bytes.
+// 4,096 patterns of 128^2 px, 27 candidates, 3 iterations: 24.3 ms (224 samples
+// per ns, the projector's rate); 39 ms with 32 slots for the 27 candidates, one
+// CTA per SM and the sampling chain as the compiler contracts it. Same bits.
+template <bool QUADS>
+__global__ void __launch_bounds__(kRefThreads, 2) k_refine(
+    const float* __restrict__ mp, int mp_h, const LambertGrid lg, const float* __restrict__ coords, int n_pix,
     const float* __restrict__ offsets, const float* __restrict__ exp_rows, int64_t ld_e,
     const float* __restrict__ q_in, int64_t n, const float* __restrict__ grid, int n_grid, int centre,
     const LaueTable ops, int fz_left, int n_iter, float shrink, float* __restrict__ q_out,
@@ -127,31 +139,24 @@ __global__ void __launch_bounds__(kRefThreads) k_refine(
             vz /= nr;
           }
           const float e = erow[p];
-          // kRefIlp candidates at a time: taps first, then their gathers
-          // together (the loop is bound by the gather latency through L2)
+          // kRefIlp candidates at a time: taps first, then their gathers together
 #pragma unroll
           for (int c0 = 0; c0 < kRefGroup; c0 += kRefIlp) {
-            BorderTaps t[kRefIlp];
+            if (c0 >= ng) break;
+            LambertTap<QUADS> t[kRefIlp];
 #pragma unroll
             for (int k = 0; k < kRefIlp; ++k) {
-              const float3 r = rotate(cand[g0 + min(c0 + k, ng - 1)], vx, vy, vz);
-              const float2 uv = lambert_side_by_side(r.x, r.y, r.z);
-              t[k] = border_taps<true>(mp_h, mp_w2, uv.x, uv.y);
+              const float4 q = cand[g0 + min(c0 + k, ng - 1)];
+              t[k] = lambert_tap<true, QUADS>(lg, q, make_float3(2.0f * q.y, 2.0f * q.z, 2.0f * q.w), vx, vy, vz);
             }
-            float gv[kRefIlp][4];
+            float4 v[kRefIlp];
 #pragma unroll
-            for (int k = 0; k < kRefIlp; ++k) {
-              gv[k][0] = __ldg(mp + t[k].i00);
-              gv[k][1] = __ldg(mp + t[k].i01);
-              gv[k][2] = __ldg(mp + t[k].i10);
-              gv[k][3] = __ldg(mp + t[k].i11);
-            }
+            for (int k = 0; k < kRefIlp; ++k) v[k] = load_taps(mp, mp_h, lg, t[k]);
 #pragma unroll
             for (int k = 0; k < kRefIlp; ++k) {
               const int c = c0 + k;
               if (c < ng) {
-                const float val = gv[k][0] * t[k].w00 + gv[k][1] * t[k].w01 + gv[k][2] * t[k].w10 +
-                                  gv[k][3] * t[k].w11;
+                const float val = blend(t[k], v[k]);
                 ad[c] = fmaf(val, e, ad[c]);
                 as[c] += val;
               }
@@ -205,13 +210,15 @@ __global__ void __launch_bounds__(kRefThreads) k_refine(
 
 using namespace ebsd;
 
-extern "C" int ebsd_refine_grid(const float* master_pattern, int mp_h, int mp_w2, const float* coords_soa,
-                                int n_pix, const float* offsets, const float* exp_rows, int64_t ld_e,
-                                const float* q_in, int64_t n, const float* grid_cu, int n_grid, int laue_id,
-                                int fz_left, int n_iter, float shrink, float* q_out, float* dots,
-                                void* stream) {
+template <bool QUADS>
+static int refine_grid(const float* master_pattern, int mp_h, int mp_w2, const float* coords_soa, int n_pix,
+                       const float* offsets, const float* exp_rows, int64_t ld_e, const float* q_in, int64_t n,
+                       const float* grid_cu, int n_grid, int laue_id, int fz_left, int n_iter, float shrink,
+                       float* q_out, float* dots, void* stream) {
   EBSD_ARG_CHECK(master_pattern && coords_soa && exp_rows && q_in && grid_cu && q_out && dots,
                  "ebsd_refine_grid: null pointer");
+  EBSD_ARG_CHECK(!QUADS || (reinterpret_cast<uintptr_t>(master_pattern) & 15) == 0, "quads must be 16-byte aligned");
+  EBSD_ARG_CHECK(!QUADS || quads_fit(mp_h, mp_w2), "master pattern shape (%d, %d) too large for quads", mp_h, mp_w2);
   EBSD_ARG_CHECK(mp_h >= 2 && mp_w2 >= 2, "master pattern shape (%d, %d) invalid", mp_h, mp_w2);
   EBSD_ARG_CHECK(n_pix >= 1 && n_pix <= kMaxRefPix && ld_e >= n_pix, "row length %d outside [1, %d]", n_pix,
                  kMaxRefPix);
@@ -224,12 +231,28 @@ extern "C" int ebsd_refine_grid(const float* master_pattern, int mp_h, int mp_w2
   LaueTable t{};
   build_laue_table(laue_id, &t);
   const size_t smem = (size_t)n_pix * sizeof(float);
-  EBSD_CUDA_CHECK(cudaFuncSetAttribute(k_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  EBSD_CUDA_CHECK(cudaFuncSetAttribute(k_refine<QUADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = (int)std::min<int64_t>(n, (int64_t)device_sm_count() * 16);
-  k_refine<<<grid, kRefThreads, smem, as_stream(stream)>>>(master_pattern, mp_h, mp_w2, coords_soa, n_pix, offsets,
-                                                           exp_rows, ld_e, q_in, n, grid_cu, n_grid,
-                                                           (n_grid - 1) / 2, t, fz_left, n_iter, shrink, q_out,
-                                                           dots);
+  k_refine<QUADS><<<grid, kRefThreads, smem, as_stream(stream)>>>(
+      master_pattern, mp_h, lambert_grid<true>(mp_h, mp_w2), coords_soa, n_pix, offsets, exp_rows, ld_e, q_in, n,
+      grid_cu, n_grid, (n_grid - 1) / 2, t, fz_left, n_iter, shrink, q_out, dots);
   EBSD_LAUNCH_CHECK();
   return 0;
+}
+
+extern "C" int ebsd_refine_grid(const float* master_pattern, int mp_h, int mp_w2, const float* coords_soa,
+                                int n_pix, const float* offsets, const float* exp_rows, int64_t ld_e,
+                                const float* q_in, int64_t n, const float* grid_cu, int n_grid, int laue_id,
+                                int fz_left, int n_iter, float shrink, float* q_out, float* dots,
+                                void* stream) {
+  return refine_grid<false>(master_pattern, mp_h, mp_w2, coords_soa, n_pix, offsets, exp_rows, ld_e, q_in, n, grid_cu,
+                            n_grid, laue_id, fz_left, n_iter, shrink, q_out, dots, stream);
+}
+
+extern "C" int ebsd_refine_grid_quads(const float* quads, int mp_h, int mp_w2, const float* coords_soa, int n_pix,
+                                      const float* offsets, const float* exp_rows, int64_t ld_e, const float* q_in,
+                                      int64_t n, const float* grid_cu, int n_grid, int laue_id, int fz_left,
+                                      int n_iter, float shrink, float* q_out, float* dots, void* stream) {
+  return refine_grid<true>(quads, mp_h, mp_w2, coords_soa, n_pix, offsets, exp_rows, ld_e, q_in, n, grid_cu, n_grid,
+                           laue_id, fz_left, n_iter, shrink, q_out, dots, stream);
 }

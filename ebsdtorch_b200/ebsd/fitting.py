@@ -238,7 +238,7 @@ def _search_dft(mp_t, padded, quats, pix64, z_vals, tilt, sec_tilt, det, bs, bat
     sub = max(1, min(bs, n_dict, MAX_SIM_BYTES // (hp * wp * 4)))
     sims = torch.empty((sub, hp * wp), dtype=torch.float32, device=dev)
     spec = torch.empty((sub, spec_len), dtype=torch.float32, device=dev)
-    quads = kernels.sampling_quads(mp_t)
+    quads = kernels.quads_for(mp_t, len(z_vals) * n_dict * hp * wp)
     for zi in range(len(z_vals)):
         rays = _rays_soa(pix64, float(z_vals[zi]), tilt, sec_tilt, det, dev)
         for j in range(0, n_dict, bs):
@@ -267,7 +267,7 @@ def _search_fft(mp_t, padded, quats, pix64, z_vals, tilt, sec_tilt, det, bs, bat
     wf = wp // 2 + 1
     sub = max(1, min(bs, MAX_PRODUCT_BYTES // (B * hp * wf * 8)))
     sims = torch.empty((min(sub, n_dict), hp * wp), dtype=torch.float32, device=dev)
-    quads = kernels.sampling_quads(mp_t)
+    quads = kernels.quads_for(mp_t, len(z_vals) * n_dict * hp * wp)
     for zi in range(len(z_vals)):
         rays = _rays_soa(pix64, float(z_vals[zi]), tilt, sec_tilt, det, dev)
         for j in range(0, n_dict, bs):

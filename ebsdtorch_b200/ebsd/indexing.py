@@ -410,7 +410,7 @@ def pca_dictionary_index_orientations(
                     sample_ori_fz_laue_angle(mp.laue_group, dictionary_resolution_index_deg, dev)
                 del ori_learn
             proj = _Projector(comps)
-            quads = kernels.sampling_quads(mp_t)
+            quads = kernels.quads_for(mp_t, ori.shape[0] * P)
             n_comp = comps.shape[0]
             pats = _pattern_source(experiment_patterns, dev)
             qfill_full = _query_fill(pats, virtual_binning, pix_index, P, subtract, dev)

@@ -101,6 +101,8 @@ def orientation_grid_refinement(
         dots = torch.zeros((experiment_patterns.n_patterns, n_iter), device=dev)
         rays = coords.t().contiguous().float().to(dev)
         mp_t = _master_pattern_tensor(mp, b, dev)
+        quads = kernels.quads_for(mp_t, indices.numel() * n_pix * n_grid * n_iter)
+        entry, img = ("ebsd_refine_grid", mp_t) if quads is None else ("ebsd_refine_grid_quads", quads)
         grid = grid_cpu.float().contiguous().to(dev)
         for c0 in range(0, indices.numel(), query_chunk):
             idx = indices[c0:c0 + query_chunk]
@@ -115,8 +117,8 @@ def orientation_grid_refinement(
             q_out = torch.empty_like(q)
             d_out = torch.empty((nq, n_iter), dtype=torch.float32, device=dev)
             off = offsets_all[idx.to(offsets_all.device)].to(dev).contiguous() if offsets_all is not None else None
-            call("ebsd_refine_grid", ptr(mp_t), mp_t.shape[0], mp_t.shape[1], ptr(rays), n_pix, ptr(off), ptr(rows),
-                 rows.stride(0), ptr(q), nq, ptr(grid), n_grid, int(mp.laue_group), int(fz_reduction == "left"),
+            call(entry, ptr(img), mp_t.shape[0], mp_t.shape[1], ptr(rays), n_pix, ptr(off), ptr(rows), rows.stride(0),
+                 ptr(q), nq, ptr(grid), n_grid, int(mp.laue_group), int(fz_reduction == "left"),
                  int(n_iter), float(shrink_factor), ptr(q_out), ptr(d_out),
                  torch.cuda.current_stream(dev).cuda_stream)
             dots[idx.to(dev)] = d_out

@@ -129,10 +129,19 @@ def sampling_quads(master_pattern: torch.Tensor) -> torch.Tensor:
 QUADS_MIN_SAMPLES, QUADS_MIN_RATIO = 1 << 22, 4
 
 
+def quads_for(master_pattern: torch.Tensor, n_samples: int) -> Optional[torch.Tensor]:
+    """The master pattern's gather table where `n_samples` samples repay it and
+    its sizes allow one (quads_fit in sampling.cuh)."""
+    h, w = master_pattern.shape
+    if n_samples < max(QUADS_MIN_SAMPLES, QUADS_MIN_RATIO * h * w) or h > 65535 or w > 1 << 22 or h * w >= 1 << 31:
+        return None
+    return sampling_quads(master_pattern)
+
+
 def project(master_pattern: torch.Tensor, rays_soa: torch.Tensor, quats: torch.Tensor, out: RowBuffers,
             subtract_mean: bool = True, quads: Optional[torch.Tensor] = None) -> None:
     """K1: simulated dictionary rows for `quats` into `out` (row i <- quats[i]).
-    quads: sampling_quads(master_pattern), for callers that project in several
+    quads: quads_for(master_pattern, all samples), for callers that project in several
     calls; without it a call that is large enough makes its own."""
     _cuda(master_pattern, "master_pattern", torch.float32)
     _cuda(rays_soa, "rays_soa", torch.float32)
@@ -140,9 +149,8 @@ def project(master_pattern: torch.Tensor, rays_soa: torch.Tensor, quats: torch.T
     if rays_soa.dim() != 2 or rays_soa.shape[0] != 3:
         raise ValueError("rays_soa must be (3, n_pix)")
     n_pix = rays_soa.shape[1]
-    if quads is None and \
-            quats.shape[0] * n_pix >= max(QUADS_MIN_SAMPLES, QUADS_MIN_RATIO * master_pattern.numel()):
-        quads = sampling_quads(master_pattern)
+    if quads is None:
+        quads = quads_for(master_pattern, quats.shape[0] * n_pix)
     name, img = ("ebsd_project_dictionary", master_pattern) if quads is None else \
         ("ebsd_project_dictionary_quads", quads)
     call(name, ptr(img), master_pattern.shape[0], master_pattern.shape[1],

@@ -405,6 +405,11 @@ int ebsd_refine_grid(const float* master_pattern, int mp_h, int mp_w2, const flo
                      const float* offsets, const float* exp_rows, int64_t ld_e, const float* q_in, int64_t n,
                      const float* grid_cu, int n_grid, int laue_id, int fz_left, int n_iter, float shrink,
                      float* q_out, float* dots, void* stream);
+/* The same from the master pattern's gather table (ebsd_sampling_quads). */
+int ebsd_refine_grid_quads(const float* quads, int mp_h, int mp_w2, const float* coords_soa, int n_pix,
+                           const float* offsets, const float* exp_rows, int64_t ld_e, const float* q_in, int64_t n,
+                           const float* grid_cu, int n_grid, int laue_id, int fz_left, int n_iter, float shrink,
+                           float* q_out, float* dots, void* stream);
 
 /* ---- experimental-pattern preprocessing --------------------------------------
  * FP32 patterns as n rows of n_pix pixels (row stride ld). */
