@@ -64,6 +64,7 @@ SIGNATURES = {
     "ebsd_refine_grid_quads": (i32, [vp, i32, i32, vp, i32, vp, vp, i64, vp, i64, vp, i32, i32, i32, i32, f32, vp, vp,
                                vp]),
     "ebsd_pattern_mean": (i32, [vp, i64, i32, i64, vp, i32, vp, vp]),
+    "ebsd_pattern_rows_mean": (i32, [vp, i32, i64, i32, i64, vp, vp, i32, vp, vp]),
     "ebsd_subtract_pattern": (i32, [vp, i64, i32, i64, vp, vp]),
     "ebsd_normalize_patterns": (i32, [vp, i64, i32, i64, i32, vp]),
     "ebsd_clahe": (i32, [vp, i64, i32, i32, i64, vp, i32, f32, i32, i32, i32, i32, vp, i64, vp]),
@@ -122,7 +123,7 @@ LAUNCHES_PER_CALL = {
     "ebsd_merge_rescore": 1, "ebsd_merge_rescore_gated": 1, "ebsd_manhattan_topk": 1, "ebsd_gemm_nt": 1, "ebsd_gemm_f32": 1, "ebsd_col_mean": 1, "ebsd_split3_bf16": 1,
     "ebsd_disori_angle": 1, "ebsd_match_topk_noalloc": 2, "ebsd_zh_to_qu": 1, "ebsd_qu_to_zh": 1,
     "ebsd_cell_to_row": 2, "ebsd_local_search": 1, "ebsd_refine_grid": 1, "ebsd_refine_grid_quads": 1,
-    "ebsd_pattern_mean": 2, "ebsd_subtract_pattern": 1, "ebsd_normalize_patterns": 1, "ebsd_clahe": 1,
+    "ebsd_pattern_mean": 2, "ebsd_pattern_rows_mean": 2, "ebsd_subtract_pattern": 1, "ebsd_normalize_patterns": 1, "ebsd_clahe": 1,
     "ebsd_nlpar_dists": 1, "ebsd_nlpar_average": 1,
     "ebsd_nlpar_dists_window": 1, "ebsd_nlpar_average_window": 1, "ebsd_nlpar_weights": 14,
     "ebsd_pcfit_prep": 1, "ebsd_pcfit_reduce": 1, "ebsd_pcfit_xcorr_tables": 1, "ebsd_pcfit_spectra": 1, "ebsd_pcfit_spectra_quads": 1,

@@ -419,6 +419,10 @@ int ebsd_refine_grid_quads(const float* quads, int mp_h, int mp_w2, const float*
  * ExperimentPatterns.subtract_overall_background (experiment_pats.py:223-232). */
 int ebsd_pattern_mean(const float* patterns, int64_t n, int n_pix, int64_t ld, double* partial, int n_splits,
                       float* mean, void* stream);
+/* The same of patterns in their detector type (EBSD_PAT_U16, _U8 or _F16; ld in
+ * values), whose FP32 rows (n, n_pix) are written on the way. */
+int ebsd_pattern_rows_mean(const void* patterns, int pattern_dtype, int64_t n, int n_pix, int64_t ld, float* rows,
+                           double* partial, int n_splits, float* mean, void* stream);
 /* patterns[r, c] -= v[c] in place. */
 int ebsd_subtract_pattern(float* patterns, int64_t n, int n_pix, int64_t ld, const float* v, void* stream);
 /* ExperimentPatterns.normalize_per_pattern (experiment_pats.py:255-285), in
