@@ -825,21 +825,23 @@ template <int H>
 struct NlAvg {
   static constexpr int ROWS = H <= 5 ? 8 : 4, THREADS = 32 * ROWS;
   static constexpr int SIDE = kNlTile + 2 * H, POINTS = (ROWS + 2 * H) * SIDE;
-  static constexpr size_t WEIGHTS = (size_t)(2 * H + 1) * SIDE * ROWS * kNlTile * sizeof(f32x2);
+  static constexpr size_t WEIGHTS = (size_t)(2 * H + 1) * SIDE * ROWS * kNlTile * sizeof(float);
   static constexpr size_t STAGE = (size_t)POINTS * kNlPix * sizeof(float);
   static constexpr int STAGES = WEIGHTS + 3 * STAGE <= 224 * 1024 ? 3 : WEIGHTS + 2 * STAGE <= 224 * 1024 ? 2 : 1;
   static constexpr size_t SMEM = WEIGHTS + STAGES * STAGE;
 };
 
 // out[pt] (+)= sum_o w[pt, o0 + o] x[pt + off[o]]. Warp: 8 scan points of one
-// row, lanes: pattern pixels. The window is walked by row di; a neighbour's
-// pixels are read from shared memory once and used for every point whose
-// window reaches it, one packed FFMA per weight and pixel pair. The weights
-// sit in shared memory as (w, w) pairs in the order of use: [di][neighbour
-// column][row][point]. Each (di, dj) may appear at most once per call; an
-// offset outside the window makes the outputs NaN. Bound by shared-memory reads
-// (the weights of a pixel pair): 65,536 patterns of 60^2 px, k_rad 3: 2.37 ->
-// 1.54 ms; 2,867 of 128^2 px, k_rad 5: 1.47 -> 0.78 ms.
+// row, lanes: pairs of pattern pixels. The window is walked by row di; a
+// neighbour's pixels are read from shared memory once and used for every point
+// whose window reaches it. The weights sit in shared memory in the order of use,
+// [di][neighbour column][row][point], four points a read. Each (di, dj) may
+// appear at most once per call; an offset outside the window makes the outputs
+// NaN. Bound by shared-memory reads with one CTA per SM (window of points and
+// weights), so weights are kept as single values: as (w, w) pairs for the packed
+// FFMA they take two points a read. 65,536 patterns of 60^2 px, k_rad 3: 1.54 ms
+// with pairs, 1.26 now (2.37 per-offset reads); 2,867 of 128^2 px, k_rad 5:
+// 0.78, 0.63 (1.47). The same sums in the same order.
 template <int H, bool VEC>
 __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float* __restrict__ data, int hs, int ws,
                                                              int n_pix, int pix_per_split, int64_t ld,
@@ -849,8 +851,8 @@ __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float
                                                              int64_t ld_out) {
   using S = NlAvg<H>;
   constexpr int side = S::SIDE, w2 = 2 * H + 1, PTS = S::ROWS * kNlTile;
-  extern __shared__ __align__(16) f32x2 w_s[];
-  float* T = reinterpret_cast<float*>(w_s + w2 * side * PTS);
+  extern __shared__ __align__(16) float w_s[];
+  float* T = w_s + w2 * side * PTS;
   __shared__ int any_bad;
   __shared__ int64_t src[S::POINTS];
   const int tiles_x = (ws + kNlTile - 1) / kNlTile;
@@ -871,7 +873,7 @@ __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float
       nl_stage<VEC, S::POINTS, S::THREADS>(T + c * S::POINTS * kNlPix, data, src, pix_begin + c * kNlPix, pix_end);
     cp_async_commit();
   }
-  for (int i = threadIdx.x; i < w2 * side * PTS; i += S::THREADS) w_s[i] = 0ull;
+  for (int i = threadIdx.x; i < w2 * side * PTS; i += S::THREADS) w_s[i] = 0.f;
   __syncthreads();
   for (int i = threadIdx.x; i < PTS * n_off; i += S::THREADS) {
     const int o = i / PTS, pt = i % PTS;
@@ -882,7 +884,7 @@ __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float
     }
     const int y = y0 + pt / kNlTile, x = x0 + pt % kNlTile;
     const float w = y < hs && x < ws ? weights[((int64_t)y * ws + x) * n_off_total + o0 + o] : 0.f;
-    w_s[((di + H) * side + pt % kNlTile + dj + H) * PTS + pt] = pack2(w, w);
+    w_s[((di + H) * side + pt % kNlTile + dj + H) * PTS + pt] = w;
   }
   const int y = y0 + wid;
   for (int c = 0; c < n_chunks; ++c) {
@@ -903,23 +905,30 @@ __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float
       __syncthreads();
     }
     if (y >= hs) continue;
-    f32x2 s[kNlTile];
+    float2 s[kNlTile];
 #pragma unroll
-    for (int j = 0; j < kNlTile; ++j) s[j] = 0ull;
+    for (int j = 0; j < kNlTile; ++j) s[j] = make_float2(0.f, 0.f);
     const float* row = T + ((c % S::STAGES) * S::POINTS + wid * side) * kNlPix;
-    const f32x2* wr = w_s + wid * kNlTile;
+    const float* wr = w_s + wid * kNlTile;
 #pragma unroll 1
     for (int a = 0; a < w2; ++a, row += side * kNlPix, wr += side * PTS) {
 #pragma unroll
       for (int k = 0; k < side; ++k) {
-        const f32x2 v = nl_px(row + k * kNlPix, lane);
-        const ulonglong2* w4 = reinterpret_cast<const ulonglong2*>(wr + k * PTS);
+        const float2 v = unpack2(nl_px(row + k * kNlPix, lane));
+        const float4* w4 = reinterpret_cast<const float4*>(wr + k * PTS);
 #pragma unroll
-        for (int j = 0; j < kNlTile; j += 2) {
-          if (k - j < 0 || k - j - 1 > 2 * H) continue;
-          const ulonglong2 w = w4[j / 2];
-          if (k - j <= 2 * H) s[j] = fma2(w.x, v, s[j]);
-          if (k - j - 1 >= 0) s[j + 1] = fma2(w.y, v, s[j + 1]);
+        for (int j = 0; j < kNlTile; j += 4) {
+          if (k - j < 0 || k - j - 3 > 2 * H) continue;
+          const float4 w = w4[j / 4];
+          auto add = [&](int i, float wi) {
+            if (k - i < 0 || k - i > 2 * H) return;
+            s[i].x = fmaf(wi, v.x, s[i].x);
+            s[i].y = fmaf(wi, v.y, s[i].y);
+          };
+          add(j, w.x);
+          add(j + 1, w.y);
+          add(j + 2, w.z);
+          add(j + 3, w.w);
         }
       }
     }
@@ -927,7 +936,7 @@ __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float
     for (int j = 0; j < kNlTile; ++j) {
       if (x0 + j >= ws) break;
       float* dp = out + ((int64_t)y * ws + x0 + j) * ld_out + p0 + 2 * lane;
-      float2 r = unpack2(s[j]);
+      float2 r = s[j];
       if (any_bad) r.x = r.y = NAN;
       if (VEC) {
         if (p0 + 2 * lane < pix_end) {
