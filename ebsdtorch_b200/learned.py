@@ -201,6 +201,10 @@ class OrientationCNN:
         B = x.shape[0]
         if B % 128:
             raise ValueError("batch size must be a multiple of 128")
+        if x.numel() != B * self.H * self.W or x.device.type != self.device.type:
+            # the layers read B * H * W pixels from x's memory
+            raise ValueError(f"{tuple(x.shape)} patterns on {x.device} do not fit a {self.H} x {self.W} network on "
+                             f"{self.device}")
         a, h, w = x.contiguous(), self.H, self.W
         if keep or a.dtype != torch.float32:
             # bf16 pixels, which backward() reads again; inference rounds them in the first layer
