@@ -359,6 +359,10 @@ static int check_row_out(const RowOut& o, int n_pix) {
   return 0;
 }
 
+// Every output may be NULL; with none wanted nothing is launched (finalize_row
+// writes FP32 rows when it is asked for nothing else).
+static bool no_output(const RowOut& o) { return !o.f32 && !o.lp && !o.norm && !o.lp_scale; }
+
 static int row_grid(int64_t n_rows, size_t smem, const void* fn, int threads) {
   int per_sm = 1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess ||
@@ -396,7 +400,7 @@ static int project_rows(const float* img, int mp_h, int mp_w2, const float* rays
   EBSD_ARG_CHECK(!QUADS || (reinterpret_cast<uintptr_t>(img) & 15) == 0, "quads must be 16-byte aligned");
   EBSD_ARG_CHECK(!QUADS || quads_fit(mp_h, mp_w2), "master pattern shape (%d, %d) too large for quads", mp_h, mp_w2);
   if (int rc = check_row_out(o, n_pix)) return rc;
-  if (n_rows == 0) return 0;
+  if (n_rows == 0 || no_output(o)) return 0;
   const float4* q = reinterpret_cast<const float4*>(quats);
   cudaStream_t s = as_stream(stream);
   if (n_pix <= kSmallRowPix)
@@ -479,7 +483,7 @@ extern "C" int ebsd_prep_patterns_typed(const void* patterns, int pattern_dtype,
   EBSD_ARG_CHECK(pattern_stride >= (int64_t)height * width, "pattern_stride too small");
   RowOut o{out_f32, ld_f32, out_lp, lp_dtype, ld_lp, out_norm, out_lp_scale};
   if (int rc = check_row_out(o, n_pix)) return rc;
-  if (n_rows == 0) return 0;
+  if (n_rows == 0 || no_output(o)) return 0;
   switch (pattern_dtype) {
     case EBSD_PAT_U16:
       return launch_prep(static_cast<const uint16_t*>(patterns), n_rows, height, width, pattern_stride, binning,

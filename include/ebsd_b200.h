@@ -104,7 +104,7 @@ int ebsd_gather_rows(const float* in, int64_t n_in, int width, const int64_t* in
  * rays_soa:       3 x n_pix fp32 unit rays (x row, y row, z row), already
  *                 masked.
  * quats:          (n_rows, 4) fp32 orientations.
- * Outputs (each may be NULL):
+ * Outputs (each may be NULL; with all four NULL nothing is done):
  *   out_f32 (n_rows x ld_f32): zero-mean rows (or raw rows if !subtract_mean)
  *   out_lp  (n_rows x ld_lp) : those rows scaled to unit L2 norm, in lp_dtype;
  *                              e4m3 rows are further scaled by 1/out_lp_scale
