@@ -196,20 +196,23 @@ class OrientationCNN:
             t.numel() for d in (self.fc1, self.fc2) for t in (d.w, d.b))
 
     def forward(self, x: torch.Tensor, keep: bool = True) -> torch.Tensor:
-        """x: (B, H, W) float32 -> (B, 6) float32 6-D rotation outputs. With
-        keep=False the activations needed by backward() are not retained."""
+        """x: (B, H, W) patterns (types other than float32 are converted) ->
+        (B, 6) float32 6-D rotation outputs. With keep=False the activations
+        needed by backward() are not retained."""
         B = x.shape[0]
         if B % 128:
             raise ValueError("batch size must be a multiple of 128")
-        if x.numel() != B * self.H * self.W or x.device.type != self.device.type:
-            # the layers read B * H * W pixels from x's memory
+        devices = {c.w.device for c in self.convs}
+        if x.numel() != B * self.H * self.W or x.device.type != self.device.type or devices - {x.device}:
+            # the layers read B * H * W pixels from x's memory, and their weights
             raise ValueError(f"{tuple(x.shape)} patterns on {x.device} do not fit a {self.H} x {self.W} network on "
                              f"{self.device}")
-        a, h, w = x.contiguous(), self.H, self.W
-        if keep or a.dtype != torch.float32:
+        a, h, w = x.float().contiguous(), self.H, self.W  # the kernels read FP32 pixels
+        if keep:
             # bf16 pixels, which backward() reads again; inference rounds them in the first layer
-            a = torch.empty((B, h, w), dtype=torch.bfloat16, device=x.device)
-            call("ebsd_cnn_scale_cast", ptr(x.contiguous()), x.numel(), 1.0, ptr(a), _stream(x))
+            x16 = torch.empty((B, h, w), dtype=torch.bfloat16, device=x.device)
+            call("ebsd_cnn_scale_cast", ptr(a), a.numel(), 1.0, ptr(x16), _stream(x))
+            a = x16
         self._keep = []
         a32 = None
         for i, conv in enumerate(self.convs):
