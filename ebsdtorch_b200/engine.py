@@ -292,16 +292,19 @@ class Searcher:
                     "manhattan": SIM_MANHATTAN}[cfg.similarity]
         self._plan()
 
-    def _plan(self):
+    def _plan(self, ask_driver: bool = False):
         drow = RowSet.bytes_per_row(self.n_pix, self.lp_dtype, self.keep_f32)
         qrow_base = RowSet.bytes_per_row(self.n_pix, self.lp_dtype, self.keep_f32)
         qrow = qrow_base + self.k * 12
         budget = self.cfg.workspace_bytes
-        if not budget and self.device.type == "cuda":
-            # all rows at once, where the allocator's cache already has room
+        self.from_cache = False
+        if not budget and not ask_driver and self.device.type == "cuda":
+            # all rows at once, where the allocator's cache already has room; how
+            # much of it one allocation can get is known when it is asked (run)
             whole = round_up(self.n_dict, TILE_D) * drow + round_up(self.n_queries, TILE_Q) * qrow
             if whole <= 0.9 * self.cfg.free_share * cached_bytes(self.device):
                 budget = whole
+                self.from_cache = True
         if not budget:
             budget = int(default_budget(self.device) * self.cfg.free_share)
         q_min = min(round_up(self.n_queries, TILE_Q), 16384)
@@ -332,6 +335,19 @@ class Searcher:
         float32) on the device. With check=False nothing synchronises (for
         CUDA-graph capture): the caller reads `status` (a device int32 word,
         non-zero after a kernel timeout) later with check_status()."""
+        if self.from_cache:
+            try:
+                return self._run(fill_dict, fill_queries, resident, check, status)
+            except torch.OutOfMemoryError:
+                if self.device.type == "cuda" and torch.cuda.is_current_stream_capturing():
+                    raise
+            # fragments and blocks of graph pools count as cached: plan as if
+            # there were no cache, with what the attempt held given back
+            torch.cuda.empty_cache()
+            self._plan(ask_driver=True)
+        return self._run(fill_dict, fill_queries, resident, check, status)
+
+    def _run(self, fill_dict, fill_queries, resident, check, status):
         dev, Q, D, k = self.device, self.n_queries, self.n_dict, self.k
         out_val = torch.empty((Q, k), dtype=torch.float32, device=dev)
         out_idx = torch.empty((Q, k), dtype=torch.int64, device=dev)
