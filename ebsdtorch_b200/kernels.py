@@ -125,17 +125,28 @@ def sampling_quads(master_pattern: torch.Tensor) -> torch.Tensor:
 
 # A table is built for one call from this many simulated pixels, and this many
 # per master-pattern pixel: a sample gains about 2 ps (6.6 against 9 ps at
-# 128 x 128 px), the table costs 3 ps a master-pattern pixel and a launch.
-QUADS_MIN_SAMPLES, QUADS_MIN_RATIO = 1 << 22, 4
+# 128 x 128 px), the table costs 3 ps a master-pattern pixel and a launch. It
+# is 4 x its image, and beyond L2 it costs more than it saves: 36,829 rows of
+# 60^2 px from masters of 2,001 / 3,001 / 4,001 rows take 0.94 / 1.27 / 1.81 ms
+# through tables of 128 / 288 / 512 MB and 1.55 / 1.57 / 1.61 without; 8,192 of
+# 160^2 px 3.2 / 5.3 / 6.0 and 4.4 / 4.9 / 6.7; the refinement of 2,048 patterns
+# of 128^2 px 13.2 / 21.2 / 29.8 and 23.5 / 25.8 / 27.2.
+QUADS_MIN_SAMPLES, QUADS_MIN_RATIO, QUADS_MAX_PIXELS = 1 << 22, 4, 20 << 20
+
+
+def quads_bytes(master_pattern: torch.Tensor, n_samples: int) -> int:
+    """Size of the master pattern's gather table where `n_samples` samples repay
+    it and its sizes allow one (quads_fit in sampling.cuh), else 0."""
+    h, w = master_pattern.shape
+    if n_samples < max(QUADS_MIN_SAMPLES, QUADS_MIN_RATIO * h * w) or h * w > QUADS_MAX_PIXELS or h > 65535 \
+            or w > 1 << 22:
+        return 0
+    return 16 * h * w
 
 
 def quads_for(master_pattern: torch.Tensor, n_samples: int) -> Optional[torch.Tensor]:
-    """The master pattern's gather table where `n_samples` samples repay it and
-    its sizes allow one (quads_fit in sampling.cuh)."""
-    h, w = master_pattern.shape
-    if n_samples < max(QUADS_MIN_SAMPLES, QUADS_MIN_RATIO * h * w) or h > 65535 or w > 1 << 22 or h * w >= 1 << 31:
-        return None
-    return sampling_quads(master_pattern)
+    """The gather table that quads_bytes asks for, or None."""
+    return sampling_quads(master_pattern) if quads_bytes(master_pattern, n_samples) else None
 
 
 def project(master_pattern: torch.Tensor, rays_soa: torch.Tensor, quats: torch.Tensor, out: RowBuffers,
