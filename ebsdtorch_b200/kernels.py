@@ -145,8 +145,14 @@ def quads_bytes(master_pattern: torch.Tensor, n_samples: int) -> int:
 
 
 def quads_for(master_pattern: torch.Tensor, n_samples: int) -> Optional[torch.Tensor]:
-    """The gather table that quads_bytes asks for, or None."""
-    return sampling_quads(master_pattern) if quads_bytes(master_pattern, n_samples) else None
+    """The gather table that quads_bytes asks for, or None; also None where the
+    device has no room for it: the route without one needs no memory."""
+    if not quads_bytes(master_pattern, n_samples):
+        return None
+    try:
+        return sampling_quads(master_pattern)
+    except torch.OutOfMemoryError:
+        return None
 
 
 def project(master_pattern: torch.Tensor, rays_soa: torch.Tensor, quats: torch.Tensor, out: RowBuffers,

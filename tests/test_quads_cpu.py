@@ -17,3 +17,11 @@ def _master(h):
 def test_rule(monkeypatch, h, samples, made):
     monkeypatch.setattr(kernels, "sampling_quads", lambda mp: "table")
     assert kernels.quads_for(_master(h), samples) == ("table" if made else None)
+
+
+def test_no_room_for_a_table_means_none(monkeypatch):
+    def full(mp):
+        raise torch.OutOfMemoryError("full")
+
+    monkeypatch.setattr(kernels, "sampling_quads", full)
+    assert kernels.quads_for(_master(1001), 1 << 30) is None
