@@ -156,10 +156,11 @@ def quads_for(master_pattern: torch.Tensor, n_samples: int) -> Optional[torch.Te
 
 
 def project(master_pattern: torch.Tensor, rays_soa: torch.Tensor, quats: torch.Tensor, out: RowBuffers,
-            subtract_mean: bool = True, quads: Optional[torch.Tensor] = None) -> None:
+            subtract_mean: bool = True, quads=None) -> None:
     """K1: simulated dictionary rows for `quats` into `out` (row i <- quats[i]).
     quads: quads_for(master_pattern, all samples), for callers that project in several
-    calls; without it a call that is large enough makes its own."""
+    calls, or False for the route without a table; with None a call that is
+    large enough makes its own."""
     _cuda(master_pattern, "master_pattern", torch.float32)
     _cuda(rays_soa, "rays_soa", torch.float32)
     _cuda(quats, "quats", torch.float32)
@@ -168,8 +169,13 @@ def project(master_pattern: torch.Tensor, rays_soa: torch.Tensor, quats: torch.T
     n_pix = rays_soa.shape[1]
     if quads is None:
         quads = quads_for(master_pattern, quats.shape[0] * n_pix)
-    name, img = ("ebsd_project_dictionary", master_pattern) if quads is None else \
-        ("ebsd_project_dictionary_quads", quads)
+    if quads is None or quads is False:
+        name, img = "ebsd_project_dictionary", master_pattern
+    else:
+        name, img = "ebsd_project_dictionary_quads", _cuda(quads, "quads", torch.float32)
+        if quads.shape != (*master_pattern.shape, 4) or quads.device != master_pattern.device:
+            raise ValueError(f"quads {tuple(quads.shape)} on {quads.device} is not the table of a "
+                             f"{tuple(master_pattern.shape)} master pattern on {master_pattern.device}")
     call(name, ptr(img), master_pattern.shape[0], master_pattern.shape[1],
          ptr(rays_soa), n_pix, ptr(quats), quats.shape[0], int(bool(subtract_mean)), *out.args(n_pix),
          _stream(quats.device))
