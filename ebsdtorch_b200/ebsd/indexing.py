@@ -23,6 +23,7 @@ Both functions also store ``experiment_patterns.raw_indexing_indices[phase]``
 
 from __future__ import annotations
 
+from dataclasses import replace
 from typing import List, Optional, Union
 
 import numpy as np
@@ -187,6 +188,33 @@ def _metric_dtype(match_dtype):
         else torch.float32
 
 
+def _plan_search(mp_t, n_samples: int, n_dict: int, n_q: int, n_pix: int, k: int, cfg: SearchConfig, dev):
+    """The Searcher of a phase, and a function that returns kernels.project's
+    gather table for its `n_samples` dictionary pixels, or False. The table is
+    made when first asked for, after the search has its own memory. A budget
+    given by the caller covers it too: there is none where the budget is less
+    than eight tables, or too small for the rows without the table's share."""
+    nbytes = kernels.quads_bytes(mp_t, n_samples)
+    searcher, made = None, []
+    if nbytes and cfg.workspace_bytes:
+        if 8 * nbytes <= cfg.workspace_bytes:
+            try:
+                searcher = Searcher(n_dict, n_q, n_pix, k, replace(cfg, workspace_bytes=cfg.workspace_bytes - nbytes),
+                                    dev)
+            except MemoryError:
+                pass
+        if searcher is None:
+            nbytes = 0
+
+    def table():
+        if not made:
+            quads = kernels.quads_for(mp_t, n_samples) if nbytes else None
+            made.append(False if quads is None else quads)
+        return made[0]
+
+    return searcher or Searcher(n_dict, n_q, n_pix, k, cfg, dev), table
+
+
 def dictionary_index_orientations(
     master_patterns,
     geometry,
@@ -234,10 +262,11 @@ def dictionary_index_orientations(
             n_pix = rays.shape[1]
             pats = _pattern_source(experiment_patterns, dev)
 
-            def fill_dict(d0, d1, bufs, mp_t=mp_t, rays=rays, grid=grid):
-                kernels.project(mp_t, rays, grid.finish()[d0:d1], bufs, subtract_mean=True)
+            searcher, table = _plan_search(mp_t, grid.n * n_pix, grid.n, n_q, n_pix, int(top_k_matches), cfg, dev)
 
-            searcher = Searcher(grid.n, n_q, n_pix, int(top_k_matches), cfg, dev)
+            def fill_dict(d0, d1, bufs, mp_t=mp_t, table=table, rays=rays, grid=grid):
+                kernels.project(mp_t, rays, grid.finish()[d0:d1], bufs, subtract_mean=True, quads=table())
+
             idx, val = searcher.run(fill_dict, _query_fill(pats, virtual_binning, pix_index, n_pix, subtract, dev))
             _store(experiment_patterns, i, grid.finish(), idx, val, _metric_dtype(match_dtype))
     experiment_patterns.combine_indexing_results(higher_is_better=(distance_metric == "angular"))
@@ -410,16 +439,20 @@ def pca_dictionary_index_orientations(
                     sample_ori_fz_laue_angle(mp.laue_group, dictionary_resolution_index_deg, dev)
                 del ori_learn
             proj = _Projector(comps)
-            quads = kernels.quads_for(mp_t, ori.shape[0] * P)
             n_comp = comps.shape[0]
+            cfg = SearchConfig(precision=precision, rescore_k=rescore_k,
+                               similarity=_similarity(distance_metric, similarity), workspace_bytes=workspace_bytes,
+                               free_share=0.7)
+            searcher, table = _plan_search(mp_t, ori.shape[0] * P, ori.shape[0], n_q, n_comp, int(top_k_matches), cfg,
+                                           dev)
             pats = _pattern_source(experiment_patterns, dev)
             qfill_full = _query_fill(pats, virtual_binning, pix_index, P, subtract, dev)
 
-            def fill_dict(d0, d1, bufs, mp_t=mp_t, quads=quads, rays=rays, ori=ori, proj=proj):
+            def fill_dict(d0, d1, bufs, mp_t=mp_t, table=table, rays=rays, ori=ori, proj=proj):
                 for s0 in range(d0, d1, sub_chunk):
                     s1 = min(d1, s0 + sub_chunk)
                     X = torch.empty((s1 - s0, P), dtype=torch.float32, device=dev)
-                    kernels.project(mp_t, rays, ori[s0:s1], RowBuffers(f32=X), subtract_mean=True, quads=quads)
+                    kernels.project(mp_t, rays, ori[s0:s1], RowBuffers(f32=X), subtract_mean=True, quads=table())
                     Y = bufs.f32[s0 - d0:s1 - d0] if bufs.f32 is not None else torch.empty(
                         (s1 - s0, n_comp), dtype=torch.float32, device=dev)
                     proj(X, Y)
@@ -435,10 +468,6 @@ def pca_dictionary_index_orientations(
                     proj(X, Y)
                     _finish_rows(Y, _slice(bufs, s0 - q0, s1 - q0))
 
-            cfg = SearchConfig(precision=precision, rescore_k=rescore_k,
-                               similarity=_similarity(distance_metric, similarity), workspace_bytes=workspace_bytes,
-                               free_share=0.7)
-            searcher = Searcher(ori.shape[0], n_q, n_comp, int(top_k_matches), cfg, dev)
             idx, val = searcher.run(fill_dict, fill_queries)
             if int(proj.status.item()) != 0:
                 raise RuntimeError("PCA projection GEMM reported a device timeout")
