@@ -74,8 +74,6 @@ class SearchConfig:
     rescore_k: int = 32
     similarity: str = "dot"
     workspace_bytes: Optional[int] = None
-    # share of the free memory the default budget may take
-    free_share: float = 1.0
     query_chunk: Optional[int] = None
     dict_chunk: Optional[int] = None
     # upper bound on the planned query chunk (host-resident patterns stream in
@@ -92,6 +90,8 @@ class SearchConfig:
     # re-score in FP32 only the candidates whose bf16 score, widened by a
     # rigorous rounding bound, can still reach the exact top-k (same results)
     rescore_gate: bool = True
+    # share of the free memory the default budget may take
+    free_share: float = 1.0
 
     def validate(self):
         if self.precision not in LP_DTYPES:
