@@ -837,12 +837,16 @@ struct NlAvg {
 // whose window reaches it. The weights sit in shared memory in the order of use,
 // [di][neighbour column][row][point], four points a read. Each (di, dj) may
 // appear at most once per call; an offset outside the window makes the outputs
-// NaN. Bound by shared-memory reads with one CTA per SM (window of points and
+// NaN. WHOLE: the call's offsets fill the window; otherwise cells that are none of
+// them are skipped, since a zero weight would let a non-finite value there
+// through (both loops in one kernel: 1.40 instead of 1.34 ms for an NLPAR call of
+// 2,867 patterns of 128^2 px, k_rad 5).
+// Bound by shared-memory reads with one CTA per SM (window of points and
 // weights), so weights are kept as single values: as (w, w) pairs for the packed
 // FFMA they take two points a read. 65,536 patterns of 60^2 px, k_rad 3: 1.54 ms
 // with pairs, 1.26 now (2.37 per-offset reads); 2,867 of 128^2 px, k_rad 5:
 // 0.78, 0.63 (1.47). The same sums in the same order.
-template <int H, bool VEC>
+template <int H, bool VEC, bool WHOLE>
 __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float* __restrict__ data, int hs, int ws,
                                                              int n_pix, int pix_per_split, int64_t ld,
                                                              const int* __restrict__ offsets, int o0, int n_off,
@@ -854,6 +858,7 @@ __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float
   extern __shared__ __align__(16) float w_s[];
   float* T = w_s + w2 * side * PTS;
   __shared__ int any_bad;
+  __shared__ unsigned present[w2];  // !WHOLE: per window row, the columns among this call's offsets
   __shared__ int64_t src[S::POINTS];
   const int tiles_x = (ws + kNlTile - 1) / kNlTile;
   const int y0 = (blockIdx.x / tiles_x) * S::ROWS, x0 = (blockIdx.x % tiles_x) * kNlTile;
@@ -861,6 +866,7 @@ __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float
   // this CTA's range of pattern pixels (blockIdx.y); outputs are disjoint
   const int pix_begin = blockIdx.y * pix_per_split, pix_end = min(n_pix, pix_begin + pix_per_split);
   if (threadIdx.x == 0) any_bad = 0;
+  if (!WHOLE && threadIdx.x < w2) present[threadIdx.x] = 0u;
   for (int i = threadIdx.x; i < S::POINTS; i += S::THREADS) {
     const int py = y0 - H + i / side, px = x0 - H + i % side;
     src[i] = py >= 0 && py < hs && px >= 0 && px < ws ? ((int64_t)py * ws + px) * ld : -1;
@@ -882,6 +888,7 @@ __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float
       any_bad = 1;
       continue;
     }
+    if (!WHOLE && pt == 0) atomicOr(&present[di + H], 1u << (dj + H));
     const int y = y0 + pt / kNlTile, x = x0 + pt % kNlTile;
     const float w = y < hs && x < ws ? weights[((int64_t)y * ws + x) * n_off_total + o0 + o] : 0.f;
     w_s[((di + H) * side + pt % kNlTile + dj + H) * PTS + pt] = w;
@@ -912,6 +919,7 @@ __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float
     const float* wr = w_s + wid * kNlTile;
 #pragma unroll 1
     for (int a = 0; a < w2; ++a, row += side * kNlPix, wr += side * PTS) {
+      const unsigned cells = WHOLE ? 0u : present[a];
 #pragma unroll
       for (int k = 0; k < side; ++k) {
         const float2 v = unpack2(nl_px(row + k * kNlPix, lane));
@@ -922,6 +930,7 @@ __global__ void __launch_bounds__(NlAvg<H>::THREADS) k_nlpar_average(const float
           const float4 w = w4[j / 4];
           auto add = [&](int i, float wi) {
             if (k - i < 0 || k - i > 2 * H) return;
+            if (!WHOLE && !(cells >> (k - i) & 1u)) return;
             s[i].x = fmaf(wi, v.x, s[i].x);
             s[i].y = fmaf(wi, v.y, s[i].y);
           };
@@ -1100,7 +1109,8 @@ static int nl_launch(bool average, const float* data, int hs, int ws, int n_pix,
   } else {
     using S = NlAvg<H>;
     const int tiles = ceil_div(hs, S::ROWS) * ceil_div(ws, kNlTile);
-    const auto fn = k_nlpar_average<H, VEC>;
+    const bool whole = n_off == (2 * H + 1) * (2 * H + 1);
+    const auto fn = whole ? k_nlpar_average<H, VEC, true> : k_nlpar_average<H, VEC, false>;
     EBSD_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
     // ranges of whole chunks, at least 8 chunks each
     const int n_chunks = ceil_div(n_pix, kNlPix);
