@@ -76,6 +76,7 @@ SIGNATURES = {
     "ebsd_pcfit_prep": (i32, [vp, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp]),
     "ebsd_pcfit_reduce": (i32, [vp, i32, i32, i32, i32, i64, vp, vp, vp]),
     "ebsd_pcfit_xcorr_table_bytes": (i64, [i32, i32]),
+    "ebsd_pcfit_xcorr_takes_quads": (i32, [i32, i32]),
     "ebsd_pcfit_xcorr_tables": (i32, [i32, i32, vp, i64, vp]),
     "ebsd_pcfit_spectra": (i32, [vp, i64, i64, i32, i32, vp, vp, vp, vp]),
     "ebsd_pcfit_spectra_quads": (i32, [vp, i64, i64, i32, i32, vp, vp, vp, vp]),

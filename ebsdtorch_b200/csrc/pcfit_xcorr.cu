@@ -729,6 +729,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_xc_max(const XcParams p) {
 // waits on its loads (16 lines of spectrum and terms per thread, from L2), so
 // their number counts: 64 loads of 4 bytes took about 0.20 of a batch's 0.507 ms
 // (16 patterns, 78 x 78 px, 1,024 simulated ones); 16 of 16 bytes: 0.465 in all.
+// The spectra then take longer to store (0.057 against 0.053 ms), and k_xc_max
+// reads quads no faster than planes, so detectors that it serves (above about
+// 96 x 96 px) keep planes (ebsd_pcfit_xcorr_takes_quads): spectra and correlation
+// of a batch 1.445 ms at 104 x 104 px, 1.459 from quads.
 template <int CPT, bool QUADS>  // x chunks of 8 per thread: NB / 8 <= 4 CPT
 __global__ void __launch_bounds__(THREADS, 1) k_xc_max_tm(const XcParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -1096,6 +1100,11 @@ XcParams base_params(const Plan& pl, const void* tables, int* status, bool quads
 }
 
 }  // namespace
+
+extern "C" int ebsd_pcfit_xcorr_takes_quads(int hp, int wp) {
+  Plan pl;
+  return make_plan(hp, wp, pl) && pl.pp_tm > 0 ? 1 : 0;
+}
 
 extern "C" int64_t ebsd_pcfit_xcorr_table_bytes(int hp, int wp) {
   Plan pl;

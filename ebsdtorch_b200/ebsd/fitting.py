@@ -213,6 +213,12 @@ def xcorr_supported(hp: int, wp: int) -> bool:
     return int(load().ebsd_pcfit_xcorr_table_bytes(int(hp), int(wp))) > 0
 
 
+def spectra_layout(hp: int, wp: int) -> str:
+    """Suffix of the spectra, terms and correlation entry points of an
+    enlarged detector: "_quads", or "" for planes."""
+    return "_quads" if load().ebsd_pcfit_xcorr_takes_quads(int(hp), int(wp)) else ""
+
+
 # sub-batch of the dictionary projected and transformed at once (the
 # correlation itself runs per dictionary batch on the spectra)
 MAX_SIM_BYTES = 2 << 30
@@ -221,19 +227,21 @@ MAX_SIM_BYTES = 2 << 30
 def _search_dft(mp_t, padded, quats, pix64, z_vals, tilt, sec_tilt, det, bs, batch_local, best, best_idx, stream):
     """The search with the correlation in the project's kernels: spectra of
     the patterns and of each projected dictionary sub-batch
-    (ebsd_pcfit_spectra_quads), the per-batch max over all shifts
-    (ebsd_pcfit_xcorr_max_quads) and the running best (ebsd_pcfit_fold)."""
+    (ebsd_pcfit_spectra), the per-batch max over all shifts
+    (ebsd_pcfit_xcorr_max) and the running best (ebsd_pcfit_fold); the spectra
+    in quads where the correlation kernel gains by them (spectra_layout)."""
     dev = padded.device
     B, hp, wp = padded.shape
     n_dict = quats.shape[0]
+    quad = spectra_layout(hp, wp)
     spec_len = 4 * (hp // 2 + 1) * (wp // 2 + 1)
     tables = torch.empty((int(load().ebsd_pcfit_xcorr_table_bytes(hp, wp)),), dtype=torch.uint8, device=dev)
     call("ebsd_pcfit_xcorr_tables", hp, wp, ptr(tables), tables.numel(), stream)
     status = torch.zeros(1, dtype=torch.int32, device=dev)
     pspec = torch.empty((B, spec_len), dtype=torch.float32, device=dev)
-    call("ebsd_pcfit_spectra_quads", ptr(padded), hp * wp, B, hp, wp, ptr(tables), ptr(pspec), ptr(status), stream)
+    call("ebsd_pcfit_spectra" + quad, ptr(padded), hp * wp, B, hp, wp, ptr(tables), ptr(pspec), ptr(status), stream)
     terms = torch.empty_like(pspec)
-    call("ebsd_pcfit_pattern_terms_quads", ptr(pspec), B, hp, wp, ptr(terms), stream)
+    call("ebsd_pcfit_pattern_terms" + quad, ptr(pspec), B, hp, wp, ptr(terms), stream)
     keys = torch.zeros((B * hp * wp,), dtype=torch.int64, device=dev)
     sub = max(1, min(bs, n_dict, MAX_SIM_BYTES // (hp * wp * 4)))
     sims = torch.empty((sub, hp * wp), dtype=torch.float32, device=dev)
@@ -247,8 +255,8 @@ def _search_dft(mp_t, padded, quats, pix64, z_vals, tilt, sec_tilt, det, bs, bat
                 n = min(sub, j_end - s)
                 kernels.project(mp_t, rays, quats[s:s + n], RowBuffers(f32=sims[:n]), subtract_mean=False,
                                quads=quads)
-                call("ebsd_pcfit_spectra_quads", ptr(sims), hp * wp, n, hp, wp, ptr(tables), ptr(spec), ptr(status), stream)
-                call("ebsd_pcfit_xcorr_max_quads", ptr(spec), n, ptr(terms), B, hp, wp, ptr(tables), ptr(keys),
+                call("ebsd_pcfit_spectra" + quad, ptr(sims), hp * wp, n, hp, wp, ptr(tables), ptr(spec), ptr(status), stream)
+                call("ebsd_pcfit_xcorr_max" + quad, ptr(spec), n, ptr(terms), B, hp, wp, ptr(tables), ptr(keys),
                      (s - j) if batch_local else s, ptr(status), stream)
             call("ebsd_pcfit_fold", ptr(keys), keys.numel(), ptr(best[zi]), ptr(best_idx[zi]), stream)
     if int(status.item()) != 0:

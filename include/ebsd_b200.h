@@ -530,7 +530,11 @@ int ebsd_pcfit_xcorr_max(const float* sim_spectra, int64_t n_sims, const float* 
                          int padded_h, int padded_w, const void* tables, unsigned long long* keys,
                          int64_t index_base, int* status, void* stream);
 /* The same three with quads: [ky][kx][trig][part], so that the correlation
- * reads 16 bytes at a time (spectra and terms 16-byte aligned). */
+ * reads 16 bytes at a time (spectra and terms 16-byte aligned).
+ * ebsd_pcfit_xcorr_takes_quads: 1 for the detectors whose correlation kernel
+ * does (up to about 96 x 96); at other sizes quads give the same results as
+ * planes but gain nothing. */
+int ebsd_pcfit_xcorr_takes_quads(int padded_h, int padded_w);
 int ebsd_pcfit_spectra_quads(const float* images, int64_t ld, int64_t n, int padded_h, int padded_w,
                              const void* tables, float* spectra, int* status, void* stream);
 int ebsd_pcfit_pattern_terms_quads(const float* spectra, int64_t n, int padded_h, int padded_w, float* terms,
