@@ -219,6 +219,13 @@ def spectra_layout(hp: int, wp: int) -> str:
     return "_quads" if load().ebsd_pcfit_xcorr_takes_quads(int(hp), int(wp)) else ""
 
 
+def _table(mp_t, n_samples: int):
+    """kernels.project's `quads` for a search of `n_samples` pixels: decided
+    here once, not again by every sub-batch."""
+    quads = kernels.quads_for(mp_t, n_samples)
+    return False if quads is None else quads
+
+
 # sub-batch of the dictionary projected and transformed at once (the
 # correlation itself runs per dictionary batch on the spectra)
 MAX_SIM_BYTES = 2 << 30
@@ -246,7 +253,7 @@ def _search_dft(mp_t, padded, quats, pix64, z_vals, tilt, sec_tilt, det, bs, bat
     sub = max(1, min(bs, n_dict, MAX_SIM_BYTES // (hp * wp * 4)))
     sims = torch.empty((sub, hp * wp), dtype=torch.float32, device=dev)
     spec = torch.empty((sub, spec_len), dtype=torch.float32, device=dev)
-    quads = kernels.quads_for(mp_t, len(z_vals) * n_dict * hp * wp)
+    quads = _table(mp_t, len(z_vals) * n_dict * hp * wp)
     for zi in range(len(z_vals)):
         rays = _rays_soa(pix64, float(z_vals[zi]), tilt, sec_tilt, det, dev)
         for j in range(0, n_dict, bs):
@@ -275,7 +282,7 @@ def _search_fft(mp_t, padded, quats, pix64, z_vals, tilt, sec_tilt, det, bs, bat
     wf = wp // 2 + 1
     sub = max(1, min(bs, MAX_PRODUCT_BYTES // (B * hp * wf * 8)))
     sims = torch.empty((min(sub, n_dict), hp * wp), dtype=torch.float32, device=dev)
-    quads = kernels.quads_for(mp_t, len(z_vals) * n_dict * hp * wp)
+    quads = _table(mp_t, len(z_vals) * n_dict * hp * wp)
     for zi in range(len(z_vals)):
         rays = _rays_soa(pix64, float(z_vals[zi]), tilt, sec_tilt, det, dev)
         for j in range(0, n_dict, bs):
