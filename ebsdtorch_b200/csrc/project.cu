@@ -45,14 +45,16 @@ __device__ __forceinline__ T sum_of_warps(const T* red, int n_warps) {
   return v;
 }
 
-// sqrt of an FP64 sum, rounded to FP32: one Newton step in FP64 from the FP32
-// reciprocal root (relative error 2^-22 squared), instead of the FP64 square
-// root's long dependent chain in every thread of the block.
+// sqrt of an FP64 sum, rounded to FP32: two Newton steps in FP64 from the FP32
+// reciprocal root (relative errors 2^-22, 2^-43, then FP64's own), instead of the
+// FP64 square root's long dependent chain in every thread of the block.
 __device__ __forceinline__ float root_of_sum(double x) {
   if (!(x >= 1e-30 && x <= 1e30)) return (float)sqrt(x);
   const float r = rsqrtf((float)x);
-  const double y = x * (double)r;
-  return (float)fma(0.5 * (double)r, fma(-y, y, x), y);
+  const double h = 0.5 * (double)r;
+  double y = x * (double)r;
+  y = fma(h, fma(-y, y, x), y);
+  return (float)fma(h, fma(-y, y, x), y);
 }
 
 // Two FP32 values as e4m3 (round to nearest even, saturating) in 16 bits.
@@ -66,16 +68,43 @@ struct RowScratch {
   float amax[16];
 };
 
-// Row values are in row[0..n); part_sum is this thread's sum of the values it
+// FP32 partial sums of a thread, added in FP64: with 512 of them in a block of any
+// size, each takes at most ceil(n / 512) of a row's n values. Fewer and longer
+// ones would round more; FP64 ones (a conversion a value, 16 a clock on an SM)
+// take K2 from 332 to 365 us for 32,768 patterns of 80^2 px.
+template <int THREADS>
+constexpr int kChains = 512 / THREADS;
+template <int N>
+__device__ __forceinline__ double sum_of_chains(const float (&c)[N]) {
+  if constexpr (N == 4) return ((double)c[0] + c[1]) + ((double)c[2] + c[3]);
+  if constexpr (N == 2) return (double)c[0] + c[1];
+  return c[0];
+}
+
+// The next value of a thread's chains in turn.
+template <int N>
+__device__ __forceinline__ void add_in_turn(float (&c)[N], float v) {
+  const float s = c[0] + v;
+#pragma unroll
+  for (int i = 0; i + 1 < N; ++i) c[i] = c[i + 1];
+  c[N - 1] = s;
+}
+
+// Row values are in row[0..n); part_sum is the sum of the values this thread
 // wrote. Finalise and write the outputs of row `r` (the shared row itself is
-// left as it was): the mean (FP64 sum), then, where a norm or low-precision
-// row is wanted, the norm and absmax of the zero-mean row, then the rows, in
-// 16-byte stores where length and strides allow. The caller's block holds a
-// power-of-two number of warps, has not synchronised since writing the row,
-// and synchronises before the row or the scratch are written again.
+// left as it was): the mean (FP64 sum over the threads), then, where a norm or
+// low-precision row is wanted, the norm and absmax of the zero-mean row, then the
+// rows, in 16-byte stores where length and strides allow. The caller's block has
+// not synchronised since writing the row, and synchronises before the row or the
+// scratch are written again. The loops are short and kept rolled: unrolled by
+// four they hold 48 to 64 registers instead of 32 to 40, which costs K2 CTAs on
+// an SM (65,536 uint16 patterns of 60^2 px 397 us, 380 rolled; half of the pixels
+// masked 294 and 219; 32,768 of 80^2 px 357 and 326).
+template <int THREADS>
 __device__ __forceinline__ void finalize_row(const float* row, int n, double inv_n, int subtract_mean,
                                              double part_sum, int64_t r, const RowOut& o, RowScratch& red) {
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5, n_warps = nt >> 5;
+  constexpr int nt = THREADS, n_warps = nt / 32, C = kChains<THREADS>;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   part_sum = warp_sum(part_sum);
   if (lane == 0) red.sum[wid] = part_sum;
   __syncthreads();
@@ -85,32 +114,36 @@ __device__ __forceinline__ void finalize_row(const float* row, int n, double inv
   const bool vec_f32 = (n & 3) == 0 && (reinterpret_cast<uintptr_t>(f32) & 15) == 0;
   if (!o.lp && !o.norm && !o.lp_scale) {
     if (vec_f32) {
+#pragma unroll 1
       for (int c = tid; c < n / 4; c += nt) {
         const float4 a = row4[c];
         reinterpret_cast<float4*>(f32)[c] = make_float4(a.x - meanf, a.y - meanf, a.z - meanf, a.w - meanf);
       }
     } else {
+#pragma unroll 1
       for (int p = tid; p < n; p += nt) f32[p] = row[p] - meanf;
     }
     return;
   }
-  float ss = 0.0f, amax = 0.0f;
+  float ss[C] = {}, amax = 0.0f;
+#pragma unroll 2
   for (int c = tid; c < n / 4; c += nt) {
     const float4 a = row4[c];
     const float v[4] = {a.x - meanf, a.y - meanf, a.z - meanf, a.w - meanf};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      ss = fmaf(v[e], v[e], ss);
+      ss[e % C] = fmaf(v[e], v[e], ss[e % C]);
       amax = fmaxf(amax, fabsf(v[e]));
     }
   }
-  for (int p = (n & ~3) + tid; p < n; p += nt) {
+  // the last threads, which have the fewest groups of four
+  for (int p = (n & ~3) + nt - 1 - tid; p < n; p += nt) {
     const float v = row[p] - meanf;
-    ss = fmaf(v, v, ss);
+    ss[0] = fmaf(v, v, ss[0]);
     amax = fmaxf(amax, fabsf(v));
   }
   const bool e4m3 = o.lp && o.lp_dtype == EBSD_DT_E4M3;
-  const double wss = warp_sum((double)ss);
+  const double wss = warp_sum(sum_of_chains(ss));
   if (e4m3) amax = warp_max(amax);
   if (lane == 0) {
     red.sq[wid] = wss;
@@ -128,10 +161,13 @@ __device__ __forceinline__ void finalize_row(const float* row, int n, double inv
     if (o.norm) o.norm[r] = nrm;
     if (o.lp_scale) o.lp_scale[r] = qscale;
   }
-  if (f32 && !vec_f32)
+  if (f32 && !vec_f32) {
+#pragma unroll 1
     for (int p = tid; p < n; p += nt) f32[p] = row[p] - meanf;
+  }
   if (!o.lp) {
     if (f32 && vec_f32)
+#pragma unroll 1
       for (int c = tid; c < n / 4; c += nt) {
         const float4 a = row4[c];
         reinterpret_cast<float4*>(f32)[c] = make_float4(a.x - meanf, a.y - meanf, a.z - meanf, a.w - meanf);
@@ -144,6 +180,7 @@ __device__ __forceinline__ void finalize_row(const float* row, int n, double inv
   const float sc = e4m3 ? inv / qscale : inv;
   uint8_t* lp = static_cast<uint8_t*>(o.lp) + r * o.ld_lp * (e4m3 ? 1 : 2);
   const bool vec_lp = (ld_lp & 7) == 0 && (reinterpret_cast<uintptr_t>(o.lp) & 15) == 0;
+#pragma unroll 1
   for (int c = tid; c < (ld_lp + 7) / 8; c += nt) {
     float v[8];
     if (8 * c + 8 <= n) {
@@ -227,7 +264,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 2) k_project(
   for (int64_t r = blockIdx.x; r < n_rows; r += gridDim.x) {
     const float4 q = quats[r];
     const float3 q2 = make_float3(2.0f * q.y, 2.0f * q.z, 2.0f * q.w);
-    float part = 0.0f, part_b = 0.0f;
+    float part[kChains<THREADS>] = {};
     int p = threadIdx.x;
     LambertTap<QUADS> t{};
     float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -242,17 +279,11 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 2) k_project(
       const float4 vn = load_taps(img, mp_h, g, tn);
       const float val = blend(t, v);
       row[p] = val;
-      if constexpr (THREADS == 512) {
-        part += val;
-      } else {
-        const float s = part + val;
-        part = part_b;
-        part_b = s;
-      }
+      add_in_turn(part, val);
       t = tn;
       v = vn;
     }
-    finalize_row(row, n_pix, inv_n, subtract_mean, (double)part + (double)part_b, r, o, red);
+    finalize_row<THREADS>(row, n_pix, inv_n, subtract_mean, sum_of_chains(part), r, o, red);
     __syncthreads();
   }
 }
@@ -291,11 +322,12 @@ __global__ void __launch_bounds__(THREADS) k_prep(const T* __restrict__ pats, in
                                                   int vec4, int subtract_mean, RowOut o) {
   extern __shared__ __align__(16) float row[];
   __shared__ RowScratch red;
+  constexpr int C = kChains<THREADS>;
   const int wb = w / b;
   const float cnt = (float)(b * b);
   for (int64_t r = blockIdx.x; r < n_rows; r += gridDim.x) {
     const T* img = pats + r * stride;
-    float part = 0.0f;
+    float part[C] = {};
     if (vec4) {
       const Vec4<T>* img4 = reinterpret_cast<const Vec4<T>*>(img);
       float4* row4 = reinterpret_cast<float4*>(row);
@@ -304,14 +336,22 @@ __global__ void __launch_bounds__(THREADS) k_prep(const T* __restrict__ pats, in
         const Vec4<T> x = load_vec4(img4 + c);
         const float4 f = make_float4(as_float(x.v[0]), as_float(x.v[1]), as_float(x.v[2]), as_float(x.v[3]));
         row4[c] = f;
-        part += (f.x + f.y) + (f.z + f.w);
+        if constexpr (C == 4) {
+          part[0] += f.x;
+          part[1] += f.y;
+          part[2] += f.z;
+          part[3] += f.w;
+        } else {
+          part[0] += f.x + f.y;
+          part[C - 1] += f.z + f.w;
+        }
       }
     } else if (b == 1) {
 #pragma unroll 4
       for (int p = threadIdx.x; p < n_pix; p += THREADS) {
         const float v = load_pixel(img, pix ? __ldg(pix + p) : p);
         row[p] = v;
-        part += v;
+        add_in_turn(part, v);
       }
     } else {
       for (int p = threadIdx.x; p < n_pix; p += THREADS) {
@@ -323,10 +363,10 @@ __global__ void __launch_bounds__(THREADS) k_prep(const T* __restrict__ pats, in
           for (int c = 0; c < b; ++c) s += load_pixel(img, src + (int64_t)a * w + c);
         const float v = s / cnt;
         row[p] = v;
-        part += v;
+        add_in_turn(part, v);
       }
     }
-    finalize_row(row, n_pix, inv_n, subtract_mean, (double)part, r, o, red);
+    finalize_row<THREADS>(row, n_pix, inv_n, subtract_mean, sum_of_chains(part), r, o, red);
     __syncthreads();
   }
 }
@@ -457,7 +497,8 @@ static int launch_prep(const T* patterns, int64_t n_rows, int height, int width,
                        void* stream) {
   // Threads for a row: enough CTAs on an SM to keep HBM busy, enough threads
   // for a long row. 60^2 px: 128 threads 6.03, 256 5.18 TB/s; 80^2 (e4m3):
-  // 5.34, 5.96; 128^2: 256 threads 5.44, 512 5.12; 160^2: 4.88, 5.31.
+  // 5.34, 5.96; 128^2: 256 threads 5.44, 512 5.12; 160^2: 4.88, 5.31 (with the
+  // finaliser's loops unrolled; rolled, what it takes now is 0 to 30 % faster).
 #define EBSD_PREP(THREADS)                                                                                       \
   launch_prep_threads<T, THREADS>(patterns, n_rows, height, width, pattern_stride, binning, pix_index, n_pix, \
                                   subtract_mean, o, as_stream(stream))
