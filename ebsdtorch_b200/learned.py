@@ -73,14 +73,12 @@ class _Conv:
         out32 = torch.empty((M, self.cout), dtype=torch.float32, device=x.device) if want32 else None
         if self.cin == 1:
             # 9 taps: a direct SIMT convolution beats a GEMM padded to K = 64
-            call("ebsd_cnn_conv_c1" if x.dtype == torch.bfloat16 else "ebsd_cnn_conv_c1_f32", ptr(x), B, H, W, ptr(self.w16), self.K_pad, ptr(self.b), self.cout, 1, ptr(out),
-                 ptr(out32), _stream(x))
-            keep.update(x=x)
+            call("ebsd_cnn_conv_c1" if x.dtype == torch.bfloat16 else "ebsd_cnn_conv_c1_f32", ptr(x), B, H, W,
+                 ptr(self.w16), self.K_pad, ptr(self.b), self.cout, 1, ptr(out), ptr(out32), _stream(x))
         elif _capi.load().ebsd_cnn_conv_supported(self.cin, self.cout, W):
             # patches gathered into the operand tiles by strided copies, no columns
             call("ebsd_cnn_conv_tc", ptr(x), B, H, W, self.cin, ptr(self.w16), self.K_pad, ptr(self.b), self.cout, 1,
                  ptr(out), ptr(out32), ptr(self.status), _stream(x))
-            keep.update(x=x)
         else:
             # one tcgen05 GEMM with the output channels on the 128-row side and
             # the long pixel axis streamed in a few hundred units; bias, ReLU
@@ -89,8 +87,7 @@ class _Conv:
             call("ebsd_cnn_conv_fwd", ptr(self.w16), self.w16.shape[0], ptr(cols), cols.shape[0], self.K_pad,
                  ptr(self.b), self.cout, M, 1, ptr(out), self.cout, ptr(out32), self.fwd_splits, ptr(self.status),
                  _stream(x))
-            keep.update(cols=cols)
-        keep.update(out=out, M=M, H=H, W=W, B=B)
+        keep.update(x=x, out=out, M=M, H=H, W=W, B=B)
         return out, out32, Ho, Wo
 
     def backward(self, dout: torch.Tensor, keep: dict, need_dx: bool, products: list) -> Optional[torch.Tensor]:
@@ -98,6 +95,7 @@ class _Conv:
         gradient's product is appended to `products` (a network launches those
         of its layers together)."""
         M, B, H, W = keep["M"], keep["B"], keep["H"], keep["W"]
+        dout = dout.contiguous()
         dev = dout.device
         s = _stream(dout)
         # ReLU gradient: rows for the column gradient, their transpose for the
@@ -105,15 +103,12 @@ class _Conv:
         ld16 = round_up(self.cout, 64)
         g16 = torch.empty((M, ld16), dtype=torch.bfloat16, device=dev) if need_dx else None
         gT = torch.empty((M // 64, round_up(self.cout, 16), 64), dtype=torch.bfloat16, device=dev)
-        call("ebsd_cnn_relu_grad_t", ptr(dout.contiguous()), ptr(keep["out"]), M, self.cout, ptr(g16), ld16, ptr(gT),
+        call("ebsd_cnn_relu_grad_t", ptr(dout), ptr(keep["out"]), M, self.cout, ptr(g16), ld16, ptr(gT),
              gT.shape[1], ptr(self.gb), s)
         # weight gradient: (cout x K) = g^T (cout x M) . cols (M x K), both
         # operands transposed and blocked by 64 pixels
-        if "cols" in keep:
-            colsT = keep["cols"][:M].view(M // 64, 64, self.K_pad).transpose(1, 2).contiguous()
-        else:
-            colsT = torch.empty((M // 64, round_up(self.K, 16), 64), dtype=torch.bfloat16, device=dev)
-            call("ebsd_cnn_im2col_t", ptr(keep["x"]), B, H, W, self.cin, ptr(colsT), colsT.shape[1], s)
+        colsT = torch.empty((M // 64, round_up(self.K, 16), 64), dtype=torch.bfloat16, device=dev)
+        call("ebsd_cnn_im2col_t", ptr(keep["x"]), B, H, W, self.cin, ptr(colsT), colsT.shape[1], s)
         products.append((gT, colsT, self.gw))
         if not need_dx:
             return None
