@@ -283,9 +283,9 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint32_t bar, uint32_t parity
 // Wait under a limit shorter than the default (a caller-set watchdog): no
 // spin phase, and every try_wait suspends for at most 200 ns, so the limit
 // is checked at least every 200 ns whatever the hardware's own suspend time.
-// Only the epilogue's waits (mbar_wait_sleep) take this path: it gives up
-// first, and the producer and MMA threads then stop on the abort flag, so
-// their latency-critical waits keep the plain form below.
+// Only the epilogues' waits (mbar_wait_sleep, mbar_wait_epilogue) take this
+// path: it gives up first, and the producer and MMA threads then stop on the
+// abort flag, so their latency-critical waits keep the plain form below.
 static __device__ __noinline__ bool mbar_wait_short(uint32_t bar, uint32_t parity, volatile int* abort,
                                              uint64_t limit_ns) {
   const uint64_t t0 = globaltimer_ns();
@@ -331,6 +331,15 @@ __device__ __forceinline__ bool mbar_wait_sleep(uint32_t bar, uint32_t parity, v
     if (globaltimer_ns() - t0 > limit_ns) return false;
     __nanosleep(500);
   }
+}
+
+// As mbar_wait, for the epilogue of a kernel whose accumulators are too short to
+// sleep for: only limits below the default take the form that counts them from
+// the first poll.
+__device__ __forceinline__ bool mbar_wait_epilogue(uint32_t bar, uint32_t parity, volatile int* abort,
+                                                   uint64_t limit_ns) {
+  if (limit_ns < kWaitLimitNs) return mbar_wait_short(bar, parity, abort, limit_ns);
+  return mbar_wait(bar, parity, abort, limit_ns);
 }
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {

@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
     uint32_t acc_phase = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < p.tiles; t += gridDim.x) {
-      ok = __all_sync(0xffffffffu, mbar_wait(accf_bar(acc), acc_phase, abort_flag, wait_ns));
+      ok = __all_sync(0xffffffffu, mbar_wait_epilogue(accf_bar(acc), acc_phase, abort_flag, wait_ns));
       if (!ok) break;
       tc_fence_after();
       const int nb = t / p.tiles_h, n = nb * p.nt + rn, h = (t - nb * p.tiles_h) * p.ht + rh;
