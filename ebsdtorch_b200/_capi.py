@@ -96,6 +96,7 @@ SIGNATURES = {
     "ebsd_cnn_bias_act": (i32, [vp, i64, vp, i64, i32, i32, vp, i64, vp, vp]),
     "ebsd_cnn_conv_c1": (i32, [vp, i32, i32, i32, vp, i32, vp, i32, i32, vp, vp, vp]),
     "ebsd_cnn_conv_c1_f32": (i32, [vp, i32, i32, i32, vp, i32, vp, i32, i32, vp, vp, vp]),
+    "ebsd_gemm_nt_takes_narrow_tiles": (i32, [i64, i64, i64, i32]),
     "ebsd_gemm_nt_group": (i32, [i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     "ebsd_cnn_im2col_t": (i32, [vp, i32, i32, i32, i32, vp, i64, vp]),
     "ebsd_cnn_relu_grad_t": (i32, [vp, vp, i64, i32, vp, i64, vp, i64, vp, vp]),

@@ -1647,11 +1647,14 @@ extern "C" int ebsd_match_topk(const void* queries_lp, int64_t n_queries_pad, co
 }
 
 // Whether a product runs k_tc_gemm_long: K long enough that one unit's chain
-// outlasts its set-up, and too few 128 x 256 tiles to occupy half of the SMs
-// (with more, the wide tiles re-read A less often). At K = 4,096 and 18 wide
-// tiles the two take 0.030 and 0.034 ms, at K = 262,144 and 2 tiles 0.70 and 1.51.
+// outlasts its set-up, and all units of 128 x 32 (or 16) outputs at once on the
+// SMs. Up to there they take 0.45 to 0.85 of the wide tiles' time (K = 2,048 to
+// 131,072; 128 x 256 outputs, K = 131,072: 471 and 659 us); in a second wave
+// 0.8 to 1.4, in a third and fourth 1.2 to 2.6 (2,048 x 1,024 and K = 10,944 181
+// against 71 us): a step of K takes a wide tile 1.4 times as long as a narrow one,
+// for eight times the outputs.
 static bool takes_long_tiles(int64_t m_tiles, int64_t n_valid, int64_t k_bytes) {
-  return k_bytes >= 4096 && m_tiles * ceil_div(n_valid, 256) <= device_sm_count() / 2;
+  return k_bytes >= 4096 && m_tiles * ceil_div(n_valid, 32) <= device_sm_count();
 }
 
 // Completes the parameters and tensor maps of one product; units: its CTAs.
@@ -1736,6 +1739,11 @@ extern "C" int ebsd_gemm_nt_group(int n, const void* const* A, const int64_t* a_
   k_tc_gemm_long_group<<<g.first[n], THREADS, LONG_SMEM_BYTES, as_stream(stream)>>>(g);
   EBSD_LAUNCH_CHECK();
   return 0;
+}
+
+extern "C" int ebsd_gemm_nt_takes_narrow_tiles(int64_t m_valid, int64_t n_valid, int64_t k_pad, int lp_dtype) {
+  if (m_valid < 1 || n_valid < 1 || k_pad < 1) return 0;
+  return takes_long_tiles(ceil_div(m_valid, BM), n_valid, k_pad * (lp_dtype == EBSD_DT_BF16 ? 2 : 1)) ? 1 : 0;
 }
 
 extern "C" int ebsd_gemm_nt(const void* A, int64_t m_pad, const void* B, int64_t n_pad, int64_t k_pad,

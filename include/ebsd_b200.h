@@ -350,6 +350,9 @@ int ebsd_match_topk_noalloc(const void* queries_lp, int64_t n_queries, int64_t n
 int ebsd_gemm_nt(const void* A, int64_t m_pad, const void* B, int64_t n_pad, int64_t k_pad,
                  int lp_dtype, float alpha, int accumulate, float* C, int64_t ldc, int64_t m_valid,
                  int64_t n_valid, int splits, int* d_status, void* stream);
+/* 1 where splits <= 0 takes narrow tiles (few outputs, long K: the same sums
+ * in the same order, one unit an SM at most), 0 where it takes 128 x 256. */
+int ebsd_gemm_nt_takes_narrow_tiles(int64_t m_valid, int64_t n_valid, int64_t k_pad, int lp_dtype);
 /* Up to 8 bf16 products A B^T with a long K in one launch, from operands
  * blocked by 64 of K: A[i] is (k / 64) x a_rows x 64, B[i] (k / 64) x b_rows x
  * 64, 16-byte aligned, C[i] (m x n_cols, row stride ldc); the sums run in the
