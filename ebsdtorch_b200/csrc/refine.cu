@@ -31,13 +31,15 @@
 namespace ebsd {
 
 constexpr int kRefThreads = 512;
-// Candidates scored per pass over the pixels, in threes whose gathers are issued
-// together. Cubes of odd side leave no slot idle (27, nearly 125 and 343), and the
-// 18 sums fit two CTAs of 512 threads on an SM: 27 candidates on 4,096 patterns of
-// 128^2 px take 24.3 ms, 16 in fours (one CTA) 30.5, 12 in twos 26.1, 8 in fours
-// 25.1, 4 27.0; 7 candidates 8.1 ms against 9.8 (16) and 6.9 (8 one by one).
-constexpr int kRefGroup = 9;
-constexpr int kRefIlp = 3;
+// GROUP candidates are scored per pass over the pixels, ILP of them with their
+// gathers issued together. Nine in threes: cubes of odd side leave no slot idle
+// (27, nearly 125 and 343), and the 18 sums fit two CTAs of 512 threads on an SM:
+// 27 candidates on 4,096 patterns of 128^2 px take 24.3 ms, 16 in fours (one CTA)
+// 30.5, 12 in twos 26.1, 8 in fours 25.1, 4 27.0; 7 candidates 8.1 ms against 9.8
+// (16) and 6.9 (8 one by one). Up to one pattern an SM there is no second CTA to
+// hide latencies, and 16 in fours are faster: 148 patterns of 60^2 px, two
+// iterations, 27 / 125 / 343 candidates 227 / 920 / 2,421 us, nine in threes 242 /
+// 1,010 / 2,736 (a master of 501 rows); 200 patterns 329 / 1,420 / 3,850 either way.
 constexpr int kMaxRefGrid = 343;  // (2 * 3 + 1)^3
 constexpr int kMaxRefPix = 40960;  // FP32 pattern row in shared memory (160 KiB)
 
@@ -59,8 +61,8 @@ __device__ __forceinline__ void qstd_d(double q[4]) {
 // 4,096 patterns of 128^2 px, 27 candidates, 3 iterations: 24.3 ms (224 samples
 // per ns, the projector's rate); 39 ms with 32 slots for the 27 candidates, one
 // CTA per SM and the sampling chain as the compiler contracts it. Same bits.
-template <bool QUADS>
-__global__ void __launch_bounds__(kRefThreads, 2) k_refine(
+template <bool QUADS, int GROUP, int ILP, int CTAS>
+__global__ void __launch_bounds__(kRefThreads, CTAS) k_refine(
     const float* __restrict__ mp, int mp_h, const LambertGrid lg, const float* __restrict__ coords, int n_pix,
     const float* __restrict__ offsets, const float* __restrict__ exp_rows, int64_t ld_e,
     const float* __restrict__ q_in, int64_t n, const float* __restrict__ grid, int n_grid, int centre,
@@ -69,8 +71,8 @@ __global__ void __launch_bounds__(kRefThreads, 2) k_refine(
   extern __shared__ float erow[];
   __shared__ float4 cand[kMaxRefGrid];
   __shared__ float score[kMaxRefGrid];
-  __shared__ float part_d[kRefThreads / 32][kRefGroup];
-  __shared__ float part_s[kRefThreads / 32][kRefGroup];
+  __shared__ float part_d[kRefThreads / 32][GROUP];
+  __shared__ float part_s[kRefThreads / 32][GROUP];
   __shared__ double qcur[4];
   __shared__ float scale_s;
   __shared__ float red[32];
@@ -119,11 +121,11 @@ __global__ void __launch_bounds__(kRefThreads, 2) k_refine(
         cand[t] = make_float4((float)best[0], (float)best[1], (float)best[2], (float)best[3]);
       }
       __syncthreads();
-      for (int g0 = 0; g0 < n_grid; g0 += kRefGroup) {
-        const int ng = min(kRefGroup, n_grid - g0);
-        float ad[kRefGroup], as[kRefGroup];
+      for (int g0 = 0; g0 < n_grid; g0 += GROUP) {
+        const int ng = min(GROUP, n_grid - g0);
+        float ad[GROUP], as[GROUP];
 #pragma unroll
-        for (int c = 0; c < kRefGroup; ++c) {
+        for (int c = 0; c < GROUP; ++c) {
           ad[c] = 0.f;
           as[c] = 0.f;
         }
@@ -139,21 +141,21 @@ __global__ void __launch_bounds__(kRefThreads, 2) k_refine(
             vz /= nr;
           }
           const float e = erow[p];
-          // kRefIlp candidates at a time: taps first, then their gathers together
+          // ILP candidates at a time: taps first, then their gathers together
 #pragma unroll
-          for (int c0 = 0; c0 < kRefGroup; c0 += kRefIlp) {
+          for (int c0 = 0; c0 < GROUP; c0 += ILP) {
             if (c0 >= ng) break;
-            LambertTap<QUADS> t[kRefIlp];
+            LambertTap<QUADS> t[ILP];
 #pragma unroll
-            for (int k = 0; k < kRefIlp; ++k) {
+            for (int k = 0; k < ILP; ++k) {
               const float4 q = cand[g0 + min(c0 + k, ng - 1)];
               t[k] = lambert_tap<true, QUADS>(lg, q, make_float3(2.0f * q.y, 2.0f * q.z, 2.0f * q.w), vx, vy, vz);
             }
-            float4 v[kRefIlp];
+            float4 v[ILP];
 #pragma unroll
-            for (int k = 0; k < kRefIlp; ++k) v[k] = load_taps(mp, mp_h, lg, t[k]);
+            for (int k = 0; k < ILP; ++k) v[k] = load_taps(mp, mp_h, lg, t[k]);
 #pragma unroll
-            for (int k = 0; k < kRefIlp; ++k) {
+            for (int k = 0; k < ILP; ++k) {
               const int c = c0 + k;
               if (c < ng) {
                 const float val = blend(t[k], v[k]);
@@ -164,7 +166,7 @@ __global__ void __launch_bounds__(kRefThreads, 2) k_refine(
           }
         }
 #pragma unroll
-        for (int c = 0; c < kRefGroup; ++c) {
+        for (int c = 0; c < GROUP; ++c) {
           const float d = warp_sum(ad[c]), s = warp_sum(as[c]);
           if (lane == 0) {
             part_d[wid][c] = d;
@@ -231,9 +233,10 @@ static int refine_grid(const float* master_pattern, int mp_h, int mp_w2, const f
   LaueTable t{};
   build_laue_table(laue_id, &t);
   const size_t smem = (size_t)n_pix * sizeof(float);
-  EBSD_CUDA_CHECK(cudaFuncSetAttribute(k_refine<QUADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const auto fn = n <= device_sm_count() ? k_refine<QUADS, 16, 4, 1> : k_refine<QUADS, 9, 3, 2>;
+  EBSD_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = (int)std::min<int64_t>(n, (int64_t)device_sm_count() * 16);
-  k_refine<QUADS><<<grid, kRefThreads, smem, as_stream(stream)>>>(
+  fn<<<grid, kRefThreads, smem, as_stream(stream)>>>(
       master_pattern, mp_h, lambert_grid<true>(mp_h, mp_w2), coords_soa, n_pix, offsets, exp_rows, ld_e, q_in, n,
       grid_cu, n_grid, (n_grid - 1) / 2, t, fz_left, n_iter, shrink, q_out, dots);
   EBSD_LAUNCH_CHECK();
