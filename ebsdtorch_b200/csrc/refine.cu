@@ -37,9 +37,10 @@ constexpr int kRefThreads = 512;
 // 27 candidates on 4,096 patterns of 128^2 px take 24.3 ms, 16 in fours (one CTA)
 // 30.5, 12 in twos 26.1, 8 in fours 25.1, 4 27.0; 7 candidates 8.1 ms against 9.8
 // (16) and 6.9 (8 one by one). Up to one pattern an SM there is no second CTA to
-// hide latencies, and 16 in fours are faster: 148 patterns of 60^2 px, two
+// hide latencies, and 16 in fours are faster from 10 candidates on: 148 patterns of 60^2 px, two
 // iterations, 27 / 125 / 343 candidates 227 / 920 / 2,421 us, nine in threes 242 /
-// 1,010 / 2,736 (a master of 501 rows); 200 patterns 329 / 1,420 / 3,850 either way.
+// 1,010 / 2,736, but 9 candidates 107 and 92 (a master of 501 rows); 200 patterns
+// 329 / 1,420 / 3,850 either way.
 constexpr int kMaxRefGrid = 343;  // (2 * 3 + 1)^3
 constexpr int kMaxRefPix = 40960;  // FP32 pattern row in shared memory (160 KiB)
 
@@ -233,7 +234,7 @@ static int refine_grid(const float* master_pattern, int mp_h, int mp_w2, const f
   LaueTable t{};
   build_laue_table(laue_id, &t);
   const size_t smem = (size_t)n_pix * sizeof(float);
-  const auto fn = n <= device_sm_count() ? k_refine<QUADS, 16, 4, 1> : k_refine<QUADS, 9, 3, 2>;
+  const auto fn = n <= device_sm_count() && n_grid > 9 ? k_refine<QUADS, 16, 4, 1> : k_refine<QUADS, 9, 3, 2>;
   EBSD_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = (int)std::min<int64_t>(n, (int64_t)device_sm_count() * 16);
   fn<<<grid, kRefThreads, smem, as_stream(stream)>>>(
