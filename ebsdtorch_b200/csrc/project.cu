@@ -98,8 +98,8 @@ __device__ __forceinline__ void add_in_turn(float (&c)[N], float v) {
 // not synchronised since writing the row, and synchronises before the row or the
 // scratch are written again. The loops are short and kept rolled: unrolled by
 // four they hold 48 to 64 registers instead of 32 to 40, which costs K2 CTAs on
-// an SM (65,536 uint16 patterns of 60^2 px 397 us, 380 rolled; half of the pixels
-// masked 294 and 219; 32,768 of 80^2 px 357 and 326).
+// an SM (65,536 uint16 patterns of 60^2 px 397 us, 348 rolled; half of the pixels
+// masked 294 and 218; 32,768 of 80^2 px 357 and 315).
 template <int THREADS>
 __device__ __forceinline__ void finalize_row(const float* row, int n, double inv_n, int subtract_mean,
                                              double part_sum, int64_t r, const RowOut& o, RowScratch& red) {
@@ -485,6 +485,11 @@ static int launch_prep_threads(const T* patterns, int64_t n_rows, int height, in
   const size_t smem = (size_t)n_pix * sizeof(float);
   const auto fn = k_prep<T, THREADS>;
   EBSD_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // No more CTAs on an SM than leave L1 room for their loads in flight: rows of
+  // 3,840 to 4,096 FP32 pixels with 12 CTAs and 28 KB of L1 take 113 us for 240 MB
+  // in, 360 MB out; with 164 KB for the rows 99
+  if (THREADS == 128)
+    EBSD_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 72));
   const int grid = row_grid(n_rows, smem, (const void*)fn, THREADS);
   const int vec4 = binning == 1 && !pix_index && n_pix % 4 == 0 && pattern_stride % 4 == 0 &&
                    reinterpret_cast<uintptr_t>(patterns) % (4 * sizeof(T)) == 0;
