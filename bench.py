@@ -1217,12 +1217,14 @@ def run_pcfit(args):
     def st_project():
         kernels.project(mp_b, rays, quats, RowBuffers(f32=sims), subtract_mean=False)
 
+    quad = F.spectra_layout(hp, wp)  # the layout that the fit uses
+
     def st_spectra():
-        _capi.call("ebsd_pcfit_spectra", sims.data_ptr(), hp * wp, n, hp, wp, tables.data_ptr(), spec.data_ptr(),
+        _capi.call("ebsd_pcfit_spectra" + quad, sims.data_ptr(), hp * wp, n, hp, wp, tables.data_ptr(), spec.data_ptr(),
                    status.data_ptr(), stream)
 
     def st_xcorr():
-        _capi.call("ebsd_pcfit_xcorr_max", spec.data_ptr(), n, terms.data_ptr(), B, hp, wp, tables.data_ptr(),
+        _capi.call("ebsd_pcfit_xcorr_max" + quad, spec.data_ptr(), n, terms.data_ptr(), B, hp, wp, tables.data_ptr(),
                    keys.data_ptr(), 0, status.data_ptr(), stream)
 
     def st_fold():
