@@ -295,8 +295,8 @@ __global__ void __launch_bounds__(256) k_relu_grad_t(const float* __restrict__ d
   if ((int)threadIdx.x < cw) atomicAdd(db + c0 + threadIdx.x, sums[threadIdx.x]);
 }
 
-// dx[b, iy, ix, c] = sum over the (output, tap) pairs that read it of dcols.
-// VEC: four channels per thread (C and ld multiples of 4, aligned).
+// dx[b, iy, ix, c] = sum over the (output, tap) pairs that read it of dcols, four
+// channels per thread (C and ld multiples of 4, both aligned).
 __global__ void k_col2im4(const float* __restrict__ dcols, int64_t ld, int B, int H, int W, int C, int Ho, int Wo,
                           float* __restrict__ dx) {
   const int c4s = C / 4;
@@ -326,6 +326,7 @@ __global__ void k_col2im4(const float* __restrict__ dcols, int64_t ld, int B, in
   }
 }
 
+// The same for any C, ld and alignment, one channel per thread.
 __global__ void k_col2im(const float* __restrict__ dcols, int64_t ld, int B, int H, int W, int C, int Ho, int Wo,
                          float* __restrict__ dx) {
   const int64_t total = (int64_t)B * H * W * C;

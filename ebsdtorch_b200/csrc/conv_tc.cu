@@ -24,8 +24,9 @@
 //
 // The im2col route wrote and re-read 9/4 of every activation and padded layer
 // 2's 64 channels to 128 rows. Batch 4,096 at 128 x 128 px: layers 2-5 3.49 ms
-// with im2col, 0.83 ms here (32 -> 64 channels 0.40, with strided copies 0.66;
-// 64 -> 128 0.21, 731 TFLOP/s; 128 -> 256 0.14, 1,079; 256 -> 256 0.07, 1,112).
+// with im2col, 0.92 ms here (32 -> 64 channels 0.43, with strided copies 0.66;
+// 64 -> 128 0.23, 660 TFLOP/s; 128 -> 256 0.15, 1,059; 256 -> 256 0.11 with its
+// FP32 copy, 0.07 without).
 #include <algorithm>
 
 #include "common.cuh"
